@@ -228,10 +228,11 @@ void launch_interpolate3(const float* gx, const float* gy, const float* gz, cons
 // ---------------------------------------------------------------------------------------------
 // Tree — tree.cu
 // ---------------------------------------------------------------------------------------------
+constexpr uint32_t NODE_FLAT = 1u << 31;  // an inner node whose children all have no octant-0 child
 struct TreeNodes {
   DevBuf geo;    // float4 centre.xyz, half
   DevBuf mass;   // float4 com.xyz, count
-  DevBuf link;   // uint4 start, end, first_child, child_mask | depth << 8
+  DevBuf link;   // uint4 start, end, first_child, child_mask | depth << 8 | NODE_FLAT
   DevBuf counters;  // u32[64]: per-level allocation counts, totals
   DevBuf prefix;    // double prefix sums of sorted positions (3 per particle + 3)
   DevBuf scan_tmp;

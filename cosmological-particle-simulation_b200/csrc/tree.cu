@@ -365,7 +365,9 @@ __global__ void __launch_bounds__(PS_THREADS) k_pos_prefix(const float* __restri
   }
 }
 
-__global__ void k_tree_com(const uint4* __restrict__ link, const double* __restrict__ P, float4* mass,
+// Centres of mass, and NODE_FLAT for the inner nodes whose children all have no octant-0 child (bit
+// 0 of the mask, which the flag's store leaves as it is for the parents that read it).
+__global__ void k_tree_com(uint4* link, const double* __restrict__ P, float4* mass,
                            const uint32_t* __restrict__ counters, uint32_t capacity) {
   uint32_t total = 0;
   for (int j = 0; j <= KEY_LEVELS; ++j) total += counters[j];
@@ -377,6 +379,12 @@ __global__ void k_tree_com(const uint4* __restrict__ link, const double* __restr
     const double sy = P[3 * (size_t)L.y + 1] - P[3 * (size_t)L.x + 1];
     const double sz = P[3 * (size_t)L.y + 2] - P[3 * (size_t)L.x + 2];
     mass[node] = make_float4((float)(sx / c), (float)(sy / c), (float)(sz / c), (float)(L.y - L.x));
+    if (L.w & 1u) {
+      const uint32_t nch = (uint32_t)__popc(L.w & 0xFFu);
+      uint32_t any = 0;
+      for (uint32_t q = 0; q < nch; ++q) any |= *(volatile uint32_t*)&link[L.z + q].w;
+      if ((any & 1u) == 0u) *(volatile uint32_t*)&link[node].w = L.w | NODE_FLAT;
+    }
   }
 }
 
