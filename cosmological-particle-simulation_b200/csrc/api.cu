@@ -49,7 +49,7 @@ struct cpm_ctx {
   FftPlan plan;
   SortScratch sort;
   TreeNodes tree;
-  DevBuf x, x_sorted, keys, okeys, okeys_sorted, vals, acc, acc_sorted, out;
+  DevBuf x, x_sorted, keys, keys_sorted, vals, acc, acc_sorted, out;
   DevBuf mesh_fx, mesh_a, mesh_b, mesh_c, mesh_d, spec;
   DevBuf status, tree_counters, pk;
   uint64_t last_nodes = 0, last_pairs = 0, last_accepts = 0;
@@ -127,9 +127,9 @@ int cpm_ctx_destroy(cpm_ctx* c) {
   if (!c) return CPM_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
   fft_plan_free(c->plan);
-  for (DevBuf* b : {&c->sort.keys_alt, &c->sort.vals_alt, &c->sort.block_hist, &c->sort.scan_tmp, &c->tree.geo,
-                    &c->tree.mass, &c->tree.link, &c->tree.counters, &c->tree.prefix, &c->tree.scan_tmp, &c->tree.x4, &c->x,
-                    &c->x_sorted, &c->keys, &c->okeys, &c->okeys_sorted, &c->vals, &c->acc, &c->acc_sorted, &c->out, &c->mesh_fx, &c->mesh_a,
+  for (DevBuf* b : {&c->sort.pairs, &c->sort.pairs_alt, &c->sort.tile_hist, &c->sort.runs, &c->tree.geo,
+                    &c->tree.mass, &c->tree.link, &c->tree.counters, &c->tree.prefix,  &c->tree.x4, &c->x,
+                    &c->x_sorted, &c->keys, &c->keys_sorted, &c->vals, &c->acc, &c->acc_sorted, &c->out, &c->mesh_fx, &c->mesh_a,
                     &c->mesh_b, &c->mesh_c, &c->mesh_d, &c->spec, &c->status, &c->tree_counters, &c->pk})
     release(*b);
   tree_walk_free(c->tree);
@@ -163,9 +163,11 @@ static int deposit_fixed_ctx(cpm_ctx* c, const float* x3, size_t n, float mass, 
     CPM_CU(c, ensure(c->keys, n * sizeof(uint64_t)));
     CPM_CU(c, ensure(c->vals, n * sizeof(uint32_t)));
     CPM_CU(c, ensure(c->x_sorted, 3 * n * sizeof(float)));
-    launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<uint32_t>(c->vals),
-                       as<DevStatus>(c->status), c->stream);
-    CPM_CU(c, radix_sort_pairs(as<uint64_t>(c->keys), as<uint32_t>(c->vals), n, 3 * KEY_LEVELS, c->sort, c->stream));
+    CPM_CU(c, ensure(c->keys_sorted, n * sizeof(uint64_t)));
+    launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<DevStatus>(c->status),
+                       c->stream);
+    CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
+                              3 * KEY_LEVELS, c->sort, c->stream));
     launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
   }
   const float h = c->box / (float)c->n_mesh;
@@ -192,9 +194,11 @@ static int deposit_common(cpm_ctx* c, const float* x3, size_t n, float mass, int
     CPM_CU(c, ensure(c->keys, n * sizeof(uint64_t)));
     CPM_CU(c, ensure(c->vals, n * sizeof(uint32_t)));
     CPM_CU(c, ensure(c->x_sorted, 3 * n * sizeof(float)));
-    launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<uint32_t>(c->vals),
-                       as<DevStatus>(c->status), c->stream);
-    CPM_CU(c, radix_sort_pairs(as<uint64_t>(c->keys), as<uint32_t>(c->vals), n, 3 * KEY_LEVELS, c->sort, c->stream));
+    CPM_CU(c, ensure(c->keys_sorted, n * sizeof(uint64_t)));
+    launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<DevStatus>(c->status),
+                       c->stream);
+    CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
+                              3 * KEY_LEVELS, c->sort, c->stream));
     launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
   }
   const float h = c->box / (float)c->n_mesh;
@@ -396,16 +400,16 @@ int cpm_tree_accel(cpm_ctx* c, const float* x3, size_t n, float box_size, const 
   CPM_CU(c, cudaMemsetAsync(c->tree_counters.p, 0, sizeof(TreeCounters), c->stream));
   // Hilbert order, as in a simulation: the tree is the same, and the walk's groups of 32 are compact
   // (in octant order their boxes, by which the walk culls nodes and sources, reach across the curve's jumps).
-  CPM_CU(c, ensure(c->okeys, n * sizeof(uint64_t)));
-  CPM_CU(c, ensure(c->okeys_sorted, n * sizeof(uint64_t)));
-  launch_octant_keys(as<float>(c->x), n, box_size, KEY_LEVELS, as<uint64_t>(c->okeys), as<uint32_t>(c->vals),
-                     as<DevStatus>(c->status), c->stream, 0, as<uint64_t>(c->keys));
-  CPM_CU(c, radix_sort_pairs(as<uint64_t>(c->keys), as<uint32_t>(c->vals), n, 3 * KEY_LEVELS, c->sort, c->stream));
-  launch_permute_u64(as<uint64_t>(c->okeys), as<uint32_t>(c->vals), n, as<uint64_t>(c->okeys_sorted), c->stream);
+  CPM_CU(c, ensure(c->keys_sorted, n * sizeof(uint64_t)));
+  launch_octant_keys(as<float>(c->x), n, box_size, KEY_LEVELS, nullptr, as<DevStatus>(c->status), c->stream, 0,
+                     as<uint64_t>(c->keys));
+  CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
+                            3 * KEY_LEVELS, c->sort, c->stream));
   launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
-  CPM_CU(c, tree_build(c->tree, as<uint64_t>(c->keys), as<float>(c->x_sorted), n, box_size, as<DevStatus>(c->status),
-                       c->stream, 0.0f, KEY_LEVELS, 0, as<uint64_t>(c->okeys_sorted)));
-  launch_tree_walk(c->tree, as<float>(c->x_sorted), n, box_size, *split, k, as<float>(c->acc_sorted), 0,
+  CPM_CU(c, tree_pack(c->tree, as<float>(c->x_sorted), n, box_size, c->stream));
+  CPM_CU(c, tree_build(c->tree, as<uint64_t>(c->keys_sorted), as<float>(c->x_sorted), n, box_size,
+                       as<DevStatus>(c->status), c->stream));
+  launch_tree_walk(c->tree, n, box_size, *split, k, as<float>(c->acc_sorted), 0,
                    as<TreeCounters>(c->tree_counters), as<DevStatus>(c->status), c->stream);
   launch_scatter3(as<float>(c->acc_sorted), as<uint32_t>(c->vals), n, as<float>(c->acc), c->stream);
   CPM_CU(c, cudaMemcpyAsync(acc3, c->acc.p, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -435,12 +439,13 @@ int cpm_octant_keys(cpm_ctx* c, const float* x3, size_t n, float box_size, int l
   if ((rc = upload_positions(c, x3, n))) return rc;
   CPM_CU(c, ensure(c->keys, n * sizeof(uint64_t)));
   CPM_CU(c, ensure(c->vals, n * sizeof(uint32_t)));
-  launch_octant_keys(as<float>(c->x), n, box_size, levels, as<uint64_t>(c->keys), as<uint32_t>(c->vals),
-                     as<DevStatus>(c->status), c->stream);
+  launch_octant_keys(as<float>(c->x), n, box_size, levels, as<uint64_t>(c->keys), as<DevStatus>(c->status), c->stream);
   if (keys_out)
     CPM_CU(c, cudaMemcpyAsync(keys_out, c->keys.p, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
   if (perm_out) {
-    CPM_CU(c, radix_sort_pairs(as<uint64_t>(c->keys), as<uint32_t>(c->vals), n, 3 * levels, c->sort, c->stream));
+    CPM_CU(c, ensure(c->keys_sorted, n * sizeof(uint64_t)));
+    CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n, 3 * levels,
+                              c->sort, c->stream));
     CPM_CU(c, cudaMemcpyAsync(perm_out, c->vals.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   }
   return sync_and_check(c);

@@ -129,22 +129,21 @@ T* as(DevBuf& b) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Radix sort of (u64 key, u32 value) pairs — keys.cu / sort.cu
+// Keys and their radix sort — sort.cu
 // ---------------------------------------------------------------------------------------------
 struct SortScratch {
-  DevBuf keys_alt, vals_alt, block_hist, scan_tmp;
+  DevBuf pairs, pairs_alt, tile_hist, runs;
 };
 
-// Octant keys (tree.rs descent) of positions (AoS f32 or float4), values = 0..n-1.
+// Octant keys (tree.rs descent) of positions (AoS f32); keys may be null.
 // With n_box > 0 (a batch of boxes of n_box particles each, in box order), the box index is placed
 // above the 3 * levels octant bits. With hkeys, also the Hilbert keys of the same cubes (the same
 // box bits): sorted by them, every octree node's particles stay contiguous.
-void launch_octant_keys(const float* x3, size_t n, float box, int levels, uint64_t* keys, uint32_t* vals,
-                        DevStatus* st, cudaStream_t s, size_t n_box = 0, uint64_t* hkeys = nullptr);
-void launch_permute_u64(const uint64_t* in, const uint32_t* perm, size_t n, uint64_t* out, cudaStream_t s);
-// Stable LSD sort of the low `bits` bits of keys; result in keys/vals (ping-pong handled inside).
-cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int bits, SortScratch& sc,
-                             cudaStream_t s);
+void launch_octant_keys(const float* x3, size_t n, float box, int levels, uint64_t* keys, DevStatus* st,
+                        cudaStream_t s, size_t n_box = 0, uint64_t* hkeys = nullptr);
+// Stable sort of keys below 2^bits: sorted[i] = keys[perm[i]]; keys stays as it is.
+cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* perm, size_t n, int bits,
+                            SortScratch& sc, cudaStream_t s);
 // Exclusive scan of u32 (in place allowed); `tmp` is grown as needed.
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DevBuf& tmp, cudaStream_t s);
 
@@ -234,9 +233,8 @@ struct TreeNodes {
   DevBuf mass;   // float4 com.xyz, count
   DevBuf link;   // uint4 start, end, first_child, child_mask | depth << 8 | NODE_FLAT
   DevBuf counters;  // u32[64]: per-level allocation counts, totals
-  DevBuf prefix;    // double prefix sums of sorted positions (3 per particle + 3)
-  DevBuf scan_tmp;
-  DevBuf x4;        // float4 copy of the sorted positions for the walk
+  DevBuf prefix;    // FP64 prefix sums of the sorted positions, per chunk and per tile
+  DevBuf x4;        // float4 copy of the sorted positions, then the walk's words (WALK_*)
   DevBuf quad;      // per node 2 float4: second moments about the centre of mass (quadrupole mode)
   bool has_quad = false;  // the last build computed `quad`; the walk then adds quadrupole terms
   int walk_warps = 4;     // warps (groups of 32 particles) per walk block: 2, 4 or 8 (autotuned)
@@ -244,24 +242,33 @@ struct TreeNodes {
   size_t capacity = 0;
   void* walk_fit = nullptr;  // fitted pair-force coefficients of the last split (walk.cu)
 };
+// The words after the n packed positions: 1 when a position lies outside [0, L]; the walk's group counter.
+constexpr int WALK_OUTSIDE = 0, WALK_TICKET = 1;
+inline uint32_t* tree_words(TreeNodes& t, size_t n) { return reinterpret_cast<uint32_t*>(static_cast<float4*>(t.x4.p) + n); }
+__device__ __forceinline__ bool outside_box(float a, float b, float c, float box) {
+  return !(fminf(a, fminf(b, c)) >= 0.0f && fmaxf(a, fmaxf(b, c)) <= box);
+}
+// Room for n packed positions and their words (zeroed), for a caller that packs the sorted positions itself
+// (launch_reorder); tree_pack does both. Either comes before tree_build.
+cudaError_t tree_positions(TreeNodes& t, size_t n, cudaStream_t s);
+cudaError_t tree_pack(TreeNodes& t, const float* sorted_x3, size_t n, float box, cudaStream_t s);
 struct TreeCounters {
   unsigned long long leaf_pairs;    // pairs within r_cut summed directly
   unsigned long long node_accepts;  // accepted centres of mass
   unsigned long long candidates;    // (particle, source) pairs tested against r_cut in direct nodes
   unsigned long long reserved;
 };
-// Builds the octree over sorted keys/positions (sorted x as AoS f32). Returns the node count
+// Builds the octree over sorted keys and packed positions (t.x4; sorted x as AoS f32 for the quadrupoles). Returns the node count
 // through the counters buffer (read by tree_node_count). quad_half_max > 0 also computes the second
 // moments of every node with half < quad_half_max (the walk then adds quadrupole terms).
 // With n_box > 0 the keys hold a batch of boxes (box index above `levels` octant digits, boxes of
 // n_box particles in order): one root per box (nodes 0 .. boxes - 1), and the walk starts each
 // group of 32 particles at its box's root.
-// sorted_keys orders the particles: octant keys, or Hilbert keys (then octant_keys gives each
-// particle's octant key in the same order, from which a child's octant is read); a node's children
-// are stored in the order of its sort digits.
+// sorted_keys orders the particles: octant keys or Hilbert keys; a node's children are stored in the
+// order of its sort digits.
 cudaError_t tree_build(TreeNodes& t, const uint64_t* sorted_keys, const float* sorted_x3, size_t n, float box,
                        DevStatus* st, cudaStream_t s, float quad_half_max = 0.0f, int levels = KEY_LEVELS,
-                       size_t n_box = 0, const uint64_t* octant_keys = nullptr);
+                       size_t n_box = 0);
 // Half size from which a node can never be accepted by the walk (prune radius r_cut + sqrt(3) half
 // from the centre, centre of mass inside the cube, 2 half < theta r): +inf when theta >= 1/sqrt(3).
 float quad_half_bound(const cpm_force_split& split);
@@ -269,7 +276,7 @@ float quad_half_bound(const cpm_force_split& split);
 // when `accumulate` (the reference's g[c] += s[c], integrator.rs:154-158).
 // The coupling k is read from *k_dev when k_dev is set. With `list`, only the sorted particles
 // list[0 .. *list_n - 1] are walked (the grid is sized for n; the count is read on the device).
-void launch_tree_walk(const TreeNodes& t, const float* sorted_x3, size_t n, float box, const cpm_force_split& split,
+void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_split& split,
                       float k, float* acc3, int accumulate, TreeCounters* counters, DevStatus* st, cudaStream_t s,
                       const float* k_dev = nullptr, const uint32_t* list = nullptr, const uint32_t* list_n = nullptr);
 // Releases the walk's per-tree state (the fitted pair-force coefficients).
@@ -311,7 +318,11 @@ void launch_kick_drift_fixed(uint32_t* q3, float* x3, float* p3, const float* g3
 void launch_to_fixed(float* x3, uint32_t* q3, size_t n, float box, cudaStream_t s);
 // Gather permutation: out[i] = in[perm[i]] for AoS triples and for u32 ids.
 void launch_permute3(const float* in3, const uint32_t* perm, size_t n, float* out3, cudaStream_t s);
-void launch_permute_u32(const uint32_t* in, const uint32_t* perm, size_t n, uint32_t* out, cudaStream_t s);
+// The sorted step's particle arrays in one pass: x, p (triples), id, q when set, and when x4 is set the
+// packed positions and their words for the tree (tree_positions).
+void launch_reorder(const uint32_t* perm, size_t n, const float* x, const float* p, const uint32_t* id,
+                    const uint32_t* q, float* x2, float* p2, uint32_t* id2, uint32_t* q2, float4* x4, uint32_t* words,
+                    float box, cudaStream_t s);
 // Scatter back to caller order: out[id[i]] = in[i].
 void launch_scatter3(const float* in3, const uint32_t* id, size_t n, float* out3, cudaStream_t s);
 // Flags a non-finite coordinate in the status word.

@@ -69,10 +69,26 @@ __global__ void k_permute3(const float* __restrict__ in3, const uint32_t* __rest
   out3[3 * i + 2] = in3[3 * j + 2];
 }
 
-__global__ void k_permute_u32(const uint32_t* __restrict__ in, const uint32_t* __restrict__ perm, size_t n,
-                              uint32_t* __restrict__ out) {
+__global__ void k_reorder(const uint32_t* __restrict__ perm, size_t n, const float* __restrict__ x,
+                          const float* __restrict__ p, const uint32_t* __restrict__ id, const uint32_t* __restrict__ q,
+                          float* __restrict__ x2, float* __restrict__ p2, uint32_t* __restrict__ id2,
+                          uint32_t* __restrict__ q2, float4* __restrict__ x4, uint32_t* __restrict__ words, float box) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = in[perm[i]];
+  if (i >= n) return;
+  const size_t j = perm[i];
+  const float a0 = x[3 * j], a1 = x[3 * j + 1], a2 = x[3 * j + 2];
+  const float b0 = p[3 * j], b1 = p[3 * j + 1], b2 = p[3 * j + 2];
+  id2[i] = id[j];
+  if (q) {
+    const uint32_t c0 = q[3 * j], c1 = q[3 * j + 1], c2 = q[3 * j + 2];
+    q2[3 * i] = c0, q2[3 * i + 1] = c1, q2[3 * i + 2] = c2;
+  }
+  x2[3 * i] = a0, x2[3 * i + 1] = a1, x2[3 * i + 2] = a2;
+  p2[3 * i] = b0, p2[3 * i + 1] = b1, p2[3 * i + 2] = b2;
+  if (x4) {
+    x4[i] = make_float4(a0, a1, a2, 0.0f);
+    if (outside_box(a0, a1, a2, box)) words[WALK_OUTSIDE] = 1u;
+  }
 }
 
 __global__ void k_scatter3(const float* __restrict__ in3, const uint32_t* __restrict__ id, size_t n,
@@ -201,10 +217,12 @@ void launch_permute3(const float* in3, const uint32_t* perm, size_t n, float* ou
   k_permute3<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in3, perm, n, out3);
 }
 
-void launch_permute_u32(const uint32_t* in, const uint32_t* perm, size_t n, uint32_t* out, cudaStream_t s) {
+void launch_reorder(const uint32_t* perm, size_t n, const float* x, const float* p, const uint32_t* id,
+                    const uint32_t* q, float* x2, float* p2, uint32_t* id2, uint32_t* q2, float4* x4, uint32_t* words,
+                    float box, cudaStream_t s) {
   if (n == 0) return;
   count_launch();
-  k_permute_u32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, perm, n, out);
+  k_reorder<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(perm, n, x, p, id, q, x2, p2, id2, q2, x4, words, box);
 }
 
 void launch_scatter3(const float* in3, const uint32_t* id, size_t n, float* out3, cudaStream_t s) {

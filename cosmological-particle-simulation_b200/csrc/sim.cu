@@ -54,7 +54,7 @@ struct cpm_sim {
   FftPlan plan;
   SortScratch sort;
   TreeNodes tree;
-  DevBuf x, p, acc, id, x2, p2, id2, keys, vals, fx, gx, gy, gz, spec, status, counters, pk;
+  DevBuf x, p, acc, id, x2, p2, id2, keys, keys_sorted, vals, fx, gx, gy, gz, spec, status, counters, pk;
   // Per-step phase events, one set per buffer parity. The set of parity q is read back when the
   // next step of parity q is issued: the step in between is already queued, so the GPU does not
   // wait for the host.
@@ -86,9 +86,6 @@ struct cpm_sim {
   float net_threshold = 50.0f;
   float net_in_scale = 1.0f;
   DevBuf flag, offset, list, list_n, scan_tmp;
-  // Octant keys of the particles (the sort is by Hilbert keys in `keys`): as computed, and in the
-  // sorted order (the tree build reads each child's octant from them).
-  DevBuf okeys, okeys_sorted;
   // A batch of nb boxes of n_box particles each (the ensemble): particles box by box, nb meshes one
   // after another, the box index above `levels` octant digits in the sort keys. nb = 1: one box.
   int nb = 1;
@@ -197,15 +194,16 @@ static int sim_accelerations(cpm_sim* s, float a, const StepScalars* dev = nullp
   // particles contiguous (the tree is the same), and the walk's groups of 32 consecutive particles
   // are more compact than in octant order, so fewer sources lie in a group's reach but outside its
   // particles' own.
-  launch_octant_keys(as<float>(s->x), n, s->box, s->levels, as<uint64_t>(s->okeys), as<uint32_t>(s->vals),
-                     as<DevStatus>(s->status), s->stream, batch_box(s), as<uint64_t>(s->keys));
-  SIM_CU(s, radix_sort_pairs(as<uint64_t>(s->keys), as<uint32_t>(s->vals), n, 63, s->sort, s->stream));
-  launch_permute_u64(as<uint64_t>(s->okeys), as<uint32_t>(s->vals), n, as<uint64_t>(s->okeys_sorted), s->stream);
-  launch_permute3(as<float>(s->x), as<uint32_t>(s->vals), n, as<float>(s->x2), s->stream);
-  launch_permute3(as<float>(s->p), as<uint32_t>(s->vals), n, as<float>(s->p2), s->stream);
-  launch_permute_u32(as<uint32_t>(s->id), as<uint32_t>(s->vals), n, as<uint32_t>(s->id2), s->stream);
-  if (fixed_point(s))  // the 32-bit words of q move like those of x
-    launch_permute3(as<float>(s->q), as<uint32_t>(s->vals), n, as<float>(s->q2), s->stream);
+  launch_octant_keys(as<float>(s->x), n, s->box, s->levels, nullptr, as<DevStatus>(s->status), s->stream,
+                     batch_box(s), as<uint64_t>(s->keys));
+  SIM_CU(s, radix_sort_keys(as<uint64_t>(s->keys), as<uint64_t>(s->keys_sorted), as<uint32_t>(s->vals), n, 63, s->sort,
+                            s->stream));
+  if (s->P.use_tree) SIM_CU(s, tree_positions(s->tree, n, s->stream));
+  launch_reorder(as<uint32_t>(s->vals), n, as<float>(s->x), as<float>(s->p), as<uint32_t>(s->id),
+                 fixed_point(s) ? as<uint32_t>(s->q) : nullptr, as<float>(s->x2), as<float>(s->p2),
+                 as<uint32_t>(s->id2), fixed_point(s) ? as<uint32_t>(s->q2) : nullptr,
+                 s->P.use_tree ? as<float4>(s->tree.x4) : nullptr, s->P.use_tree ? tree_words(s->tree, n) : nullptr,
+                 s->box, s->stream);
   swap_sorted(s);
   if (s->x_out) {
     SIM_CU(s, cudaEventRecord(s->ev_sorted, s->stream));
@@ -246,12 +244,12 @@ static int sim_accelerations(cpm_sim* s, float a, const StepScalars* dev = nullp
     const uint32_t* walk_list = learned ? as<uint32_t>(s->list) : nullptr;
     const uint32_t* walk_n = learned ? as<uint32_t>(s->list_n) : nullptr;
     const float quad_half = (s->P.flags & CPM_SIM_QUADRUPOLE) ? quad_half_bound(s->P.split) : 0.0f;
-    SIM_CU(s, tree_build(s->tree, as<uint64_t>(s->keys), as<float>(s->x), n, s->box, as<DevStatus>(s->status),
-                         s->stream, quad_half, s->levels, batch_box(s), as<uint64_t>(s->okeys_sorted)));
+    SIM_CU(s, tree_build(s->tree, as<uint64_t>(s->keys_sorted), as<float>(s->x), n, s->box, as<DevStatus>(s->status),
+                         s->stream, quad_half, s->levels, batch_box(s)));
     mark(s, 6);
     SIM_CU(s, cudaMemsetAsync(s->counters.p, 0, sizeof(TreeCounters), s->stream));
     const float k = tree_coupling(s->P.cosmo.omega_m, s->box, a, per_box(s));
-    launch_tree_walk(s->tree, as<float>(s->x), n, s->box, s->P.split, k, as<float>(s->acc), 1,
+    launch_tree_walk(s->tree, n, s->box, s->P.split, k, as<float>(s->acc), 1,
                      as<TreeCounters>(s->counters), as<DevStatus>(s->status), s->stream,
                      dev ? &dev->tree_k : nullptr, walk_list, walk_n);
   } else {
@@ -357,7 +355,7 @@ static int sim_autotune(cpm_sim* s) {
     for (int k = 0; k < 3; ++k) {
       s->tree.walk_warps = TUNE_WARPS[k];
       c.ms[6 + k] = time_ms(s->stream, e0, e1, [&] {
-        launch_tree_walk(s->tree, as<float>(s->x), s->n, s->box, s->P.split, kk, as<float>(s->host_tmp), 0, nullptr,
+        launch_tree_walk(s->tree, s->n, s->box, s->P.split, kk, as<float>(s->host_tmp), 0, nullptr,
                          as<DevStatus>(s->status), s->stream, nullptr, wl, wn);
       });
     }
@@ -420,8 +418,7 @@ static int sim_new(const cpm_sim_params* params, float a0, cpm_sim** out, int nb
   for (DevBuf* b : {&s->x, &s->p, &s->acc, &s->x2, &s->p2}) ok = ok && ensure(*b, 3 * n * sizeof(float)) == cudaSuccess;
   for (DevBuf* b : {&s->id, &s->id2, &s->vals}) ok = ok && ensure(*b, n * sizeof(uint32_t)) == cudaSuccess;
   ok = ok && ensure(s->keys, n * sizeof(uint64_t)) == cudaSuccess;
-  ok = ok && ensure(s->okeys, n * sizeof(uint64_t)) == cudaSuccess;
-  ok = ok && ensure(s->okeys_sorted, n * sizeof(uint64_t)) == cudaSuccess;
+  ok = ok && ensure(s->keys_sorted, n * sizeof(uint64_t)) == cudaSuccess;
   ok = ok && ensure(s->fx, m * sizeof(unsigned long long)) == cudaSuccess;
   for (DevBuf* b : {&s->gx, &s->gy, &s->gz}) ok = ok && ensure(*b, m * sizeof(float)) == cudaSuccess;
   ok = ok && ensure(s->spec, 3 * half * (size_t)nb * sizeof(float2)) == cudaSuccess;
@@ -949,7 +946,7 @@ int cpm_sim_short_range(cpm_sim* s, float* sr3) {
   // the tree of the last force evaluation was built on the current positions (the kick that ends a
   // step changes the momenta only)
   const float k = tree_coupling(s->P.cosmo.omega_m, s->box, s->a, per_box(s));
-  launch_tree_walk(s->tree, as<float>(s->x), n, s->box, s->P.split, k, as<float>(s->host_tmp), 0, nullptr,
+  launch_tree_walk(s->tree, n, s->box, s->P.split, k, as<float>(s->host_tmp), 0, nullptr,
                    as<DevStatus>(s->status), s->stream);
   launch_scatter3(as<float>(s->host_tmp), as<uint32_t>(s->id), n, as<float>(s->x2), s->stream);
   SIM_CU(s, cudaMemcpyAsync(sr3, s->x2.p, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
@@ -1005,11 +1002,11 @@ int cpm_sim_destroy(cpm_sim* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->side) cudaStreamSynchronize(s->side);
   fft_plan_free(s->plan);
-  for (DevBuf* b : {&s->sort.keys_alt, &s->sort.vals_alt, &s->sort.block_hist, &s->sort.scan_tmp, &s->tree.geo,
-                    &s->tree.mass, &s->tree.link, &s->tree.counters, &s->tree.prefix, &s->tree.scan_tmp, &s->tree.x4, &s->tree.quad, &s->x, &s->p,
+  for (DevBuf* b : {&s->sort.pairs, &s->sort.pairs_alt, &s->sort.tile_hist, &s->sort.runs, &s->keys_sorted, &s->tree.geo,
+                    &s->tree.mass, &s->tree.link, &s->tree.counters, &s->tree.prefix,  &s->tree.x4, &s->tree.quad, &s->x, &s->p,
                     &s->acc, &s->id, &s->x2, &s->p2, &s->id2, &s->keys, &s->vals, &s->fx, &s->gx, &s->gy, &s->gz,
                     &s->spec, &s->status, &s->counters, &s->pk, &s->q, &s->q2, &s->snap, &s->flag, &s->offset,
-                    &s->list, &s->list_n, &s->scan_tmp, &s->okeys, &s->okeys_sorted})
+                    &s->list, &s->list_n, &s->scan_tmp})
     release(*b);
   tree_walk_free(s->tree);
   release(s->host_tmp);

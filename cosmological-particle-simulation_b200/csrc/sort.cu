@@ -1,6 +1,8 @@
-// sort.cu — octant keys of the tree descent, stable LSD radix sort of (u64 key, u32 value)
-// pairs, and exclusive scans. HBM-bound integer work: coalesced tiles, per-warp ranking with
-// ballots, no tensor cores.
+// sort.cu — octant and Hilbert keys of the tree descent, the stable radix sort of u64 keys, and
+// exclusive scans. HBM-bound integer work: coalesced tiles, per-warp ranking with ballots, no
+// tensor cores.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -197,8 +199,8 @@ static const HilbertFsm& hilbert_fsm(int bits) {
 }
 
 __global__ void k_octant_keys(const float* __restrict__ x3, size_t n, float half0, int levels,
-                              uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, DevStatus* st,
-                              size_t n_box, int box_shift, uint64_t* __restrict__ hkeys, HilbertFsm fsm) {
+                              uint64_t* __restrict__ keys, DevStatus* st, size_t n_box,
+                              int box_shift, uint64_t* __restrict__ hkeys, HilbertFsm fsm) {
   __shared__ unsigned char table[HFSM_STATES * 8];
   const bool use_fsm = hkeys && fsm.ok;
   if (use_fsm) {
@@ -232,38 +234,24 @@ __global__ void k_octant_keys(const float* __restrict__ x3, size_t n, float half
     half = q;
   }
   const uint64_t boxbits = n_box ? (uint64_t)(i / n_box) << box_shift : 0ull;
-  keys[i] = key | boxbits;
+  if (keys) keys[i] = key | boxbits;
   if (hkeys) {
     const uint64_t h = use_fsm ? hkey
                                : (levels == KEY_LEVELS ? hilbert_from_axes<KEY_LEVELS>(a0, a1, a2)
                                                        : hilbert_from_axes<KEY_LEVELS - 2>(a0, a1, a2));
     hkeys[i] = h | boxbits;
   }
-  if (vals) vals[i] = (uint32_t)i;
 }
 
-void launch_octant_keys(const float* x3, size_t n, float box, int levels, uint64_t* keys, uint32_t* vals,
-                        DevStatus* st, cudaStream_t s, size_t n_box, uint64_t* hkeys) {
+void launch_octant_keys(const float* x3, size_t n, float box, int levels, uint64_t* keys, DevStatus* st,
+                        cudaStream_t s, size_t n_box, uint64_t* hkeys) {
   if (n == 0) return;
   const int T = 256;
   count_launch();
   HilbertFsm fsm;  // ok = 0: the direct transform
   if (hkeys && (levels == KEY_LEVELS || levels == KEY_LEVELS - 2)) fsm = hilbert_fsm(levels);
-  k_octant_keys<<<(unsigned)((n + T - 1) / T), T, 0, s>>>(x3, n, box / 2.0f, levels, keys, vals, st, n_box,
-                                                          3 * levels, hkeys, fsm);
-}
-
-__global__ void k_permute_u64(const uint64_t* __restrict__ in, const uint32_t* __restrict__ perm, size_t n,
-                              uint64_t* __restrict__ out) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    out[i] = in[perm[i]];
-}
-
-void launch_permute_u64(const uint64_t* in, const uint32_t* perm, size_t n, uint64_t* out, cudaStream_t s) {
-  if (n == 0) return;
-  count_launch();
-  const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
-  k_permute_u64<<<blocks, 256, 0, s>>>(in, perm, n, out);
+  k_octant_keys<<<(unsigned)((n + T - 1) / T), T, 0, s>>>(x3, n, box / 2.0f, levels, keys, st, n_box, 3 * levels,
+                                                          hkeys, fsm);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -369,16 +357,31 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DevB
 }
 
 // ---------------------------------------------------------------------------------------------
-// LSD radix sort, 8-bit digits. Per pass: block histograms (digit-major), exclusive scan of the
-// histograms, then a stable scatter. Within a block each warp ranks a contiguous sub-tile in
-// warp-striped rounds (lanes with equal digits found by ballots), so equal digits keep their
-// input order.
+// Stable radix sort of u64 keys, 8-bit digits, giving the sorted keys and the permutation.
+//
+// Only the upper 32 bits of the keys go through LSD passes, as 8-byte elements (those bits and the
+// 32-bit index); the last pass fetches each element's whole key. The particles of a simulation then
+// are in order but for short runs that share a cube of level 10 or 11 (0.16 of the mean spacing at
+// 256^3 particles; a handful of particles, a few hundred in the core of a cluster): a run of up to
+// RUN_SHORT elements is put in order by one thread, of up to RUN_MID by one warp, a longer one by one
+// CTA, whatever its length (a rank count in shared memory, or for runs over RUN_RANKED LSD passes over
+// the run). Eight passes of (u64 key, u32 index) moved 3.2 GB at 256^3 instead of 1.1.
+//
+// Per pass: digit counts per tile of 4096 (digit-major), their exclusive scan (one CTA per digit; with
+// up to RS_FEW tiles every tile of the scatter adds its digits' few counts itself), then a stable
+// scatter. Within a tile each warp ranks a contiguous sub-tile in warp-striped rounds (lanes with
+// equal digits found by ballots), so equal digits keep their input order.
+//
+// Up to SMALL_SORT keys go through the passes of their upper 24 bits in one launch of one cluster of
+// CTAs.
 // ---------------------------------------------------------------------------------------------
 constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 16;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
+constexpr int RS_FEW = 64;
+static_assert(RS_THREADS == RS_BINS, "one thread per digit");
 
 // The lanes whose 9-bit value d equals this lane's (a digit, or 0x100 | lane for a lane without
 // an element): one ballot per bit, the same mask as __match_any_sync.
@@ -392,61 +395,111 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
   return peers;
 }
 
-__global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const uint64_t* __restrict__ keys, size_t n, int shift,
-                                                           uint32_t* __restrict__ block_hist, int nblocks) {
+// Digit counts of each tile, by shared-memory atomics: the elements are in no order by the digit that
+// is counted, so lanes seldom meet. FIRST: the elements are the keys themselves, in their order
+// (neighbours share their upper digits then, which `same` takes out).
+template <bool FIRST>
+__global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const uint64_t* __restrict__ keys, int drop,
+                                                           const uint2* __restrict__ in, size_t n, int shift,
+                                                           uint32_t* __restrict__ tile_hist, int ntiles,
+                                                           uint32_t* __restrict__ runs) {
   __shared__ uint32_t h[RS_BINS];
-  for (int t = threadIdx.x; t < RS_BINS; t += RS_THREADS) h[t] = 0;
+  h[threadIdx.x] = 0;
+  if (runs && blockIdx.x == 0 && threadIdx.x < 2) runs[threadIdx.x] = 0;
   __syncthreads();
   const size_t base = (size_t)blockIdx.x * RS_TILE;
-  const int lane = threadIdx.x & 31;
-#pragma unroll 4
+  uint32_t v[RS_ITEMS];
+#pragma unroll
   for (int j = 0; j < RS_ITEMS; ++j) {
     const size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
-    const bool valid = i < n;
-    const uint32_t d = valid ? (uint32_t)((keys[i] >> shift) & (RS_BINS - 1)) : (0x100u | (uint32_t)lane);
-    const uint32_t peers = match_digit(d);
-    if (valid && (__ffs(peers) - 1) == lane) atomicAdd(&h[d], (uint32_t)__popc(peers));
+    v[j] = i >= n ? 0u : FIRST ? (uint32_t)(keys[i] >> drop) : in[i].x;
+  }
+#pragma unroll
+  for (int j = 0; j < RS_ITEMS; ++j) {
+    const bool valid = base + (size_t)j * RS_THREADS + threadIdx.x < n;
+    const uint32_t d = (v[j] >> shift) & (RS_BINS - 1);
+    const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
+    const bool same = __all_sync(0xffffffffu, valid && d == d0);
+    if (same ? (threadIdx.x & 31) == 0 : valid) atomicAdd(&h[d], same ? 32u : 1u);
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < RS_BINS; t += RS_THREADS) block_hist[(size_t)t * nblocks + blockIdx.x] = h[t];
+  tile_hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Dynamic shared memory of k_radix_scatter: per-warp digit counts, the block's digit starts and
-// global bases, and the tile reordered by digit.
-constexpr size_t RS_SCATTER_SMEM =
-    sizeof(uint32_t) * (RS_WARPS * RS_BINS + 2 * RS_BINS) + (sizeof(uint64_t) + sizeof(uint32_t)) * RS_TILE;
+// Exclusive scan of the tile counts of digit blockIdx.x, in place; its total to totals[digit].
+__global__ void __launch_bounds__(SC_THREADS) k_radix_scan(uint32_t* __restrict__ tile_hist, int ntiles,
+                                                           uint32_t* __restrict__ totals) {
+  __shared__ uint32_t ws[SC_THREADS / 32];
+  uint32_t* row = tile_hist + (size_t)blockIdx.x * ntiles;
+  uint32_t carry = 0;
+  for (int c0 = 0; c0 < ntiles; c0 += SC_TILE) {
+    const int i0 = c0 + threadIdx.x * SC_ITEMS;
+    uint32_t v[SC_ITEMS], sum = 0;
+#pragma unroll
+    for (int j = 0; j < SC_ITEMS; ++j) {
+      v[j] = i0 + j < ntiles ? row[i0 + j] : 0u;
+      sum += v[j];
+    }
+    uint32_t total;
+    uint32_t run = carry + block_exclusive_scan(sum, &total, ws);
+#pragma unroll
+    for (int j = 0; j < SC_ITEMS; ++j) {
+      if (i0 + j < ntiles) row[i0 + j] = run;
+      run += v[j];
+    }
+    carry += total;
+    __syncthreads();  // the next round reuses the warp sums
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
 
 // One stable pass: the tile is ranked by digit (per warp with match_digit, warps in order),
 // reordered in shared memory, and each digit's run is written out contiguously, so consecutive
-// threads store consecutive addresses.
-__global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __restrict__ kin,
-                                                              const uint32_t* __restrict__ vin,
-                                                              uint64_t* __restrict__ kout,
-                                                              uint32_t* __restrict__ vout, size_t n, int shift,
-                                                              const uint32_t* __restrict__ offsets, int nblocks) {
-  extern __shared__ __align__(16) unsigned char rs_smem[];
-  uint64_t* sk = reinterpret_cast<uint64_t*>(rs_smem);                       // [RS_TILE]
-  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + RS_TILE);                  // [RS_TILE]
-  uint32_t(*wc)[RS_BINS] = reinterpret_cast<uint32_t(*)[RS_BINS]>(sv + RS_TILE);  // [RS_WARPS][RS_BINS]
-  uint32_t* dstart = &wc[RS_WARPS][0];                                       // [RS_BINS]
-  uint32_t* gbase = dstart + RS_BINS;                                        // [RS_BINS]
-  __shared__ uint32_t warp_tot[RS_WARPS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int t = threadIdx.x; t < RS_WARPS * RS_BINS; t += RS_THREADS) (&wc[0][0])[t] = 0;
+// threads store consecutive addresses. LAST: whole keys and indices are written.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __restrict__ keys, int drop,
+                                                              const uint2* __restrict__ in, uint2* __restrict__ out,
+                                                              uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                              size_t n, int shift,
+                                                              const uint32_t* __restrict__ tile_hist,
+                                                              const uint32_t* __restrict__ totals, int ntiles) {
+  __shared__ uint2 se[RS_TILE];
+  __shared__ uint32_t wc[RS_WARPS][RS_BINS];
+  __shared__ uint32_t gbase[RS_BINS];
+  __shared__ uint32_t ws[SC_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < RS_WARPS; ++q) wc[q][t] = 0;
   __syncthreads();
   const unsigned lt_mask = (1u << lane) - 1u;
   const size_t tile0 = (size_t)blockIdx.x * RS_TILE;
   const size_t wbase = tile0 + (size_t)warp * 32 * RS_ITEMS;
-  uint64_t k[RS_ITEMS];
-  uint32_t v[RS_ITEMS];
+  uint2 e[RS_ITEMS];
   uint32_t rank[RS_ITEMS];
 #pragma unroll
   for (int j = 0; j < RS_ITEMS; ++j) {
     const size_t i = wbase + (size_t)j * 32 + lane;
-    const bool valid = i < n;
-    k[j] = valid ? kin[i] : 0ull;
-    v[j] = valid ? vin[i] : 0u;
-    const uint32_t d = valid ? (uint32_t)((k[j] >> shift) & (RS_BINS - 1)) : (0x100u | (uint32_t)lane);
+    e[j] = make_uint2(0u, 0u);
+    if (i < n) e[j] = FIRST ? make_uint2((uint32_t)(keys[i] >> drop), (uint32_t)i) : in[i];
+  }
+  // Thread t = digit t: where its elements of this tile start in the output.
+  uint32_t before = 0, all = 0;
+  if (totals) {
+    before = tile_hist[(size_t)t * ntiles + blockIdx.x];
+    all = totals[t];
+  } else {
+    for (int q = 0; q < ntiles; ++q) {
+      const uint32_t c = tile_hist[(size_t)t * ntiles + q];
+      all += c;
+      before += q < (int)blockIdx.x ? c : 0u;
+    }
+  }
+  uint32_t sum;
+  before += block_exclusive_scan(all, &sum, ws);
+#pragma unroll
+  for (int j = 0; j < RS_ITEMS; ++j) {
+    const bool valid = wbase + (size_t)j * 32 + lane < n;
+    const uint32_t d = valid ? (e[j].x >> shift) & (RS_BINS - 1) : (0x100u | (uint32_t)lane);
     const uint32_t peers = match_digit(d);
     uint32_t prev = 0;
     if (valid) prev = wc[warp][d];
@@ -458,25 +511,12 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __
     __syncwarp();
   }
   __syncthreads();
-  // Thread t = digit t: its block total, then the exclusive scan over digits (block-local starts).
-  static_assert(RS_THREADS == RS_BINS, "one thread per digit");
-  const int t = threadIdx.x;
+  // Thread t = digit t: its tile total, then the exclusive scan over digits (tile-local starts).
   uint32_t tot = 0;
 #pragma unroll
   for (int w = 0; w < RS_WARPS; ++w) tot += wc[w][t];
-  uint32_t incl = tot;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  uint32_t before = 0;
-  for (int w = 0; w < warp; ++w) before += warp_tot[w];
-  const uint32_t start = before + incl - tot;
-  dstart[t] = start;
-  gbase[t] = offsets[(size_t)t * nblocks + blockIdx.x] - start;
+  const uint32_t start = block_exclusive_scan(tot, &sum, ws);
+  gbase[t] = before - start;
   uint32_t run = start;
 #pragma unroll
   for (int w = 0; w < RS_WARPS; ++w) {
@@ -486,56 +526,347 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < RS_ITEMS; ++j) {
-    const size_t i = wbase + (size_t)j * 32 + lane;
-    if (i < n) {
-      const uint32_t d = (uint32_t)((k[j] >> shift) & (RS_BINS - 1));
-      const uint32_t lp = wc[warp][d] + rank[j];
-      sk[lp] = k[j];
-      sv[lp] = v[j];
-    }
-  }
+  for (int j = 0; j < RS_ITEMS; ++j)
+    if (wbase + (size_t)j * 32 + lane < n) se[wc[warp][(e[j].x >> shift) & (RS_BINS - 1)] + rank[j]] = e[j];
   __syncthreads();
   const uint32_t count = (uint32_t)min((size_t)RS_TILE, n - tile0);
-  for (uint32_t q = threadIdx.x; q < count; q += RS_THREADS) {
-    const uint64_t key = sk[q];
-    const uint32_t pos = gbase[(uint32_t)((key >> shift) & (RS_BINS - 1))] + q;
-    kout[pos] = key;
-    vout[pos] = sv[q];
+#pragma unroll 4
+  for (uint32_t q = t; q < count; q += RS_THREADS) {
+    const uint2 v = se[q];
+    const uint32_t pos = gbase[(v.x >> shift) & (RS_BINS - 1)] + q;
+    if constexpr (LAST) {
+      kout[pos] = __ldg(keys + v.y);
+      vout[pos] = v.y;
+    } else {
+      out[pos] = v;
+    }
   }
 }
 
-cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, size_t n, int bits, SortScratch& sc, cudaStream_t s) {
-  if (n <= 1 || bits <= 0) return cudaSuccess;
-  if (n > 0xFFFFFFFFull) return cudaErrorInvalidValue;
-  const int nblocks = (int)((n + RS_TILE - 1) / RS_TILE);
-  cudaError_t e;
-  if ((e = ensure(sc.keys_alt, n * sizeof(uint64_t))) != cudaSuccess) return e;
-  if ((e = ensure(sc.vals_alt, n * sizeof(uint32_t))) != cudaSuccess) return e;
-  if ((e = ensure(sc.block_hist, (size_t)RS_BINS * nblocks * sizeof(uint32_t))) != cudaSuccess) return e;
-  uint64_t* ka = keys;
-  uint32_t* va = vals;
-  uint64_t* kb = as<uint64_t>(sc.keys_alt);
-  uint32_t* vb = as<uint32_t>(sc.vals_alt);
-  uint32_t* hist = as<uint32_t>(sc.block_hist);
-  const int passes = (bits + 7) / 8;
-  // The attribute belongs to the current device, so it is set on every call (a cheap host call).
-  if ((e = cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)RS_SCATTER_SMEM)) != cudaSuccess)
-    return e;
+// ---------------------------------------------------------------------------------------------
+// The runs of elements that share key >> drop, put in order by their lower bits (stable: a run arrives
+// in input order).
+// ---------------------------------------------------------------------------------------------
+constexpr int RUN_SHORT = 8;
+constexpr int RUN_MID = 256;
+constexpr int RUN_RANKED = 2048;
+
+// The lists of runs: runs[0] of more than RUN_SHORT elements, their starts from runs[2]; runs[1] of
+// more than RUN_MID, their starts from the end downwards.
+
+// The thread of a run's first element sorts it by insertion, or lists it.
+__global__ void k_short_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop, uint32_t* runs) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i + 1 >= n) return;
+  // (another thread's insertions leave the upper bits of its run's slots as they are)
+  const volatile uint64_t* keys = sorted;
+  const uint64_t h = keys[i] >> drop;
+  if ((keys[i + 1] >> drop) != h || (i > 0 && (keys[i - 1] >> drop) == h)) return;
+  int len = 2;
+  while (len <= RUN_SHORT && i + len < n && (keys[i + len] >> drop) == h) ++len;
+  if (len > RUN_SHORT) {
+    runs[2 + atomicAdd(&runs[0], 1u)] = (uint32_t)i;
+    return;
+  }
+  uint64_t* k = sorted + i;
+  uint32_t* v = perm + i;
+  for (int a = 1; a < len; ++a) {
+    const uint64_t key = k[a];
+    const uint32_t val = v[a];
+    int b = a;
+    for (; b > 0 && k[b - 1] > key; --b) {
+      k[b] = k[b - 1];
+      v[b] = v[b - 1];
+    }
+    k[b] = key;
+    v[b] = val;
+  }
+}
+
+// One warp per listed run of up to RUN_MID elements, RUN_MID / 32 to a lane: every element's place is
+// the number of elements before it.
+__global__ void __launch_bounds__(256) k_mid_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop, uint32_t* runs,
+                                                  uint32_t runs_end) {
+  constexpr int PER = RUN_MID / 32;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t count = runs[0];
+  for (uint32_t r = blockIdx.x * 8 + (threadIdx.x >> 5); r < count; r += gridDim.x * 8) {
+    const size_t start = runs[2 + r];
+    const uint64_t h = sorted[start] >> drop;
+    uint64_t k[PER];
+    uint32_t v[PER];
+    int len = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const size_t i = start + 32 * q + lane;
+      k[q] = ~0ull;
+      const bool in = len == 32 * q && i < n && (sorted[i] >> drop) == h;
+      if (in) {
+        k[q] = sorted[i];
+        v[q] = perm[i];
+      }
+      len += __popc(__ballot_sync(FULL, in));
+    }
+    if (len == RUN_MID && start + RUN_MID < n && (sorted[start + RUN_MID] >> drop) == h) {
+      if (lane == 0) runs[runs_end - 1 - atomicAdd(&runs[1], 1u)] = (uint32_t)start;
+      continue;
+    }
+    int place[PER] = {};
+#pragma unroll
+    for (int b = 0; b < PER; ++b) {
+      for (int j = 32 * b; j < min(len, 32 * b + 32); ++j) {
+        const uint64_t other = __shfl_sync(FULL, k[b], j & 31);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) place[q] += (int)(other < k[q] || (other == k[q] && j < 32 * q + lane));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+      if (32 * q + lane < len) {
+        sorted[start + place[q]] = k[q];
+        perm[start + place[q]] = v[q];
+      }
+  }
+}
+
+// One CTA per run of more than RUN_MID elements. Up to RUN_RANKED elements: every element's place is the number of elements
+// before it. Longer ones: LSD passes over the run through the scratch arrays, an even number of them.
+__global__ void __launch_bounds__(RS_THREADS) k_long_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop,
+                                                          const uint32_t* __restrict__ runs, uint32_t runs_end,
+                                                          uint64_t* kalt, uint32_t* valt) {
+  __shared__ uint64_t sk[RUN_RANKED];
+  __shared__ uint32_t sv[RUN_RANKED];
+  __shared__ uint32_t base[RS_BINS], wc[RS_WARPS][RS_BINS], ws[SC_THREADS / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint64_t low = (1ull << drop) - 1ull;
+  for (uint32_t r = blockIdx.x; r < runs[1]; r += gridDim.x) {
+    const size_t start = runs[runs_end - 1 - r];
+    const uint64_t h = sorted[start] >> drop;
+    size_t len = 0;
+    for (int got = RS_THREADS; got == RS_THREADS; len += got) {
+      const size_t i = start + len + t;
+      got = __syncthreads_count(i < n && (sorted[i] >> drop) == h);
+    }
+    if (len <= (size_t)RUN_RANKED) {
+      for (int q = t; q < (int)len; q += RS_THREADS) {
+        sk[q] = sorted[start + q];
+        sv[q] = perm[start + q];
+      }
+      __syncthreads();
+      for (int q = t; q < (int)len; q += RS_THREADS) {
+        const uint64_t k = sk[q];
+        int place = 0;
+        for (int j = 0; j < (int)len; ++j) place += (int)(sk[j] < k || (sk[j] == k && j < q));
+        sorted[start + place] = k;
+        perm[start + place] = sv[q];
+      }
+      __syncthreads();
+      continue;
+    }
+    uint64_t *ka = sorted + start, *kb = kalt + start;
+    uint32_t *va = perm + start, *vb = valt + start;
+    const int passes = (drop + 15) / 16 * 2;
+    for (int p = 0; p < passes; ++p) {
+      const int shift = 8 * p;
+      base[t] = 0;
+      __syncthreads();
+      for (size_t i = t; i < len; i += RS_THREADS) atomicAdd(&base[(ka[i] & low) >> shift & (RS_BINS - 1)], 1u);
+      __syncthreads();
+      const uint32_t c = base[t];
+      uint32_t sum;
+      const uint32_t before = block_exclusive_scan(c, &sum, ws);
+      base[t] = before;
+      for (size_t i0 = 0; i0 < len; i0 += RS_THREADS) {  // in order, one element per thread
+        const size_t i = i0 + t;
+        const bool valid = i < len;
+        const uint64_t k = valid ? ka[i] : 0ull;
+        const uint32_t v = valid ? va[i] : 0u;
+        const uint32_t d = valid ? (uint32_t)((k & low) >> shift) & (RS_BINS - 1) : (0x100u | (uint32_t)lane);
+        const uint32_t peers = match_digit(d);
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) wc[w][t] = 0;
+        __syncthreads();
+        if (valid && (__ffs(peers) - 1) == lane) wc[warp][d] = (uint32_t)__popc(peers);
+        __syncthreads();
+        uint32_t run = base[t];  // thread t = digit t: where each warp's elements go
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) {
+          const uint32_t q = wc[w][t];
+          wc[w][t] = run;
+          run += q;
+        }
+        base[t] = run;
+        __syncthreads();
+        if (valid) {
+          const uint32_t pos = wc[warp][d] + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+          kb[pos] = k;
+          vb[pos] = v;
+        }
+        __syncthreads();
+      }
+      uint64_t* tk = ka;
+      ka = kb;
+      kb = tk;
+      uint32_t* tv = va;
+      va = vb;
+      vb = tv;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Small sorts: the passes over the keys' digits from `drop` up in one launch of one cluster. CTA c holds the c-th
+// contiguous part of the elements in registers (warps contiguous within it, rounds of 32 within
+// them), ranks them by digit as k_radix_scatter does, exchanges the digit totals with the other CTAs
+// through global memory and stores the elements where they go; a cluster barrier on either side.
+// ---------------------------------------------------------------------------------------------
+constexpr int SS_CTAS = 8;
+constexpr int SS_THREADS = 1024;
+constexpr int SS_WARPS = SS_THREADS / 32;
+constexpr int SS_ITEMS = 8;
+constexpr size_t SMALL_SORT = (size_t)SS_CTAS * SS_THREADS * SS_ITEMS;  // 65,536 keys
+
+__global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS)
+    k_sort_small(const uint64_t* __restrict__ keys, uint64_t* sorted, uint32_t* perm, uint64_t* kalt, uint32_t* valt,
+                 uint32_t* cta_hist, uint32_t n, int drop, int passes, uint32_t* runs) {
+  __shared__ uint32_t wc[SS_WARPS][RS_BINS];  // 32 KB
+  __shared__ uint32_t gbase[RS_BINS], ws[SS_WARPS];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t cta = blockIdx.x;
+  const uint32_t rounds = (n + SS_CTAS * SS_THREADS - 1) / (SS_CTAS * SS_THREADS);
+  const uint32_t first = ((cta * SS_WARPS + warp) * rounds) * 32 + lane;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  if (runs && cta == 0 && t < 2) runs[t] = 0;
   for (int p = 0; p < passes; ++p) {
+    // the last pass writes to `sorted`, the passes before it alternate
+    const bool to_sorted = ((passes - 1 - p) & 1) == 0;
+    const uint64_t* kin = p == 0 ? keys : (to_sorted ? kalt : sorted);
+    const uint32_t* vin = to_sorted ? valt : perm;
+    uint64_t* kout = to_sorted ? sorted : kalt;
+    uint32_t* vout = to_sorted ? perm : valt;
+    const int shift = drop + 8 * p;
+    for (int q = t; q < SS_WARPS * RS_BINS; q += SS_THREADS) (&wc[0][0])[q] = 0;
+    uint64_t k[SS_ITEMS];
+    uint32_t v[SS_ITEMS], rank[SS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SS_ITEMS; ++j) {
+      const uint32_t i = first + 32u * j;
+      const bool valid = j < (int)rounds && i < n;
+      k[j] = valid ? __ldcg(kin + i) : 0ull;
+      v[j] = valid ? (p == 0 ? i : __ldcg(vin + i)) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < SS_ITEMS; ++j) {
+      if (j >= (int)rounds) break;
+      const bool valid = first + 32u * j < n;
+      const uint32_t d = valid ? (uint32_t)(k[j] >> shift) & (RS_BINS - 1) : (0x100u | (uint32_t)lane);
+      const uint32_t peers = match_digit(d);
+      uint32_t prev = 0;
+      if (valid) prev = wc[warp][d];
+      __syncwarp();
+      rank[j] = prev + (uint32_t)__popc(peers & lt_mask);
+      if (valid && (__ffs(peers) - 1) == lane) wc[warp][d] = prev + (uint32_t)__popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    if (t < RS_BINS) {  // thread t = digit t: each warp's start within the CTA, the CTA's total
+      uint32_t run = 0;
+      for (int w = 0; w < SS_WARPS; ++w) {
+        const uint32_t c = wc[w][t];
+        wc[w][t] = run;
+        run += c;
+      }
+      __stcg(cta_hist + cta * RS_BINS + t, run);
+    }
+    cluster.sync();
+    uint32_t all = 0, before = 0;
+    if (t < RS_BINS)
+      for (uint32_t c = 0; c < SS_CTAS; ++c) {
+        const uint32_t x = __ldcg(cta_hist + c * RS_BINS + t);
+        all += x;
+        before += c < cta ? x : 0u;
+      }
+    uint32_t incl = all;  // exclusive scan of the digit totals over threads 0..255
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) ws[warp] = incl;
+    __syncthreads();
+    if (t < RS_BINS) {
+      uint32_t lead = 0;
+      for (int w = 0; w < warp; ++w) lead += ws[w];
+      gbase[t] = lead + incl - all + before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < SS_ITEMS; ++j)
+      if (j < (int)rounds && first + 32u * j < n) {
+        const uint32_t d = (uint32_t)(k[j] >> shift) & (RS_BINS - 1);
+        const uint32_t pos = gbase[d] + wc[warp][d] + rank[j];
+        __stcg(kout + pos, k[j]);
+        __stcg(vout + pos, v[j]);
+      }
+    cluster.sync();
+  }
+}
+
+cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* perm, size_t n, int bits,
+                            SortScratch& sc, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  if (n > 0xFFFFFFFFull || bits < 1 || bits > 64) return cudaErrorInvalidValue;
+  const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
+  cudaError_t e;
+  if ((e = ensure(sc.pairs, n * sizeof(uint2))) != cudaSuccess) return e;
+  if ((e = ensure(sc.pairs_alt, n * sizeof(uint2))) != cudaSuccess) return e;
+  const size_t hist_words = (size_t)RS_BINS * std::max(ntiles, SS_CTAS) + RS_BINS;
+  if ((e = ensure(sc.tile_hist, hist_words * sizeof(uint32_t))) != cudaSuccess) return e;
+  uint32_t* hist = as<uint32_t>(sc.tile_hist);
+  const bool small = n <= SMALL_SORT;
+  const int drop = std::max(0, bits - (small ? 24 : 32));
+  uint32_t* runs = nullptr;
+  // a listed run holds more than RUN_SHORT elements, one of the second list more than RUN_MID
+  const uint32_t runs_end = (uint32_t)(2 + n / (RUN_SHORT + 1) + n / (RUN_MID + 1) + 2);
+  if (drop) {
+    if ((e = ensure(sc.runs, (size_t)runs_end * sizeof(uint32_t))) != cudaSuccess) return e;
+    runs = as<uint32_t>(sc.runs);
+  }
+  uint2 *in = as<uint2>(sc.pairs), *out = as<uint2>(sc.pairs_alt);
+  uint32_t* totals = ntiles > RS_FEW ? hist + (size_t)RS_BINS * ntiles : nullptr;
+  const int passes = (bits - drop + 7) / 8;
+  if (small) {
+    count_launch();
+    k_sort_small<<<SS_CTAS, SS_THREADS, 0, s>>>(keys, sorted, perm, as<uint64_t>(sc.pairs), as<uint32_t>(sc.pairs_alt),
+                                                hist, (uint32_t)n, drop, passes, runs);
+  }
+  for (int p = 0; p < passes && !small; ++p) {
+    const bool first = p == 0, last = p == passes - 1;
     const int shift = 8 * p;
     count_launch();
-    k_radix_hist<<<nblocks, RS_THREADS, 0, s>>>(ka, n, shift, hist, nblocks);
-    if ((e = exclusive_scan_u32(hist, hist, (size_t)RS_BINS * nblocks, sc.scan_tmp, s)) != cudaSuccess) return e;
+    (first ? k_radix_hist<true> : k_radix_hist<false>)<<<ntiles, RS_THREADS, 0, s>>>(
+        keys, drop, in, n, shift, hist, ntiles, first ? runs : nullptr);
+    if (totals) {
+      count_launch();
+      k_radix_scan<<<RS_BINS, SC_THREADS, 0, s>>>(hist, ntiles, totals);
+    }
+    auto scatter = first ? (last ? k_radix_scatter<true, true> : k_radix_scatter<true, false>)
+                         : (last ? k_radix_scatter<false, true> : k_radix_scatter<false, false>);
     count_launch();
-    k_radix_scatter<<<nblocks, RS_THREADS, RS_SCATTER_SMEM, s>>>(ka, va, kb, vb, n, shift, hist, nblocks);
-    std::swap(ka, kb);
-    std::swap(va, vb);
+    scatter<<<ntiles, RS_THREADS, 0, s>>>(keys, drop, in, out, sorted, perm, n, shift, hist, totals, ntiles);
+    std::swap(in, out);
   }
-  if (ka != keys) {
-    if ((e = cudaMemcpyAsync(keys, ka, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(vals, va, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
+  if (drop) {
+    count_launch();
+    k_short_runs<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sorted, perm, n, drop, runs);
+    count_launch();
+    k_mid_runs<<<(unsigned)std::min<size_t>(n / 2048 + 1, 148 * 8), 256, 0, s>>>(sorted, perm, n, drop, runs, runs_end);
+    count_launch();
+    k_long_runs<<<148, RS_THREADS, 0, s>>>(sorted, perm, n, drop, runs, runs_end, as<uint64_t>(sc.pairs),
+                                           as<uint32_t>(sc.pairs_alt));
   }
   return cudaGetLastError();
 }

@@ -13,9 +13,11 @@
 // digits that still holds more than LEAF_SIZE particles stays a leaf (the reference would keep
 // splitting to depth 40); such nodes are counted.
 //
-// Centres of mass come from an FP64 exclusive prefix sum of the sorted positions: the sum over a
-// node is P[end] - P[start], divided by the count and rounded once to f32. (The reference sums
-// in f32 sequentially in input order; the difference is f32 round-off of that sum.)
+// Centres of mass are FP64 sums of the sorted positions over a node's range, divided by the count
+// and rounded once to f32. (The reference sums in f32 sequentially in input order; the difference is
+// f32 round-off of that sum.)
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <vector>
 
@@ -25,6 +27,8 @@ namespace cpm {
 
 constexpr int BUILD_THREADS = 256;
 constexpr int BUILD_BLOCKS = 148 * 4;
+constexpr int TOP_LEVEL = 4;             // the levels down to it are made in one launch
+constexpr size_t CLUSTER_TAIL = 262144;  // particles up to which the deep levels start early in one cluster
 
 // counters layout (u32): [0..KEY_LEVELS+1] per-level node counts (level 0 = root),
 // [32] nodes that hit the key-depth limit with > LEAF_SIZE particles, [33] max depth.
@@ -34,95 +38,156 @@ constexpr int CNT_WORDS = 64;
 
 __device__ __forceinline__ uint32_t digit_at(uint64_t key, int shift) { return (uint32_t)(key >> shift) & 7u; }
 
-// First index in [lo, hi) whose digit at `shift` is >= o, or hi if none (digits non-decreasing in
-// the range), found by the whole warp: each round probes 32 evenly spaced keys and keeps the
-// interval between the last probe below o and the first at or above it, so a range of c keys
-// takes about log32(c) rounds of one load per lane.
-__device__ __forceinline__ uint32_t warp_lower_bound(const uint64_t* __restrict__ keys, uint32_t lo, uint32_t hi,
-                                                     uint32_t o, int shift, int lane) {
+// The seven boundaries of a range [s, e) of more than 32 keys whose digits at `shift` do not decrease:
+// lane 4 o (o = 1..7) returns the first index whose digit is >= o (e if none). One round of 32 evenly
+// spaced probes narrows all of them to a 32nd of the range, then each group of four lanes narrows its own
+// to a fifth per round: a range of 32,768 keys takes 6 dependent loads instead of 21.
+__device__ __forceinline__ uint32_t warp_boundaries(const uint64_t* __restrict__ keys, uint32_t s, uint32_t e,
+                                                    int shift, int lane) {
   const unsigned FULL = 0xffffffffu;
-  while (hi - lo >= 32u) {
-    const uint32_t p = lo + (uint32_t)(((uint64_t)(hi - lo) * (uint32_t)lane) >> 5);  // p_0 = lo
-    const uint32_t ge = __ballot_sync(FULL, digit_at(__ldg(keys + p), shift) >= o);
-    if (ge & 1u) return lo;
-    const int j = ge ? __ffs(ge) - 1 : 32;  // first probe at or above o (32: none)
-    const uint32_t plo = __shfl_sync(FULL, p, j - 1);
-    const uint32_t phi = j < 32 ? __shfl_sync(FULL, p, j & 31) : hi;
-    lo = plo + 1u;
-    hi = phi;
+  const uint32_t o = (uint32_t)lane >> 2, c = e - s;
+  const uint32_t mine = digit_at(__ldg(keys + s + (uint32_t)(((uint64_t)c * (uint32_t)lane) >> 5)), shift);
+  uint32_t below = 0;  // probes with a digit below o: the boundary lies after the last of them
+#pragma unroll
+  for (uint32_t q = 1; q < 8; ++q) {
+    const uint32_t m = __ballot_sync(FULL, mine < q);
+    if (o == q) below = (uint32_t)__popc(m);
   }
-  const uint32_t p = lo + (uint32_t)lane;
-  const uint32_t ge = __ballot_sync(FULL, p >= hi || digit_at(__ldg(keys + p), shift) >= o);
-  return lo + (uint32_t)(__ffs(ge) - 1);  // lane hi - lo (< 32) always votes
-}
-
-// The root of every box (one box, or a batch of `roots` boxes of n_box particles each, sorted box by
-// box): node b covers the particles of box b, the cube [0, L]^3 of its own box.
-__global__ void k_tree_root(uint4* link, float4* geo, uint32_t* counters, uint32_t n, float half0, uint32_t roots,
-                            uint32_t n_box) {
-  for (uint32_t b = threadIdx.x; b < roots; b += blockDim.x) {
-    const uint32_t s0 = roots > 1 ? b * n_box : 0u, e0 = roots > 1 ? min(n, (b + 1) * n_box) : n;
-    link[b] = make_uint4(s0, e0, 0u, 0u);
-    geo[b] = make_float4(half0, half0, half0, half0);
+  uint32_t lo = s, hi = s;
+  if (o != 0u && below != 0u) {
+    lo = s + (uint32_t)(((uint64_t)c * (below - 1u)) >> 5) + 1u;
+    hi = below < 32u ? s + (uint32_t)(((uint64_t)c * below) >> 5) : e;
   }
-  if (threadIdx.x < CNT_WORDS) counters[threadIdx.x] = threadIdx.x == 0 ? roots : 0u;
-}
-
-// first index in [lo, hi) whose digit is >= o (digits non-decreasing in the range)
-__device__ __forceinline__ uint32_t lower_bound_digit(const uint64_t* __restrict__ keys, uint32_t lo, uint32_t hi,
-                                                      uint32_t o, int shift) {
-  while (lo < hi) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    if (digit_at(__ldg(keys + mid), shift) < o)
-      lo = mid + 1;
-    else
-      hi = mid;
+  while (__any_sync(FULL, lo < hi)) {
+    const uint32_t len = hi - lo, j = (uint32_t)lane & 3u;
+    const uint32_t p = lo + (uint32_t)(((uint64_t)len * (j + 1u)) / 5u);  // p < hi
+    const bool lt = lo < hi && digit_at(__ldg(keys + p), shift) < o;
+    const uint32_t k = (uint32_t)__popc((__ballot_sync(FULL, lt) >> (lane & ~3)) & 15u);  // probes below
+    const uint32_t nlo = k ? lo + (uint32_t)(((uint64_t)len * k) / 5u) + 1u : lo;
+    const uint32_t nhi = k < 4u ? lo + (uint32_t)(((uint64_t)len * (k + 1u)) / 5u) : hi;
+    if (lo < hi) {
+      lo = nlo;
+      hi = nhi;
+    }
   }
   return lo;
 }
 
-// Splits the nodes of level d. A level with more nodes than the grid has warps takes one node
-// per thread: the 8 octant sub-ranges by counting the digits d+1 of a small node's keys, or by
-// binary search on them in a larger one. A smaller level (the top
-// levels, and the sparse deep levels of clustered states), where a thread's searches would be
-// a long chain of dependent loads with little else in flight, takes one node per warp: nodes of
-// up to SMALL_NODE particles count the digits of all their keys (coalesced loads, a ballot per
-// octant), larger ones search the 7 boundaries with warp_lower_bound.
-constexpr uint32_t SMALL_NODE = 256;
-constexpr uint32_t SCAN_NODE = 64;  // thread path: nodes up to this size count their digits
+// The root of every box (one box, or a batch of `roots` boxes of n_box particles each, sorted box by
+// box): node b covers the particles of box b, the cube [0, L]^3 of its own box. One CTA.
+__device__ __forceinline__ void make_roots(uint4* link, float4* geo, uint32_t* counters, uint32_t n, float half0,
+                                           uint32_t roots, uint32_t n_box) {
+  for (uint32_t b = threadIdx.x; b < roots; b += blockDim.x) {
+    const uint32_t s0 = roots > 1 ? b * n_box : 0u, e0 = roots > 1 ? min(n, (b + 1) * n_box) : n;
+    __stcg(link + b, make_uint4(s0, e0, 0u, 0u));
+    __stcg(geo + b, make_float4(half0, half0, half0, half0));
+  }
+  if (threadIdx.x < CNT_WORDS) __stcg(counters + threadIdx.x, threadIdx.x == 0 ? roots : 0u);
+}
 
-// keys: the sort keys (octant or Hilbert digits split the node); okeys: the particles' octant keys
-// (a child's octant is the digit of its first particle; the same array as keys for octant order).
-__global__ void __launch_bounds__(BUILD_THREADS) k_tree_level(int d, int levels, const uint64_t* __restrict__ keys,
-                                                              const uint64_t* __restrict__ okeys, uint4* link,
-                                                              float4* geo, uint32_t* counters, uint32_t capacity,
-                                                              DevStatus* st) {
+// Splits the nodes of level d. A level with more nodes than the grid has warps takes one node
+// per thread: the 8 octant sub-ranges by counting the digits d+1 of a small node's keys, larger
+// nodes by the warp. A smaller level (the top levels, and the sparse deep levels of clustered
+// states) takes one node per warp.
+constexpr uint32_t SMALL_NODE = 256;
+constexpr uint32_t SCAN_NODE = 32;  // thread path: nodes up to this size count their digits
+
+// The octant of a position against a node's centre (tree.rs:186-190), the digit that the descent
+// gives it there.
+__device__ __forceinline__ uint32_t octant_of(const float4& x, const float4& G) {
+  return (uint32_t)(x.x >= G.x) | ((uint32_t)(x.y >= G.y) << 1) | ((uint32_t)(x.z >= G.z) << 2);
+}
+
+// The boundaries of a node's eight sub-ranges, by a warp: lane o (1..7) returns the first index whose
+// digit is >= o. Nodes of up to SMALL_NODE particles count the digits of all their keys (coalesced
+// loads, a ballot per octant).
+__device__ __forceinline__ uint32_t node_boundaries(const uint64_t* __restrict__ keys, uint32_t s, uint32_t e, int shift,
+                                                    int lane) {
+  const unsigned FULL = 0xffffffffu;
+  if (e - s > SMALL_NODE) {
+    const uint32_t bo = warp_boundaries(keys, s, e, shift, lane);
+    return __shfl_sync(FULL, bo, (lane & 7) * 4);
+  }
+  uint32_t below = 0;  // lane o: keys with digit < o
+  for (uint32_t i0 = s; i0 < e; i0 += 32) {
+    const uint32_t i = i0 + (uint32_t)lane;
+    const uint32_t dg = i < e ? digit_at(__ldg(keys + i), shift) : 8u;
+#pragma unroll
+    for (uint32_t o = 1; o < 8; ++o) {
+      const uint32_t bal = __ballot_sync(FULL, dg < o);
+      if ((uint32_t)lane == o) below += (uint32_t)__popc(bal);
+    }
+  }
+  return s + below;
+}
+
+// After a capacity failure: the counted nodes from `first` on that are still in the arrays become empty
+// leaves (the next levels read every counted node).
+__device__ __forceinline__ void clear_nodes(uint4* link, float4* geo, uint32_t first, uint32_t capacity) {
+  for (uint32_t q = first; q < min(first + 8u, capacity); ++q) {
+    __stcg(link + q, make_uint4(0u, 0u, 0u, 0u));
+    __stcg(geo + q, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+  }
+}
+
+// Room for the children of a CTA's nodes, `want` by this warp: one atomic per CTA and round on the
+// level's counter (one per warp, or per node on levels of a node per warp, come to 4,000 and more on one
+// address: 20 us a level at 91,125 clustered particles). Returns the warp's first.
+__device__ __forceinline__ uint32_t claim_nodes(uint32_t want, uint32_t* counter) {
+  __shared__ uint32_t part[32];
+  const unsigned FULL = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  if (lane == 0) part[warp] = want;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t v = lane < warps ? part[lane] : 0u;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    uint32_t base = 0;
+    if (lane == 31 && incl > 0u) base = atomicAdd(counter, incl);
+    base = __shfl_sync(FULL, base, 31);
+    if (lane < warps) part[lane] = base + incl - v;
+  }
+  __syncthreads();
+  return part[warp];
+}
+
+// keys: the sort keys (octant or Hilbert digits split the node); a child's octant is that of its
+// first particle.
+// lb, cnt: the level's first node and its size. The level is shared by nblocks CTAs, of which this is
+// number `block`; nodes are written and read past L1, since one launch may build several levels.
+__device__ __forceinline__ void split_level(int d, int levels, uint32_t lb, uint32_t cnt,
+                                            const uint64_t* __restrict__ keys, const float4* __restrict__ x4,
+                                            uint4* link, float4* geo, uint32_t* counters, uint32_t capacity,
+                                            DevStatus* st, uint32_t block, uint32_t nblocks) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  uint32_t lb = 0;
-  for (int j = 0; j < d; ++j) lb += counters[j];
-  const uint32_t cnt = counters[d];
   const uint32_t next_base = lb + cnt;
   // After a capacity failure the counters overshoot; never touch nodes past the arrays.
   const uint32_t level_end = min(next_base, capacity);
   const int shift = 3 * (levels - 1 - d);
-  const uint32_t warps = gridDim.x * (BUILD_THREADS / 32);
-  if (cnt > warps) {
-    // Thread per node; each warp allocates the children of its 32 nodes with one atomic (an
-    // atomic per node on the level's single counter serialises wide levels).
-    for (uint32_t base = lb + blockIdx.x * BUILD_THREADS + (threadIdx.x & ~31u); base < level_end;
-         base += gridDim.x * BUILD_THREADS) {
-      const uint32_t node = base + (uint32_t)lane;
+  const uint32_t warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  bool any_split = false;
+  if (cnt > nblocks * warps) {
+    // Thread per node. A warp's nodes are a stride apart: large nodes lie next to one another, and a
+    // warp takes its large ones in turn.
+    const uint32_t stride = nblocks * warps;
+    for (uint32_t base = lb + block * warps + warp; base - (block * warps + warp) < level_end; base += 32u * stride) {
+      const uint32_t node = base + (uint32_t)lane * stride;
       const bool valid = node < level_end;
-      const uint4 L = valid ? link[node] : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 L = valid ? __ldcg(link + node) : make_uint4(0u, 0u, 0u, 0u);
       const uint32_t s = L.x, e = L.y, c = e - s;
       bool split = false;
       if (valid) {
         if (c <= (uint32_t)LEAF_SIZE || d >= MAX_DEPTH) {
-          link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
+          __stcg(link + node, make_uint4(s, e, 0u, (uint32_t)d << 8));
         } else if (d >= levels) {
           atomicAdd(&counters[CNT_DEPTH_LIMIT], 1u);
-          link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
+          __stcg(link + node, make_uint4(s, e, 0u, (uint32_t)d << 8));
         } else {
           split = true;
         }
@@ -134,35 +199,44 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_tree_level(int d, int levels,
       if (split) {
         if (c <= SCAN_NODE) {
           // Small node: read its keys in order and count each digit (eight 8-bit counters in
-          // one word); a few sectors instead of the scattered probes of seven binary searches.
+          // one word); a few sectors instead of the scattered probes of a search.
           unsigned long long counts = 0ull;
+#pragma unroll 4
           for (uint32_t i = s; i < e; ++i) counts += 1ull << (8u * digit_at(__ldg(keys + i), shift));
 #pragma unroll
           for (int o = 1; o < 8; ++o) b[o] = b[o - 1] + (uint32_t)((counts >> (8 * (o - 1))) & 0xFFull);
-        } else {
-          uint32_t lo = s;
-#pragma unroll
-          for (uint32_t o = 1; o < 8; ++o) {
-            lo = lower_bound_digit(keys, lo, e, o, shift);
-            b[o] = lo;
-          }
         }
+      }
+      // The warp's larger nodes, one after another by the whole warp (a thread's own binary searches
+      // are 50 and more dependent loads).
+      for (uint32_t big = __ballot_sync(FULL, split && c > SCAN_NODE); big; big &= big - 1) {
+        const int owner = __ffs(big) - 1;
+        const uint32_t bo = node_boundaries(keys, __shfl_sync(FULL, s, owner), __shfl_sync(FULL, e, owner), shift, lane);
+#pragma unroll
+        for (int o = 1; o < 8; ++o) {
+          const uint32_t v = __shfl_sync(FULL, bo, o);
+          if (lane == owner) b[o] = v;
+        }
+      }
+      if (split) {
 #pragma unroll
         for (int o = 0; o < 8; ++o)
           if (b[o + 1] > b[o]) mask |= 1u << o;
       }
       // octant of each non-empty sub-range (its first particle's octant digit)
       uint32_t octmask = 0, octs = 0;
+      float4 G = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (split) {
+        G = __ldcg(geo + node);
 #pragma unroll
         for (int o = 0; o < 8; ++o)
           if (mask & (1u << o)) {
-            const uint32_t oc = okeys == keys ? (uint32_t)o : digit_at(__ldg(okeys + b[o]), shift);
+            const uint32_t oc = octant_of(__ldg(x4 + b[o]), G);
             octmask |= 1u << oc;
             octs |= oc << (3 * o);
           }
       }
-      // Children of the warp's nodes: an inclusive scan of their counts, one atomic by lane 31.
+      // Children of the warp's nodes: an inclusive scan of their counts.
       const uint32_t nch = (uint32_t)__popc(mask);
       uint32_t incl = nch;
 #pragma unroll
@@ -170,19 +244,16 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_tree_level(int d, int levels,
         const uint32_t y = __shfl_up_sync(FULL, incl, o);
         if (lane >= o) incl += y;
       }
-      uint32_t wbase = 0;
-      if (lane == 31 && incl > 0u) wbase = atomicAdd(&counters[d + 1], incl);
-      wbase = __shfl_sync(FULL, wbase, 31);
-      const uint32_t any_split = __ballot_sync(FULL, split);
-      if (lane == 0 && any_split != 0u) atomicMax(&counters[CNT_MAX_DEPTH], (uint32_t)(d + 1));
+      const uint32_t wbase = claim_nodes(__shfl_sync(FULL, incl, 31), &counters[d + 1]);
+      any_split |= split;
       if (!split) continue;
       const uint32_t first = next_base + wbase + incl - nch;
       if (first + nch > capacity) {
         dev_fail(st, DEV_NODE_CAPACITY, (int)(first + nch));
-        link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
+        __stcg(link + node, make_uint4(s, e, 0u, (uint32_t)d << 8));
+        clear_nodes(link, geo, first, capacity);
         continue;
       }
-      const float4 G = geo[node];
       const float q = G.w * 0.5f;  // half / 2.0
       uint32_t r = 0;
 #pragma unroll
@@ -190,89 +261,82 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_tree_level(int d, int levels,
         if (!(mask & (1u << o))) continue;
         const uint32_t child = first + r++;
         const uint32_t oc = (octs >> (3 * o)) & 7u;
-        link[child] = make_uint4(b[o], b[o + 1], 0u, 0u);
-        geo[child] = make_float4(__fadd_rn(G.x, (oc & 1) ? q : -q), __fadd_rn(G.y, (oc & 2) ? q : -q),
-                                 __fadd_rn(G.z, (oc & 4) ? q : -q), q);
+        __stcg(link + child, make_uint4(b[o], b[o + 1], 0u, 0u));
+        __stcg(geo + child, make_float4(__fadd_rn(G.x, (oc & 1) ? q : -q), __fadd_rn(G.y, (oc & 2) ? q : -q),
+                                 __fadd_rn(G.z, (oc & 4) ? q : -q), q));
       }
-      link[node] = make_uint4(s, e, first, octmask | ((uint32_t)d << 8));
+      __stcg(link + node, make_uint4(s, e, first, octmask | ((uint32_t)d << 8)));
     }
-    return;
-  }
-  for (uint32_t node = lb + blockIdx.x * (BUILD_THREADS / 32) + (threadIdx.x >> 5); node < level_end;
-       node += warps) {
-    const uint4 L = link[node];
-    const uint32_t s = L.x, e = L.y, c = e - s;
-    if (c <= (uint32_t)LEAF_SIZE || d >= MAX_DEPTH) {
-      if (lane == 0) link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
-      continue;
-    }
-    if (d >= levels) {
-      if (lane == 0) {
-        atomicAdd(&counters[CNT_DEPTH_LIMIT], 1u);
-        link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
+  } else {
+    // Warp per node.
+    for (uint32_t base = lb + block * warps; base < level_end; base += nblocks * warps) {
+      const uint32_t node = base + warp;
+      const uint4 L = node < level_end ? __ldcg(link + node) : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t s = L.x, e = L.y, c = e - s;
+      const bool split = c > (uint32_t)LEAF_SIZE && d < MAX_DEPTH && d < levels;
+      if (lane == 0 && node < level_end && !split) {
+        if (c > (uint32_t)LEAF_SIZE && d < MAX_DEPTH) atomicAdd(&counters[CNT_DEPTH_LIMIT], 1u);
+        __stcg(link + node, make_uint4(s, e, 0u, (uint32_t)d << 8));
       }
-      continue;
-    }
-    uint32_t bo = s;  // lane o (1..7): first index whose digit is >= o
-    if (c <= SMALL_NODE) {
-      uint32_t below = 0;  // lane o: keys with digit < o
-      for (uint32_t i0 = s; i0 < e; i0 += 32) {
-        const uint32_t i = i0 + (uint32_t)lane;
-        const uint32_t dg = i < e ? digit_at(__ldg(keys + i), shift) : 8u;
-#pragma unroll
-        for (uint32_t o = 1; o < 8; ++o) {
-          const uint32_t bal = __ballot_sync(FULL, dg < o);
-          if ((uint32_t)lane == o) below += (uint32_t)__popc(bal);
+      // Lane o < 8: octant o's range [olo, ohi) (lane o >= 1: first index whose digit is >= o).
+      uint32_t olo = 0, ohi = 0;
+      if (split) {
+        const uint32_t bo = node_boundaries(keys, s, e, shift, lane);
+        const uint32_t nb = __shfl_sync(FULL, bo, (lane + 1) & 31);
+        olo = lane == 0 ? s : bo;
+        ohi = lane == 7 ? e : nb;
+      }
+      const uint32_t mask = __ballot_sync(FULL, lane < 8 && ohi > olo);
+      const uint32_t nch = (uint32_t)__popc(mask);
+      const uint32_t first = next_base + claim_nodes(nch, &counters[d + 1]);
+      any_split |= split;
+      if (!split) continue;
+      if (first + nch > capacity) {
+        if (lane == 0) {
+          dev_fail(st, DEV_NODE_CAPACITY, (int)(first + nch));
+          __stcg(link + node, make_uint4(s, e, 0u, (uint32_t)d << 8));
+          clear_nodes(link, geo, first, capacity);
         }
+        continue;
       }
-      bo = s + below;
-    } else {
-      uint32_t lo = s;
-      for (uint32_t o = 1; o < 8; ++o) {
-        lo = warp_lower_bound(keys, lo, e, o, shift, lane);
-        if ((uint32_t)lane == o) bo = lo;
+      // lane o: the octant of sub-range o (its first particle's octant digit)
+      const bool live = lane < 8 && ((mask >> lane) & 1u);
+      const float4 G = __ldcg(geo + node);
+      const uint32_t oc = live ? octant_of(__ldg(x4 + olo), G) : 0u;
+      const uint32_t octmask = __reduce_or_sync(FULL, live ? 1u << oc : 0u);
+      if (live) {
+        const float q = G.w * 0.5f;  // half / 2.0
+        const uint32_t child = first + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+        __stcg(link + child, make_uint4(olo, ohi, 0u, 0u));
+        __stcg(geo + child, make_float4(__fadd_rn(G.x, (oc & 1) ? q : -q), __fadd_rn(G.y, (oc & 2) ? q : -q),
+                                        __fadd_rn(G.z, (oc & 4) ? q : -q), q));
       }
-    }
-    // Lane o < 8: octant o's range [olo, ohi) (b[0] = s, b[8] = e).
-    const uint32_t nb = __shfl_sync(FULL, bo, (lane + 1) & 31);
-    const uint32_t olo = lane == 0 ? s : bo, ohi = lane == 7 ? e : nb;
-    const uint32_t mask = __ballot_sync(FULL, lane < 8 && ohi > olo);
-    const uint32_t nch = (uint32_t)__popc(mask);
-    uint32_t first = 0;
-    if (lane == 0) first = next_base + atomicAdd(&counters[d + 1], nch);
-    first = __shfl_sync(FULL, first, 0);
-    if (first + nch > capacity) {
-      if (lane == 0) {
-        dev_fail(st, DEV_NODE_CAPACITY, (int)(first + nch));
-        link[node] = make_uint4(s, e, 0u, (uint32_t)d << 8);
-      }
-      continue;
-    }
-    // lane o: the octant of sub-range o (its first particle's octant digit)
-    const bool live = lane < 8 && ((mask >> lane) & 1u);
-    const uint32_t oc = !live ? 0u : (okeys == keys ? (uint32_t)lane : digit_at(__ldg(okeys + olo), shift));
-    const uint32_t octmask = __reduce_or_sync(FULL, live ? 1u << oc : 0u);
-    if (live) {
-      const float4 G = geo[node];
-      const float q = G.w * 0.5f;  // half / 2.0
-      const uint32_t child = first + (uint32_t)__popc(mask & ((1u << lane) - 1u));
-      link[child] = make_uint4(olo, ohi, 0u, 0u);
-      geo[child] = make_float4(__fadd_rn(G.x, (oc & 1) ? q : -q), __fadd_rn(G.y, (oc & 2) ? q : -q),
-                               __fadd_rn(G.z, (oc & 4) ? q : -q), q);
-    }
-    if (lane == 0) {
-      link[node] = make_uint4(s, e, first, octmask | ((uint32_t)d << 8));
-      atomicMax(&counters[CNT_MAX_DEPTH], (uint32_t)(d + 1));
+      if (lane == 0) __stcg(link + node, make_uint4(s, e, first, octmask | ((uint32_t)d << 8)));
     }
   }
+  if (__syncthreads_or(any_split) && threadIdx.x == 0) atomicMax(&counters[CNT_MAX_DEPTH], (uint32_t)(d + 1));
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS) k_tree_level(int d, int levels, const uint64_t* __restrict__ keys,
+                                                              const float4* __restrict__ x4, uint4* link,
+                                                              float4* geo, uint32_t* counters, uint32_t capacity,
+                                                              DevStatus* st) {
+  uint32_t lb = 0;
+  for (int j = 0; j < d; ++j) lb += counters[j];
+  split_level(d, levels, lb, counters[d], keys, x4, link, geo, counters, capacity, st, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------
-// FP64 exclusive prefix sums of sorted positions: P[i] = sum_{j<i} x_j, P[n] = total.
+// Centres of mass: FP64 sums of the sorted positions over each node's range. A node of up to
+// SUM_DIRECT particles adds them itself; a larger one takes the difference of prefix sums, kept per
+// CHUNK of particles (the partial chunk at either end is added by the node), chunk prefixes within
+// tiles of CHUNKS_PER_TILE and tile prefixes apart. A prefix sum per particle instead (24 bytes each)
+// cost 0.49 ms of FP64 stores and reads at 256^3 particles.
 // ---------------------------------------------------------------------------------------------
-constexpr int PS_THREADS = 256;
-constexpr int PS_ITEMS = 8;
-constexpr int PS_TILE = PS_THREADS * PS_ITEMS;
+constexpr uint32_t SUM_DIRECT = 32;
+constexpr uint32_t CHUNK = 32;
+constexpr uint32_t CHUNKS_PER_TILE = 32;
+constexpr uint32_t SUM_TILE = CHUNK * CHUNKS_PER_TILE;
 
 struct D3 {
   double x, y, z;
@@ -284,108 +348,295 @@ __device__ __forceinline__ D3 shfl_up_d3(D3 v, int o) {
             __shfl_up_sync(0xffffffffu, v.z, o)};
 }
 
-// Block-wide exclusive scan of D3 (per-thread partial), returns the thread's prefix and the total.
-__device__ __forceinline__ D3 block_scan_d3(D3 v, D3* total, D3* ws) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  D3 x = v;
+// Sum of the positions a .. b - 1.
+__device__ __forceinline__ D3 sum_range(const float4* __restrict__ x4, uint32_t a, uint32_t b) {
+  D3 s{0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (uint32_t i = a; i < b; ++i) {
+    const float4 x = __ldg(x4 + i);
+    s = d3add(s, D3{(double)x.x, (double)x.y, (double)x.z});
+  }
+  return s;
+}
+
+// Inclusive scan over the warp.
+__device__ __forceinline__ D3 warp_scan_d3(D3 x, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const D3 y = shfl_up_d3(x, o);
     if (lane >= o) x = d3add(x, y);
   }
-  if (lane == 31) ws[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    D3 w = lane < PS_THREADS / 32 ? ws[lane] : D3{0.0, 0.0, 0.0};
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const D3 y = shfl_up_d3(w, o);
-      if (lane >= o) w = d3add(w, y);
-    }
-    if (lane < PS_THREADS / 32) ws[lane] = w;
-  }
-  __syncthreads();
-  const D3 wp = warp ? ws[warp - 1] : D3{0.0, 0.0, 0.0};
-  *total = ws[PS_THREADS / 32 - 1];
-  return D3{wp.x + x.x - v.x, wp.y + x.y - v.y, wp.z + x.z - v.z};
+  return x;
 }
 
-__global__ void __launch_bounds__(PS_THREADS) k_pos_reduce(const float* __restrict__ x3, size_t n, D3* partial) {
-  __shared__ D3 ws[PS_THREADS / 32];
-  const size_t base = (size_t)blockIdx.x * PS_TILE + (size_t)threadIdx.x * PS_ITEMS;
-  D3 s{0.0, 0.0, 0.0};
-#pragma unroll
-  for (int j = 0; j < PS_ITEMS; ++j) {
-    const size_t i = base + j;
-    if (i < n) s = d3add(s, D3{(double)x3[3 * i], (double)x3[3 * i + 1], (double)x3[3 * i + 2]});
-  }
-  D3 total;
-  block_scan_d3(s, &total, ws);
-  if (threadIdx.x == 0) partial[blockIdx.x] = total;
+// One warp per tile: lane c sums chunk c, then the exclusive scan over the tile's chunks and the
+// tile's total.
+__device__ __forceinline__ void sum_tile(const float4* __restrict__ x4, uint32_t n, uint32_t tile, D3* chunk,
+                                         D3* totals) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t i0 = min(n, tile * SUM_TILE + (uint32_t)lane * CHUNK), i1 = min(n, i0 + CHUNK);
+  const D3 s = sum_range(x4, i0, i1);
+  const D3 incl = warp_scan_d3(s, lane);
+  chunk[(size_t)tile * CHUNKS_PER_TILE + lane] = D3{incl.x - s.x, incl.y - s.y, incl.z - s.z};
+  if (lane == 31) totals[tile] = incl;
 }
 
-// Exclusive scan of the block partials in one block (sequential chunks of PS_THREADS).
-__global__ void __launch_bounds__(PS_THREADS) k_partial_scan(D3* partial, size_t nb) {
-  __shared__ D3 ws[PS_THREADS / 32];
+__global__ void __launch_bounds__(BUILD_THREADS) k_sum_tiles(const float4* __restrict__ x4, uint32_t n, D3* chunk,
+                                                             D3* totals, uint32_t tiles) {
+  for (uint32_t t = blockIdx.x * (BUILD_THREADS / 32) + (threadIdx.x >> 5); t < tiles;
+       t += gridDim.x * (BUILD_THREADS / 32))
+    sum_tile(x4, n, t, chunk, totals);
+}
+
+// Exclusive scan of the tile totals in place, one CTA of up to 1024 threads, four tiles per thread and
+// round.
+__device__ __forceinline__ void scan_tiles(D3* totals, uint32_t tiles, D3* ws) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   D3 carry{0.0, 0.0, 0.0};
-  for (size_t c0 = 0; c0 < nb; c0 += PS_THREADS) {
-    const size_t i = c0 + threadIdx.x;
-    const D3 v = i < nb ? partial[i] : D3{0.0, 0.0, 0.0};
-    D3 total;
-    const D3 ex = block_scan_d3(v, &total, ws);
-    if (i < nb) partial[i] = d3add(carry, ex);
-    carry = d3add(carry, total);
+  for (uint32_t c0 = 0; c0 < tiles; c0 += 4 * blockDim.x) {
+    const uint32_t i = c0 + 4 * threadIdx.x;
+    D3 v[4], sum{0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      v[q] = i + q < tiles ? totals[i + q] : D3{0.0, 0.0, 0.0};
+      sum = d3add(sum, v[q]);
+    }
+    const D3 x = warp_scan_d3(sum, lane);
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      const D3 w = warp_scan_d3(lane < warps ? ws[lane] : D3{0.0, 0.0, 0.0}, lane);
+      if (lane < warps) ws[lane] = w;
+    }
+    __syncthreads();
+    D3 run = d3add(carry, D3{x.x - sum.x, x.y - sum.y, x.z - sum.z});
+    if (warp) run = d3add(run, ws[warp - 1]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (i + q < tiles) totals[i + q] = run;
+      run = d3add(run, v[q]);
+    }
+    carry = d3add(carry, ws[warps - 1]);
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(PS_THREADS) k_pos_prefix(const float* __restrict__ x3, size_t n,
-                                                           const D3* __restrict__ partial, double* P) {
-  __shared__ D3 ws[PS_THREADS / 32];
-  const size_t base = (size_t)blockIdx.x * PS_TILE + (size_t)threadIdx.x * PS_ITEMS;
-  D3 v[PS_ITEMS];
-  D3 s{0.0, 0.0, 0.0};
-#pragma unroll
-  for (int j = 0; j < PS_ITEMS; ++j) {
-    const size_t i = base + j;
-    v[j] = i < n ? D3{(double)x3[3 * i], (double)x3[3 * i + 1], (double)x3[3 * i + 2]} : D3{0.0, 0.0, 0.0};
-    s = d3add(s, v[j]);
+// The prefix sum of the whole chunks before particle i.
+__device__ __forceinline__ D3 chunk_prefix(const D3* chunk, const D3* totals, uint32_t c) {
+  return d3add(totals[c / CHUNKS_PER_TILE], chunk[c]);
+}
+
+// Centre of mass of one node, and NODE_FLAT for an inner node whose children all have no octant-0
+// child (bit 0 of the mask, which the flag's store leaves as it is for the parents that read it).
+__device__ __forceinline__ void finish_node(uint32_t node, uint4* link, const float4* __restrict__ x4, const D3* chunk,
+                                            const D3* totals, float4* mass) {
+  const uint4 L = __ldcg(link + node);
+  D3 s;
+  if (L.y - L.x <= SUM_DIRECT) {
+    s = sum_range(x4, L.x, L.y);
+  } else {
+    const uint32_t c0 = (L.x + CHUNK - 1) / CHUNK, c1 = L.y / CHUNK;  // whole chunks c0 .. c1 - 1
+    const D3 p0 = chunk_prefix(chunk, totals, c0), p1 = chunk_prefix(chunk, totals, c1);
+    s = d3add(D3{p1.x - p0.x, p1.y - p0.y, p1.z - p0.z},
+              d3add(sum_range(x4, L.x, c0 * CHUNK), sum_range(x4, c1 * CHUNK, L.y)));
   }
-  D3 total;
-  D3 run = d3add(block_scan_d3(s, &total, ws), partial[blockIdx.x]);
-#pragma unroll
-  for (int j = 0; j < PS_ITEMS; ++j) {
-    const size_t i = base + j;
-    if (i <= n) {
-      P[3 * i] = run.x;
-      P[3 * i + 1] = run.y;
-      P[3 * i + 2] = run.z;
-    }
-    run = d3add(run, v[j]);
+  const double c = (double)(L.y - L.x);
+  mass[node] = make_float4((float)(s.x / c), (float)(s.y / c), (float)(s.z / c), (float)(L.y - L.x));
+  if (L.w & 1u) {
+    const uint32_t nch = (uint32_t)__popc(L.w & 0xFFu);
+    uint32_t any = 0;
+    for (uint32_t q = 0; q < nch; ++q) any |= __ldcg(&link[L.z + q].w);
+    if ((any & 1u) == 0u) __stcg(&link[node].w, L.w | NODE_FLAT);
   }
 }
 
-// Centres of mass, and NODE_FLAT for the inner nodes whose children all have no octant-0 child (bit
-// 0 of the mask, which the flag's store leaves as it is for the parents that read it).
-__global__ void k_tree_com(uint4* link, const double* __restrict__ P, float4* mass,
-                           const uint32_t* __restrict__ counters, uint32_t capacity) {
+__global__ void __launch_bounds__(BUILD_THREADS) k_tree_com(uint4* link, const float4* __restrict__ x4, const D3* chunk,
+                                                            const D3* totals, float4* mass,
+                                                            const uint32_t* __restrict__ counters, uint32_t capacity) {
   uint32_t total = 0;
   for (int j = 0; j <= KEY_LEVELS; ++j) total += counters[j];
   total = min(total, capacity);
-  for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < total; node += gridDim.x * blockDim.x) {
-    const uint4 L = link[node];
-    const double c = (double)(L.y - L.x);
-    const double sx = P[3 * (size_t)L.y] - P[3 * (size_t)L.x];
-    const double sy = P[3 * (size_t)L.y + 1] - P[3 * (size_t)L.x + 1];
-    const double sz = P[3 * (size_t)L.y + 2] - P[3 * (size_t)L.x + 2];
-    mass[node] = make_float4((float)(sx / c), (float)(sy / c), (float)(sz / c), (float)(L.y - L.x));
-    if (L.w & 1u) {
-      const uint32_t nch = (uint32_t)__popc(L.w & 0xFFu);
-      uint32_t any = 0;
-      for (uint32_t q = 0; q < nch; ++q) any |= *(volatile uint32_t*)&link[L.z + q].w;
-      if ((any & 1u) == 0u) *(volatile uint32_t*)&link[node].w = L.w | NODE_FLAT;
-    }
+  for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < total; node += gridDim.x * blockDim.x)
+    finish_node(node, link, x4, chunk, totals, mass);
+}
+
+// The top of a single box's tree: CTA 0 finds where each of the 8^TOP_LEVEL cells of level TOP_LEVEL
+// starts in the sorted keys (all searches at once), from which the nodes of the levels above follow
+// without another look at the keys, and makes them down to level TOP_LEVEL. The other CTAs form the
+// prefix sums' tiles meanwhile. As a level per launch, or per barrier of one cluster, the same
+// levels are a chain of searches: 60 us at 32,768 particles.
+constexpr int TOP_CELLS = 1 << (3 * TOP_LEVEL);
+constexpr int TOP_THREADS = 1024;
+constexpr int TOP_PARENTS = TOP_CELLS / 8;  // nodes of the last level that is split here
+__global__ void __launch_bounds__(TOP_THREADS) k_tree_top(int levels, const uint64_t* __restrict__ keys,
+                                                          const float4* __restrict__ x4, uint32_t n, float half0,
+                                                          uint4* link, float4* geo, uint32_t* counters,
+                                                          uint32_t capacity, D3* chunk, D3* totals, uint32_t tiles,
+                                                          DevStatus* st) {
+  if (blockIdx.x > 0) {
+    for (uint32_t t = (blockIdx.x - 1) * (TOP_THREADS / 32) + (threadIdx.x >> 5); t < tiles;
+         t += (gridDim.x - 1) * (TOP_THREADS / 32))
+      sum_tile(x4, n, t, chunk, totals);
+    return;
   }
+  __shared__ uint32_t start[TOP_CELLS + 1];
+  __shared__ uint16_t prefix[2][TOP_PARENTS];  // of the level's nodes
+  __shared__ float4 centre[2][TOP_PARENTS];
+  __shared__ uint32_t ws[TOP_THREADS / 32];
+  static_assert(TOP_PARENTS <= TOP_THREADS && TOP_PARENTS <= 65536, "a thread per node");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  {
+    // The first key of cell q or after: seven probes a round, a thread's cells side by side.
+    constexpr int PER = TOP_CELLS / TOP_THREADS;
+    const int shift = 3 * (levels - TOP_LEVEL);
+    uint32_t lo[PER], hi[PER];
+#pragma unroll
+    for (int c = 0; c < PER; ++c) {
+      lo[c] = 0;
+      hi[c] = n;
+    }
+    for (uint32_t left = n; left > 0; left >>= 3) {  // a round leaves an eighth of the range
+#pragma unroll
+      for (int c = 0; c < PER; ++c) {
+        const uint32_t len = hi[c] - lo[c], q = (uint32_t)(t + c * TOP_THREADS);
+        uint32_t k = 0;
+        if (len) {
+#pragma unroll
+          for (uint32_t j = 1; j < 8; ++j)
+            k += (uint32_t)((__ldg(keys + lo[c] + (uint32_t)(((uint64_t)len * j) >> 3)) >> shift) < (uint64_t)q);
+        }
+        const uint32_t nlo = k ? lo[c] + (uint32_t)(((uint64_t)len * k) >> 3) + 1u : lo[c];
+        if (k < 7u) hi[c] = lo[c] + (uint32_t)(((uint64_t)len * (k + 1u)) >> 3);
+        lo[c] = nlo;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < PER; ++c) start[t + c * TOP_THREADS] = lo[c];
+    if (t == 0) start[TOP_CELLS] = n;
+  }
+  if (t < CNT_WORDS) __stcg(counters + t, t == 0 ? 1u : 0u);
+  if (t == 0) {
+    prefix[0][0] = 0;
+    centre[0][0] = make_float4(half0, half0, half0, half0);
+    geo[0] = centre[0][0];
+    link[0] = make_uint4(0u, n, 0u, 0u);
+  }
+  __syncthreads();
+  uint32_t lb = 0, cnt = 1;
+  for (int d = 0; d < TOP_LEVEL && cnt; ++d) {
+    const int cur = d & 1, below = 3 * (TOP_LEVEL - 1 - d);  // a child's cells: 2^below
+    uint32_t b[9], mask = 0;
+    bool split = false;
+    const uint32_t node = lb + (uint32_t)t;
+    uint32_t p = 0;
+    float4 G = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if ((uint32_t)t < cnt) {
+      p = prefix[cur][t];
+      G = centre[cur][t];
+#pragma unroll
+      for (int o = 0; o < 9; ++o) b[o] = start[((p << 3) + o) << below];
+      split = b[8] - b[0] > (uint32_t)LEAF_SIZE;
+      if (split) {
+#pragma unroll
+        for (int o = 0; o < 8; ++o)
+          if (b[o + 1] > b[o]) mask |= 1u << o;
+      }
+    }
+    const uint32_t nch = (uint32_t)__popc(mask);
+    uint32_t incl = nch;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) ws[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int w = 0; w < TOP_THREADS / 32; ++w) {
+      before += w < warp ? ws[w] : 0u;
+      total += ws[w];
+    }
+    const uint32_t base = lb + cnt, slot = before + incl - nch, first = base + slot;
+    if ((uint32_t)t < cnt) {
+      uint32_t octmask = 0, r = 0;
+      if (split && first + nch > capacity) {
+        dev_fail(st, DEV_NODE_CAPACITY, (int)(first + nch));
+        clear_nodes(link, geo, first, capacity);
+        split = false;
+      }
+      if (split) {
+        const float q = G.w * 0.5f;  // half / 2.0
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+          if (!(mask & (1u << o))) continue;
+          const uint32_t oc = octant_of(__ldg(x4 + b[o]), G);
+          const float4 C = make_float4(__fadd_rn(G.x, (oc & 1) ? q : -q), __fadd_rn(G.y, (oc & 2) ? q : -q),
+                                       __fadd_rn(G.z, (oc & 4) ? q : -q), q);
+          octmask |= 1u << oc;
+          link[first + r] = make_uint4(b[o], b[o + 1], 0u, 0u);
+          geo[first + r] = C;
+          if (d + 1 < TOP_LEVEL) {
+            prefix[cur ^ 1][slot + r] = (uint16_t)((p << 3) + o);
+            centre[cur ^ 1][slot + r] = C;
+          }
+          ++r;
+        }
+        link[node] = make_uint4(b[0], b[8], first, octmask | ((uint32_t)d << 8));
+      } else {
+        link[node] = make_uint4(b[0], b[8], 0u, (uint32_t)d << 8);
+      }
+    }
+    if (t == 0 && total) {
+      counters[d + 1] = total;
+      counters[CNT_MAX_DEPTH] = (uint32_t)(d + 1);
+    }
+    __syncthreads();
+    lb += cnt;
+    cnt = lb + total <= capacity ? total : 0u;
+  }
+}
+
+// Levels first .. last of the build by one cluster of CTAs in one launch, a level per cluster barrier,
+// ending at the deepest level there is: the top levels of a batch, and the levels below every node of a
+// smooth distribution, of which a clustered one has some and a smooth one none (as launches of their
+// own they are 2 to 4 us each). first = 0 also makes the roots; with `chunk` one CTA scans the tile
+// totals.
+constexpr int CLUSTER_CTAS = 8;
+constexpr int CLUSTER_THREADS = 1024;
+__global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
+    k_tree_cluster(int first, int last, int levels, const uint64_t* __restrict__ keys, const float4* __restrict__ x4,
+                   uint32_t n, float half0, uint32_t roots, uint32_t n_box, uint4* link, float4* geo,
+                   uint32_t* counters, uint32_t capacity, D3* totals, uint32_t tiles, DevStatus* st) {
+  __shared__ D3 ws[32];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const uint32_t block = blockIdx.x;
+  if (first == 0) {
+    if (block == 0) make_roots(link, geo, counters, n, half0, roots, n_box);
+    cluster.sync();
+  }
+  if (totals && block == CLUSTER_CTAS - 1) scan_tiles(totals, tiles, ws);
+  uint32_t lb = 0;
+  for (int d = 0; d < first; ++d) lb += __ldcg(counters + d);
+  for (int d = first; d <= last; ++d) {
+    const uint32_t cnt = __ldcg(counters + d);
+    if (cnt == 0) break;
+    split_level(d, levels, lb, cnt, keys, x4, link, geo, counters, capacity, st, block, CLUSTER_CTAS);
+    lb += cnt;
+    cluster.sync();
+  }
+}
+
+// Packs AoS positions into float4 (x, y, z, 0); words[WALK_OUTSIDE] becomes 1 when a position lies
+// outside [0, L] (zeroed by the caller).
+__global__ void k_pack4(const float* __restrict__ x3, size_t n, float box, float4* __restrict__ x4,
+                        uint32_t* __restrict__ words) {
+  bool out = false;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const float a = x3[3 * i], b = x3[3 * i + 1], c = x3[3 * i + 2];
+    x4[i] = make_float4(a, b, c, 0.0f);
+    out |= outside_box(a, b, c, box);
+  }
+  if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31) == 0) words[WALK_OUTSIDE] = 1u;
 }
 
 // Second moments about the centre of mass, T = sum_j (x_j - com)(x_j - com)^T over the node's
@@ -427,9 +678,23 @@ __global__ void k_tree_quad(const uint4* __restrict__ link, const float4* __rest
   }
 }
 
+cudaError_t tree_positions(TreeNodes& t, size_t n, cudaStream_t s) {
+  cudaError_t e = ensure(t.x4, (n + 1) * sizeof(float4));
+  if (e != cudaSuccess) return e;
+  return cudaMemsetAsync(tree_words(t, n), 0, sizeof(float4), s);
+}
+
+cudaError_t tree_pack(TreeNodes& t, const float* sorted_x3, size_t n, float box, cudaStream_t s) {
+  cudaError_t e = tree_positions(t, n, s);
+  if (e != cudaSuccess || n == 0) return e;
+  count_launch();
+  k_pack4<<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, s>>>(sorted_x3, n, box, as<float4>(t.x4),
+                                                                               tree_words(t, n));
+  return cudaGetLastError();
+}
+
 cudaError_t tree_build(TreeNodes& t, const uint64_t* sorted_keys, const float* sorted_x3, size_t n, float box,
-                       DevStatus* st, cudaStream_t s, float quad_half_max, int levels, size_t n_box,
-                       const uint64_t* octant_keys) {
+                       DevStatus* st, cudaStream_t s, float quad_half_max, int levels, size_t n_box) {
   if (n == 0) return cudaSuccess;
   const size_t cap = 2 * n + 64;
   cudaError_t e;
@@ -440,39 +705,49 @@ cudaError_t tree_build(TreeNodes& t, const uint64_t* sorted_keys, const float* s
     t.capacity = cap;
   }
   if ((e = ensure(t.counters, CNT_WORDS * sizeof(uint32_t))) != cudaSuccess) return e;
-  if ((e = ensure(t.prefix, 3 * (n + 1) * sizeof(double))) != cudaSuccess) return e;
-  const size_t nb = (n + 1 + PS_TILE - 1) / PS_TILE;
-  if ((e = ensure(t.scan_tmp, (nb + 1) * sizeof(D3))) != cudaSuccess) return e;
+  const uint32_t tiles = (uint32_t)(n / SUM_TILE + 1);  // the last one may be empty: prefixes up to n
+  if ((e = ensure(t.prefix, (size_t)tiles * (CHUNKS_PER_TILE + 1) * sizeof(D3))) != cudaSuccess) return e;
 
   uint4* link = as<uint4>(t.link);
-  float4* geo = as<float4>(t.geo);
+  float4 *geo = as<float4>(t.geo), *mass = as<float4>(t.mass);
   uint32_t* counters = as<uint32_t>(t.counters);
+  D3 *chunk = as<D3>(t.prefix), *totals = chunk + (size_t)tiles * CHUNKS_PER_TILE;
+  const uint32_t roots = n_box ? (uint32_t)((n + n_box - 1) / n_box) : 1u, capacity = (uint32_t)t.capacity;
+  const float4* x4 = as<float4>(t.x4);
+  // The cells of level `spread` are about as many as the particles, so that a smooth distribution has
+  // nothing to split below it; a clustered one has, fewer and fewer: their first levels still fill
+  // launches (1.0 ms of 2.4 at 256^3 clustered particles went into one cluster from level spread + 3 on).
+  int spread = 0;
+  for (size_t c = n; c > 1; c >>= 3) ++spread;
+  const int tail = std::min(levels, std::max(TOP_LEVEL + 1, spread + (n > CLUSTER_TAIL ? 6 : 3)));
   count_launch();
-  const uint32_t roots = n_box ? (uint32_t)((n + n_box - 1) / n_box) : 1u;
-  k_tree_root<<<1, 256, 0, s>>>(link, geo, counters, (uint32_t)n, box / 2.0f, roots, (uint32_t)n_box);
-  for (int d = 0; d <= levels; ++d) {
+  if (roots == 1) {
+    const unsigned sums = std::min(148u, (tiles + TOP_THREADS / 32 - 1) / (TOP_THREADS / 32));
+    k_tree_top<<<1 + sums, TOP_THREADS, 0, s>>>(levels, sorted_keys, x4, (uint32_t)n, box / 2.0f, link, geo, counters,
+                                                capacity, chunk, totals, tiles, st);
+  } else {
+    k_tree_cluster<<<CLUSTER_CTAS, CLUSTER_THREADS, 0, s>>>(0, TOP_LEVEL - 1, levels, sorted_keys, x4, (uint32_t)n,
+                                                            box / 2.0f, roots, (uint32_t)n_box, link, geo, counters,
+                                                            capacity, nullptr, 0, st);
     count_launch();
-    k_tree_level<<<BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(d, levels, sorted_keys,
-                                                        octant_keys ? octant_keys : sorted_keys, link, geo,
-                                                        counters, (uint32_t)t.capacity, st);
+    k_sum_tiles<<<BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(x4, (uint32_t)n, chunk, totals, tiles);
   }
-
-  D3* partial = as<D3>(t.scan_tmp);
-  double* P = as<double>(t.prefix);
+  for (int d = TOP_LEVEL; d < tail; ++d) {
+    count_launch();
+    k_tree_level<<<BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(d, levels, sorted_keys, x4, link, geo, counters, capacity, st);
+  }
   count_launch();
-  k_pos_reduce<<<(unsigned)nb, PS_THREADS, 0, s>>>(sorted_x3, n, partial);
+  k_tree_cluster<<<CLUSTER_CTAS, CLUSTER_THREADS, 0, s>>>(tail, levels, levels, sorted_keys, x4, (uint32_t)n, box / 2.0f,
+                                                          roots, (uint32_t)n_box, link, geo, counters, capacity, totals,
+                                                          tiles, st);
   count_launch();
-  k_partial_scan<<<1, PS_THREADS, 0, s>>>(partial, nb);
-  count_launch();
-  k_pos_prefix<<<(unsigned)nb, PS_THREADS, 0, s>>>(sorted_x3, n, partial, P);
-  count_launch();
-  k_tree_com<<<BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, P, as<float4>(t.mass), counters, (uint32_t)t.capacity);
+  k_tree_com<<<2 * BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, x4, chunk, totals, mass, counters, capacity);
   t.has_quad = quad_half_max > 0.0f;
   if (t.has_quad) {
     if ((e = ensure(t.quad, 2 * t.capacity * sizeof(float4))) != cudaSuccess) return e;
     count_launch();
     k_tree_quad<<<BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, geo, as<float4>(t.mass), sorted_x3, as<float4>(t.quad),
-                                                       counters, (uint32_t)t.capacity, quad_half_max);
+                                                       counters, capacity, quad_half_max);
   }
   return cudaGetLastError();
 }

@@ -74,7 +74,6 @@ constexpr int WINDOW = 448;   // direct-sum sources collected before they are su
 // whose warps each repeat the traversal.
 constexpr size_t WALK_FILL = 148 * 96;
 constexpr int WALK_WARPS_PER_SM = 20;  // resident warps the register budget is set for
-constexpr int WALK_OUTSIDE = 0, WALK_TICKET = 1;  // the walk's words: see k_pack4, the group counter
 constexpr int STAGE = 64;     // candidate sources fetched at a time, two per lane
 constexpr uint32_t FIRST_BITS = 29;  // a stack entry: first node (29 bits) | (count - 1) << 29
 constexpr int FIT_DEG = 12;
@@ -948,19 +947,6 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
   }
 }
 
-// Packs AoS positions into float4 (x, y, z, 0) for 16-byte loads; words[WALK_OUTSIDE] becomes 1 when
-// a position lies outside [0, L] (the walk's words are zeroed by the caller).
-__global__ void k_pack4(const float* __restrict__ x3, size_t n, float box, float4* __restrict__ x4,
-                        uint32_t* __restrict__ words) {
-  bool out = false;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float a = x3[3 * i], b = x3[3 * i + 1], c = x3[3 * i + 2];
-    x4[i] = make_float4(a, b, c, 0.0f);
-    out |= !(fminf(a, fminf(b, c)) >= 0.0f && fmaxf(a, fmaxf(b, c)) <= box);
-  }
-  if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31) == 0) words[WALK_OUTSIDE] = 1u;
-}
-
 // ------------------------------------------------------------------ host launch
 
 // Fitted pair-force coefficients of one tree's last split (refitted when the split changes; a
@@ -982,7 +968,7 @@ void tree_walk_free(TreeNodes& t) {
   t.walk_fit = nullptr;
 }
 
-void launch_tree_walk(const TreeNodes& t, const float* sorted_x3, size_t n, float box, const cpm_force_split& split,
+void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_split& split,
                       float k, float* acc3, int accumulate, TreeCounters* counters, DevStatus* st, cudaStream_t s,
                       const float* k_dev, const uint32_t* list, const uint32_t* list_n) {
   if (n == 0) return;
@@ -996,13 +982,7 @@ void launch_tree_walk(const TreeNodes& t, const float* sorted_x3, size_t n, floa
     fc.r_split = split.r_split;
     fc.r_cut = split.r_cut;
   }
-  // the packed positions, then the walk's words
-  if (ensure(tm.x4, (n + 1) * sizeof(float4)) != cudaSuccess) return;
-  uint32_t* words = reinterpret_cast<uint32_t*>(as<float4>(tm.x4) + n);
-  cudaMemsetAsync(words, 0, sizeof(float4), s);
-  const unsigned pb = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
-  count_launch();
-  k_pack4<<<pb, 256, 0, s>>>(sorted_x3, n, box, as<float4>(tm.x4), words);
+  uint32_t* words = tree_words(tm, n);
 
   WalkParams w;
   w.box = box;
@@ -1047,6 +1027,7 @@ void launch_tree_walk(const TreeNodes& t, const float* sorted_x3, size_t n, floa
   const size_t smem = (size_t)warps * (sizeof(WalkShared) + (t.has_quad ? SLOTS * sizeof(uint32_t) : 0));
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (team == 1) {  // as many blocks as fit on the chip at once
+    cudaMemsetAsync(words + WALK_TICKET, 0, sizeof(uint32_t), s);
     int per_sm = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem) == cudaSuccess && per_sm > 0)
       blocks = std::min(blocks, (unsigned)per_sm * 148u);
