@@ -147,15 +147,24 @@ __global__ void k_step_factors64(StepScalars* dev, cpm_cosmology c, double a0, d
                                  double net_per_cell_h) {
   // integrator.rs:273-285: the scale factor where the kick integral is half its total
   const double half = 0.5 * simpson_warp64(c, a0, a1, 0);
-  double lo = a0, hi = a1;
+  double lo = a0, hi = a1, am = 0.5 * (a0 + a1);
   for (int it = 0; it < 60; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (simpson_warp64(c, a0, mid, 0) < half)
-      lo = mid;
+    const double f = simpson_warp64(c, a0, am, 0) - half;
+    if (f < 0.0)
+      lo = am;
     else
-      hi = mid;
+      hi = am;
+    double next = 0.5 * (lo + hi);
+    if (a1 > a0) {
+      // Newton's method, the integrand being the derivative, kept inside the bracket: about 4 integrals
+      // of the warp in a row instead of 60, which took 0.25 ms. (For a step back in time the
+      // reference's bisection runs to one end of the interval, and so does this one.)
+      const double newton = am - f * am * cosmo_e64(c, am);
+      if (newton >= lo && newton <= hi) next = newton;
+      if (fabs(next - am) <= 4.0e-16 * am) break;
+    }
+    am = next;
   }
-  const double am = 0.5 * (lo + hi);
   const double k1 = simpson_warp64(c, a0, am, 0), k2 = simpson_warp64(c, am, a1, 0);
   const double d = simpson_warp64(c, a0, a1, 1);
   if ((threadIdx.x & 31) == 0) {
