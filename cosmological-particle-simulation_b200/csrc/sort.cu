@@ -367,9 +367,8 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DevB
 // CTA, whatever its length (a rank count in shared memory, or for runs over RUN_RANKED LSD passes over
 // the run). Eight passes of (u64 key, u32 index) moved 3.2 GB at 256^3 instead of 1.1.
 //
-// Per pass: digit counts per tile of 4096 (digit-major), their exclusive scan (one CTA per digit; with
-// up to RS_FEW tiles every tile of the scatter adds its digits' few counts itself), then a stable
-// scatter. Within a tile each warp ranks a contiguous sub-tile in warp-striped rounds (lanes with
+// Per pass: digit counts per tile of 4096 (digit-major), their exclusive scan (one CTA per digit), then
+// a stable scatter. Within a tile each warp ranks a contiguous sub-tile in warp-striped rounds (lanes with
 // equal digits found by ballots), so equal digits keep their input order.
 //
 // Up to SMALL_SORT keys go through the passes of their upper 24 bits in one launch of one cluster of
@@ -380,7 +379,6 @@ constexpr int RS_ITEMS = 16;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
-constexpr int RS_FEW = 64;
 static_assert(RS_THREADS == RS_BINS, "one thread per digit");
 
 // The lanes whose 9-bit value d equals this lane's (a digit, or 0x100 | lane for a lane without
@@ -483,19 +481,8 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __
     if (i < n) e[j] = FIRST ? make_uint2((uint32_t)(keys[i] >> drop), (uint32_t)i) : in[i];
   }
   // Thread t = digit t: where its elements of this tile start in the output.
-  uint32_t before = 0, all = 0;
-  if (totals) {
-    before = tile_hist[(size_t)t * ntiles + blockIdx.x];
-    all = totals[t];
-  } else {
-    for (int q = 0; q < ntiles; ++q) {
-      const uint32_t c = tile_hist[(size_t)t * ntiles + q];
-      all += c;
-      before += q < (int)blockIdx.x ? c : 0u;
-    }
-  }
   uint32_t sum;
-  before += block_exclusive_scan(all, &sum, ws);
+  const uint32_t before = tile_hist[(size_t)t * ntiles + blockIdx.x] + block_exclusive_scan(totals[t], &sum, ws);
 #pragma unroll
   for (int j = 0; j < RS_ITEMS; ++j) {
     const bool valid = wbase + (size_t)j * 32 + lane < n;
@@ -836,7 +823,7 @@ cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* pe
     runs = as<uint32_t>(sc.runs);
   }
   uint2 *in = as<uint2>(sc.pairs), *out = as<uint2>(sc.pairs_alt);
-  uint32_t* totals = ntiles > RS_FEW ? hist + (size_t)RS_BINS * ntiles : nullptr;
+  uint32_t* totals = hist + (size_t)RS_BINS * ntiles;
   const int passes = (bits - drop + 7) / 8;
   if (small) {
     count_launch();
@@ -849,10 +836,8 @@ cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* pe
     count_launch();
     (first ? k_radix_hist<true> : k_radix_hist<false>)<<<ntiles, RS_THREADS, 0, s>>>(
         keys, drop, in, n, shift, hist, ntiles, first ? runs : nullptr);
-    if (totals) {
-      count_launch();
-      k_radix_scan<<<RS_BINS, SC_THREADS, 0, s>>>(hist, ntiles, totals);
-    }
+    count_launch();
+    k_radix_scan<<<RS_BINS, SC_THREADS, 0, s>>>(hist, ntiles, totals);
     auto scatter = first ? (last ? k_radix_scatter<true, true> : k_radix_scatter<true, false>)
                          : (last ? k_radix_scatter<false, true> : k_radix_scatter<false, false>);
     count_launch();

@@ -27,7 +27,7 @@ namespace cpm {
 
 constexpr int BUILD_THREADS = 256;
 constexpr int BUILD_BLOCKS = 148 * 4;
-constexpr int TOP_LEVEL = 4;             // the levels down to it are made in one launch
+constexpr int TOP_LEVEL = 3;             // the levels down to it are made in one launch
 constexpr size_t CLUSTER_TAIL = 262144;  // particles up to which the deep levels start early in one cluster
 
 // counters layout (u32): [0..KEY_LEVELS+1] per-level node counts (level 0 = root),
@@ -464,9 +464,10 @@ __global__ void __launch_bounds__(BUILD_THREADS) k_tree_com(uint4* link, const f
 // starts in the sorted keys (all searches at once), from which the nodes of the levels above follow
 // without another look at the keys, and makes them down to level TOP_LEVEL. The other CTAs form the
 // prefix sums' tiles meanwhile. As a level per launch, or per barrier of one cluster, the same
-// levels are a chain of searches: 60 us at 32,768 particles.
+// levels are a chain of searches: 60 us at 32,768 particles. (One level more, 4096 cells, is 44 us: its
+// probes are more than one SM fetches quickly.)
 constexpr int TOP_CELLS = 1 << (3 * TOP_LEVEL);
-constexpr int TOP_THREADS = 1024;
+constexpr int TOP_THREADS = 512;
 constexpr int TOP_PARENTS = TOP_CELLS / 8;  // nodes of the last level that is split here
 __global__ void __launch_bounds__(TOP_THREADS) k_tree_top(int levels, const uint64_t* __restrict__ keys,
                                                           const float4* __restrict__ x4, uint32_t n, float half0,
