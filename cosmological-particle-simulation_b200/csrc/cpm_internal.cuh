@@ -173,7 +173,9 @@ struct FftPlan {
   DevBuf twiddle;  // exp(-2 pi i m / n), m < n, float2 built from double
   DevBuf deconv;   // per-axis 1 / sinc^4(pi m / n): CIC window of deposit and gather, squared
 };
-// Elements of one half spectrum [n][n][n/2+2] (one padding column per row).
+// Row pitch of a half spectrum: n/2 + 1 columns in whole 32-byte sectors.
+__host__ __device__ constexpr int half_row(int n) { return (n / 2 + 1 + 3) / 4 * 4; }
+// Elements of one half spectrum [n][n][half_row(n)].
 size_t half_spectrum_elems(int n);
 cudaError_t fft_plan_init(FftPlan& p, int n);
 void fft_plan_free(FftPlan& p);
@@ -192,7 +194,7 @@ struct PoissonParams {
 };
 // Input: either f32 delta (delta != nullptr) or the u64 fixed-point mass mesh (fx != nullptr,
 // converted to delta = c/mean - 1 on load). Output: three f32 meshes. spec: 3 half spectra
-// of n*n*(n/2+1) float2 each; slot 0 also holds the forward spectrum.
+// of n*n*half_row(n) float2 each; slot 0 also holds the forward spectrum.
 void launch_poisson(const FftPlan& p, const PoissonParams& pp, const float* delta, const unsigned long long* fx,
                     int fx_shift, float mean, float2* spec, float* gx, float* gy, float* gz, cudaStream_t s);
 

@@ -2,22 +2,23 @@
 //
 // Layouts in HBM
 //   real mesh      f32  [n][n][n]            (ix*n + iy)*n + iz, z fastest (mesh.rs:11)
-//   half spectrum  c32  [n][n][n/2+2]        kz in [0, n/2]; one padding column keeps rows 16-byte
-//                                            aligned; the rest of kz follows from Hermitian symmetry
+//   half spectrum  c32  [n][n][half_row(n)]  kz in [0, n/2], rows padded to whole 32-byte sectors; the
+//                                            rest of kz follows from Hermitian symmetry
 //
-// Every pass moves tiles of W = 16 lines between HBM and shared memory once. In shared memory
-// element t of line l sits at t*(W+1) + l ("transposed", line index fastest):
-//   - FFT stages give the line index to consecutive lanes, so each half-warp touches 16
-//     consecutive elements (one 128-byte row) whatever the stage's stride: no bank conflicts;
-//   - transfers of contiguous z rows give t to consecutive lanes; the odd stride W+1 spreads those
-//     16 elements over all banks, again without conflicts;
-//   - transfers of strided y/x lines give the line (the contiguous kz column) to consecutive
-//     lanes, so global accesses are 128-byte rows.
-// Each pass is a persistent kernel that walks its tiles with two shared-memory buffers: while one
-// tile is transformed, the next one streams in with cp.async, so HBM stays busy during the
-// shared-memory work. Lines are transformed by radix-8/4/2 Stockham stages in place (each stage
-// reads its butterflies into registers, synchronises, writes them to their autosorted positions).
+// Every pass reads and writes each of its spectra once (the y gradient pass the potential twice, from
+// L2), in tiles of 8 or 16 lines, one tile per CTA. Lines are transformed by radix-8/4/2/3/5 Stockham stages; the
+// first takes its inputs straight from global memory into registers, the last stores its outputs there, and
+// shared memory carries the exchanges between them.
+//   - Strided y/x lines: the line (the contiguous kz column) is on consecutive lanes, in global memory
+//     (64 or 128 contiguous bytes) and in the exchanges (no bank conflicts whatever the stage's stride).
+//   - Contiguous z rows: the first and last stage run along the row on consecutive lanes.
 // Twiddles come from a table exp(-2 pi i m / n) built in double precision on the host.
+//
+// What bounds them: at n = 512 (no pass fits L2) the five passes take 0.48 (R2C, 3.3 TB/s), 0.23 (y, 4.4),
+// 0.72 (x, 2.2), 0.82 (y gradient, 3.6) and 0.77 ms (C2R, 4.2), together 3.02: the first and last by
+// shared-memory and L1 wavefronts (81 % in C2R), the x pass by issue and barriers (three transforms and the Green's
+// function per line). As persistent kernels that copied tiles in by cp.async, transformed them in place and copied
+// them out they took 3.97 (256: 0.489, now 0.400; 128: 0.092, now 0.067).
 //
 // Real z lines use the half-length complex transform: z[m] = x[2m] + i x[2m+1] is transformed
 // with n/2 points and split into the n/2+1 outputs with the twiddles of length n (and the
@@ -42,12 +43,7 @@
 
 namespace cpm {
 
-constexpr int TW = 16;       // lines per tile
-constexpr int TLD = TW + 1;  // shared-memory row pitch (elements)
-constexpr size_t SMEM_LIMIT = 227 * 1024;
-
-template <int L, int MR = 8>
-constexpr int threads_for();
+constexpr int TW = 16;  // lines per tile, unless said otherwise
 
 // ---------------------------------------------------------------------------------------------
 // Complex helpers and small DFTs
@@ -141,60 +137,6 @@ __device__ __forceinline__ void dft(float2* v) {
   else dft8<INV>(v);
 }
 
-// One Stockham stage of radix R on the TW lines of a tile (element t of line l at t*TLD + l),
-// T threads. Twiddle exp(-2 pi i m / N) is tw[m * TS] (TS = 2 when the table is for length 2N).
-// NT = 2 transforms a second tile (sm1) in the same stage: one pair of barriers and one set of
-// twiddle loads serve both.
-template <int N, int R, int NS, bool INV, int T, int TS, int NT = 1>
-__device__ __forceinline__ void stockham_stage(float2* sm0, float2* sm1, const float2* __restrict__ tw) {
-  constexpr int NB = N / R;
-  constexpr int TOTAL = TW * NB;
-  constexpr int BPT = (TOTAL + T - 1) / T;
-  float2 v[NT][BPT][R];
-#pragma unroll
-  for (int q = 0; q < BPT; ++q) {
-    const int b = threadIdx.x + q * T;
-    if (TOTAL % T == 0 || b < TOTAL) {
-      const int l = b % TW, j = b / TW;
-#pragma unroll
-      for (int p = 0; p < NT; ++p) {
-        const float2* sm = p ? sm1 : sm0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[p][q][r] = sm[(j + r * NB) * TLD + l];
-      }
-      if constexpr (NS > 1) {
-        const int k = j % NS;
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 w = __ldg(tw + r * k * (N / (NS * R)) * TS);
-          if (INV) w.y = -w.y;
-#pragma unroll
-          for (int p = 0; p < NT; ++p) v[p][q][r] = cmul(v[p][q][r], w);
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < NT; ++p) dft<R, INV>(v[p][q]);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < BPT; ++q) {
-    const int b = threadIdx.x + q * T;
-    if (TOTAL % T == 0 || b < TOTAL) {
-      const int l = b % TW, j = b / TW;
-      const int k = j % NS;
-      const int base = (j / NS) * NS * R + k;
-#pragma unroll
-      for (int p = 0; p < NT; ++p) {
-        float2* sm = p ? sm1 : sm0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) sm[(base + r * NS) * TLD + l] = v[p][q][r];
-      }
-    }
-  }
-  __syncthreads();
-}
-
 // Radix of the next Stockham stage for a remaining length L = 2^a 3^b 5^c under a plan whose
 // largest radix is MR: MR = 8 takes 8 while it divides, then 4 or 2, then 3s, then 5s (512 = 8.8.8);
 // MR = 4 takes 4 while it divides, then 2, 3s, 5s (512 = 4.4.4.4.2). The autotuner picks the plan.
@@ -205,214 +147,14 @@ constexpr int next_radix() {
   else
     return L % 4 == 0 ? 4 : (L % 2 == 0 ? 2 : (L % 3 == 0 ? 3 : 5));
 }
-constexpr bool smooth235(int n) {
-  if (n <= 0) return false;
-  while (n % 2 == 0) n /= 2;
-  while (n % 3 == 0) n /= 3;
-  while (n % 5 == 0) n /= 5;
-  return n == 1;
-}
-
-template <int N, int NS, bool INV, int T, int TS, int MR, int NT = 1>
-__device__ __forceinline__ void fft_stages(float2* sm0, float2* sm1, const float2* __restrict__ tw) {
-  if constexpr (NS < N) {
-    constexpr int R = next_radix<N / NS, MR>();
-    stockham_stage<N, R, NS, INV, T, TS, NT>(sm0, sm1, tw);
-    fft_stages<N, NS * R, INV, T, TS, MR, NT>(sm0, sm1, tw);
-  }
-}
-
 // ---------------------------------------------------------------------------------------------
-// Warp-per-line plan (MR = 0) for N = 256 and 512: warp w transforms line w of the tile by itself,
-// with three register stages of radix R1, R2, R3 (N = R1 R2 R3; 8.8.8 and 4.8.8) and two exchanges
-// through the line's own shared-memory elements, synchronised with __syncwarp only. With
-// n = s + S1 r (S1 = N / R1), s = sa + R3 sb, k = k1 + R1 (k2 + R2 k3):
-//   A: Y[s][k1]   = w_N^(s k1)     sum_r  x[s + S1 r] w_R1^(r k1)        stored at s + S1 k1
-//   B: Z[sa][k2]  = w_S1^(sa k2)   sum_sb Y[sa + R3 sb][k1] w_R2^(sb k2)  stored at sa + R3 k2 + S1 k1
-//   C: X[k]       =                sum_sa Z[sa][k2] w_R3^(sa k3)         stored at k (natural order)
-// Element t of the line sits in bank pair (t + l) mod 16 (pitch TW + 1 = 17 float2), so an access is
-// conflict-free when the 16 lanes of each half-warp hold distinct t mod 16. The lanes of stages B
-// and C take their inputs in an order rotated per lane so that this holds (B: by k1 mod 2; C: by
-// k1 + 4 ((k2 / 2) mod 2), mod 8), and put the values back in place with register selects.
-template <int N>
-struct WarpPlan {
-  static constexpr bool ok = false;
-};
-template <>
-struct WarpPlan<512> {
-  static constexpr bool ok = true;
-  static constexpr int R1 = 8, R2 = 8, R3 = 8;
-};
-template <>
-struct WarpPlan<256> {
-  static constexpr bool ok = true;
-  static constexpr int R1 = 4, R2 = 8, R3 = 8;
-};
-
-// Threads of a CTA that transforms TW lines of length L: one warp per line for the warp plan, else
-// about one radix-8 butterfly each, a multiple of 32 in 256..1024.
-template <int L, int MR>
-constexpr int threads_for() {
-  if constexpr (MR == 0 && WarpPlan<L>::ok) {
-    return 32 * TW;
-  } else {
-    constexpr int t = (TW * L / 8 + 31) / 32 * 32;
-    return t < 256 ? 256 : (t > 1024 ? 1024 : t);
-  }
-}
-
-template <bool INV>
-__device__ __forceinline__ float2 twiddle(const float2* __restrict__ tw, int idx) {
-  float2 w = __ldg(tw + idx);
-  if (INV) w.y = -w.y;
-  return w;
-}
-
-// v[j] = u[(j - k) mod R] when `on` (a rotation of the array by k places), else unchanged
-template <int R, int K>
-__device__ __forceinline__ void rotate_if(float2 (&v)[R], bool on) {
-  float2 u[R];
-#pragma unroll
-  for (int j = 0; j < R; ++j) u[j] = v[j];
-#pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const float2 a = u[(j - K + R) % R];
-    v[j].x = on ? a.x : u[j].x;
-    v[j].y = on ? a.y : u[j].y;
-  }
-}
-
-template <int N, bool INV, int TS>
-__device__ __forceinline__ void warp_fft_line(float2* sm, int l, const float2* __restrict__ tw) {
-  using P = WarpPlan<N>;
-  constexpr int R1 = P::R1, R2 = P::R2, R3 = P::R3, S1 = N / R1;
-  static_assert(R2 == 8 && R3 == 8 && S1 == 64, "plans with S1 = 64 = 8 x 8");
-  const int lane = threadIdx.x & 31;
-  float2* line = sm + l;
-  // A: columns s = lane + 32 q
-  {
-    constexpr int QA = S1 / 32;
-    float2 v[QA][R1];
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int s = lane + 32 * q;
-#pragma unroll
-      for (int r = 0; r < R1; ++r) v[q][r] = line[(s + S1 * r) * TLD];
-      dft<R1, INV>(v[q]);
-#pragma unroll
-      for (int k1 = 1; k1 < R1; ++k1) v[q][k1] = cmul(v[q][k1], twiddle<INV>(tw, s * k1 * TS));
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int s = lane + 32 * q;
-#pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) line[(s + S1 * k1) * TLD] = v[q][k1];
-    }
-    __syncwarp();
-  }
-  // B: pairs p = lane + 32 q -> (sa = p % R3, k1 = p / R3); lanes with odd k1 rotate sb by one
-  {
-    constexpr int QB = R3 * R1 / 32;
-    float2 v[QB][R2];
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int p = lane + 32 * q, sa = p % R3, k1 = p / R3, rho = k1 & 1;
-#pragma unroll
-      for (int i = 0; i < R2; ++i) v[q][i] = line[(sa + R3 * ((i + rho) % R2) + S1 * k1) * TLD];
-      rotate_if<R2, 1>(v[q], rho);  // v[sb]
-      dft<R2, INV>(v[q]);
-#pragma unroll
-      for (int k2 = 1; k2 < R2; ++k2) v[q][k2] = cmul(v[q][k2], twiddle<INV>(tw, R1 * sa * k2 * TS));
-      rotate_if<R2, R2 - 1>(v[q], rho);  // v[i] = Z[(i + rho) % R2]
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int p = lane + 32 * q, sa = p % R3, k1 = p / R3, rho = k1 & 1;
-#pragma unroll
-      for (int i = 0; i < R2; ++i) line[(sa + R3 * ((i + rho) % R2) + S1 * k1) * TLD] = v[q][i];
-    }
-    __syncwarp();
-  }
-  // C: pairs p = lane + 32 q -> (k1 = p % R1, k2 = p / R1); lane rotation rho of sa
-  {
-    constexpr int QC = R1 * R2 / 32;
-    float2 v[QC][R3];
-#pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      const int p = lane + 32 * q, k1 = p % R1, k2 = p / R1, rho = (k1 + 4 * ((k2 >> 1) & 1)) & 7;
-#pragma unroll
-      for (int i = 0; i < R3; ++i) v[q][i] = line[(((i + rho) & 7) + R3 * k2 + S1 * k1) * TLD];
-      rotate_if<R3, 1>(v[q], rho & 1);
-      rotate_if<R3, 2>(v[q], rho & 2);
-      rotate_if<R3, 4>(v[q], rho & 4);  // v[sa]
-      dft<R3, INV>(v[q]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      const int p = lane + 32 * q, k1 = p % R1, k2 = p / R1;
-#pragma unroll
-      for (int k3 = 0; k3 < R3; ++k3) line[(k1 + R1 * k2 + R1 * R2 * k3) * TLD] = v[q][k3];
-    }
-  }
-}
-
-// Full length-N transform of the tile (N = 2^a 3^b 5^c) with the radix plan MR (MR = 0: the
-// warp-per-line plan where it exists, else the radix-8 Stockham plan).
-template <int N, bool INV, int T, int TS = 1, int MR = 8>
-__device__ __forceinline__ void fft_lines(float2* sm, const float2* __restrict__ tw) {
-  static_assert(N >= 2 && N <= 1024 && smooth235(N), "lengths 2..1024 with prime factors 2, 3, 5");
-  if constexpr (MR == 0 && WarpPlan<N>::ok) {
-    static_assert(T == 32 * TW, "one warp per line");
-    warp_fft_line<N, INV, TS>(sm, threadIdx.x >> 5, tw);
-    __syncthreads();
-  } else {
-    fft_stages<N, 1, INV, T, TS, (MR == 0 ? 8 : MR)>(sm, sm, tw);
-  }
-}
-
-// Two independent tiles transformed together (the same length and direction).
-template <int N, bool INV, int T, int TS = 1, int MR = 8>
-__device__ __forceinline__ void fft_lines2(float2* a, float2* b, const float2* __restrict__ tw) {
-  if constexpr (MR == 0 && WarpPlan<N>::ok) {
-    static_assert(T == 32 * TW, "one warp per line");
-    warp_fft_line<N, INV, TS>(a, threadIdx.x >> 5, tw);
-    warp_fft_line<N, INV, TS>(b, threadIdx.x >> 5, tw);
-    __syncthreads();
-  } else {
-    fft_stages<N, 1, INV, T, TS, (MR == 0 ? 8 : MR), 2>(a, b, tw);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Asynchronous global -> shared copies (cp.async, completion tracked per thread by groups)
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory");
-}
-
-// ---------------------------------------------------------------------------------------------
-// Tile geometry. Strided passes: element t of column c of tile (o, ct) is at
-//   o * outer_stride + (ct * TW + c) + t * elem_stride   (columns contiguous in memory).
-// Row passes: tile r covers rows r*TW .. r*TW + TW - 1, each contiguous.
+// Geometry of a strided pass: element t of column c of outer index o is at
+//   o * outer_stride + c + t * elem_stride   (columns contiguous in memory).
 // ---------------------------------------------------------------------------------------------
 struct ColGeo {
   long long outer_stride;
   long long elem_stride;
   int cols;       // valid columns along the contiguous axis
-  int col_tiles;  // ceil(cols / TW)
   int outer;      // number of outer indices (over every box of a batch)
   int per_box = 0;            // outer indices per box when a batch's boxes are not one linear run
   long long box_stride = 0;   // elements between the boxes of such a batch
@@ -423,386 +165,457 @@ struct ColGeo {
   __host__ __device__ int in_box(int o) const { return per_box ? o % per_box : o; }
 };
 
-// Row transfers: chunks of TT = min(L, 16) consecutive t go to consecutive lanes, chunk-major
-// over the TW rows: work item q -> (t, l) with t < L, l < TW.
-template <int L>
-__device__ __forceinline__ int row_t(int q) {
-  constexpr int TT = L < 16 ? L : 16;
-  return (q % TT) + TT * (q / (TT * TW));
+// ---------------------------------------------------------------------------------------------
+// Transforms from and to global memory. The first Stockham stage takes its inputs straight from
+// global memory into registers and the last one stores its outputs there, so shared memory only
+// carries the exchanges between the stages (element t of line l at tile_at(t, l)): for 512 = 8.8.8
+// two writes and two reads of the tile and four barriers. Nothing is staged ahead: a CTA issues all of
+// a tile's loads at once, and two or more CTAs per SM overlap their loads, stages and stores.
+// ---------------------------------------------------------------------------------------------
+// The extra element after every 8 rows spreads the 16 lanes of a stage that runs along a line (JFAST
+// below), whose writes are 8 rows apart, over all banks.
+// (Tiles of 8 lines: an extra row after every 8, for the two rows that a half-warp touches.)
+template <int W = TW>
+__device__ __forceinline__ int tile_at(int t, int l) {
+  static_assert(W == 16 || W == 8, "tiles of 16 or 8 lines");
+  return W == 16 ? t * 17 + (t >> 3) + l : (t + (t >> 3)) * 8 + l;
 }
-template <int L>
-__device__ __forceinline__ int row_l(int q) {
-  constexpr int TT = L < 16 ? L : 16;
-  return (q / TT) % TW;
-}
-// Work items that cover t < count on every row.
-template <int L>
-__device__ __forceinline__ int row_span(int count) {
-  constexpr int TT = L < 16 ? L : 16;
-  return TT * TW * ((count + TT - 1) / TT);
-}
+constexpr size_t direct_elems(int n, int w = TW) { return w == 16 ? n * 17 + n / 8 + 1 : (n + n / 8 + 1) * 8; }
+constexpr size_t direct_tile(int n, int w = TW) { return direct_elems(n, w) * sizeof(float2); }
 
-// Column transfers: thread tid moves column l = tid % TW of rows t = tid / TW, tid / TW + T / TW, ...;
-// its global address advances by a fixed (T / TW) rows per step (T is a multiple of TW).
-template <int N, int T>
-__device__ __forceinline__ void async_load_cols(float2* buf, const float2* src, long long base, long long es,
-                                                int valid) {
-  static_assert(T % TW == 0, "whole rows per step");
-  constexpr int RS = T / TW;
-  const int l = threadIdx.x % TW;
-  if (l >= valid) return;
-  const float2* g = src + base + l + (long long)(threadIdx.x / TW) * es;
-  const long long step = (long long)RS * es;
-#pragma unroll 2
-  for (int t = threadIdx.x / TW; t < N; t += RS, g += step) cp_async8(buf + t * TLD + l, g);
+// Threads of a CTA: two radix-8 butterflies each (tiles of 8 lines: one).
+template <int L, int W>
+constexpr int direct_threads() {
+  constexpr int t = ((W == 16 ? L : W * L / 8) + 31) / 32 * 32;
+  return t < 128 ? 128 : (t > 1024 ? 1024 : t);
 }
+// Lines per tile: the x pass of the Poisson solve, row passes, other column passes (narrow tiles give a small
+// mesh's pass more CTAs: the five passes of a 128^3 mesh 67 us instead of 74; those of 512^3
+// 3.25 ms instead of 3.02).
+constexpr int XW = 8, RW = 16;
+constexpr int col_width(int n) { return n <= 160 ? 8 : 16; }
+// CTAs per SM that the register budget is set for (64 registers a thread).
+constexpr int direct_ctas(int threads) { return 1024 / threads; }
 
-template <int N, int T>
-__device__ __forceinline__ void store_cols(const float2* buf, float2* dst, long long base, long long es, int valid) {
-  static_assert(T % TW == 0, "whole rows per step");
-  constexpr int RS = T / TW;
-  const int l = threadIdx.x % TW;
-  if (l >= valid) return;
-  float2* g = dst + base + l + (long long)(threadIdx.x / TW) * es;
-  const long long step = (long long)RS * es;
-#pragma unroll 2
-  for (int t = threadIdx.x / TW; t < N; t += RS, g += step) *g = buf[t * TLD + l];
-}
+// Butterfly q of a stage of NB per line -> (j, line): lines fastest, or (JFAST) 16 consecutive j
+// fastest, for stages whose global side runs along the lines.
+template <int NB, bool JFAST, int W = TW>
+struct StageMap {
+  static constexpr int TT = NB < 16 ? NB : 16;
+  static constexpr int SPAN = JFAST ? TT * W * ((NB + TT - 1) / TT) : NB * W;
+  __device__ static int j(int q) { return JFAST ? (q % TT) + TT * (q / (TT * W)) : q / W; }
+  __device__ static int l(int q) { return JFAST ? (q / TT) % W : q % W; }
+  __device__ static bool ok(int q) { return q < SPAN && (!JFAST || j(q) < NB); }
+};
 
-// Persistent pipeline: each CTA walks tiles blockIdx.x, +gridDim.x, ...; with NBUF = 2 the next
-// tile's copies are in flight while the current one is processed. `tile_elems` is the size of one
-// buffer in float2 units.
-template <int NBUF, typename Load, typename Work>
-__device__ __forceinline__ void pipeline(float2* smem, int tile_elems, int total, Load load, Work work) {
-  int k = 0;
-  int tile = blockIdx.x;
-  if (tile < total) load(smem, tile);
-  cp_async_commit();
-  for (; tile < total; tile += gridDim.x, ++k) {
-    const int next = tile + gridDim.x;
-    float2* cur = smem + (NBUF == 2 ? (k & 1) * tile_elems : 0);
-    if constexpr (NBUF == 2) {
-      if (next < total) load(smem + ((k + 1) & 1) * tile_elems, next);
-      cp_async_commit();
-      cp_async_wait<1>();
+// The stages after the first: NS = product of the radices so far. store(t, l, value) takes the result.
+template <int N, int NS, bool INV, int T, int TS, int MR, bool JOUT, int W, typename Store>
+__device__ __forceinline__ void direct_rest(float2* sm, const float2* __restrict__ tw, const Store& store) {
+  if constexpr (NS < N) {
+    constexpr int R = next_radix<N / NS, MR>();
+    constexpr int NB = N / R;
+    constexpr bool LAST = NS * R == N;
+    using Map = StageMap<NB, LAST && JOUT, W>;
+    constexpr int BPT = (Map::SPAN + T - 1) / T;
+    float2 v[LAST ? 1 : BPT][R];
+    auto butterfly = [&](int q, float2* u) {
+      const int l = Map::l(q), j = Map::j(q), k = j % NS;
+#pragma unroll
+      for (int r = 0; r < R; ++r) u[r] = sm[tile_at<W>(j + r * NB, l)];
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        float2 w = __ldg(tw + r * k * (N / (NS * R)) * TS);
+        if (INV) w.y = -w.y;
+        u[r] = cmul(u[r], w);
+      }
+      dft<R, INV>(u);
+    };
+    if constexpr (LAST) {
+#pragma unroll
+      for (int b = 0; b < BPT; ++b) {
+        const int q = threadIdx.x + b * T;
+        if (Map::SPAN % T != 0 || JOUT) {
+          if (!Map::ok(q)) continue;
+        }
+        butterfly(q, v[0]);
+#pragma unroll
+        for (int r = 0; r < R; ++r) store(Map::j(q) + r * NS, Map::l(q), v[0][r]);
+      }
     } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    work(cur, tile);
-    __syncthreads();
-    if constexpr (NBUF == 1) {
-      if (next < total) load(cur, next);
-      cp_async_commit();
+#pragma unroll
+      for (int b = 0; b < BPT; ++b) {
+        const int q = threadIdx.x + b * T;
+        if (Map::SPAN % T == 0 || Map::ok(q)) butterfly(q, v[b]);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < BPT; ++b) {
+        const int q = threadIdx.x + b * T;
+        if (Map::SPAN % T == 0 || Map::ok(q)) {
+          const int l = Map::l(q), j = Map::j(q), base = (j / NS) * NS * R + j % NS;
+#pragma unroll
+          for (int r = 0; r < R; ++r) sm[tile_at<W>(base + r * NS, l)] = v[b][r];
+        }
+      }
+      __syncthreads();
+      direct_rest<N, NS * R, INV, T, TS, MR, JOUT, W>(sm, tw, store);
     }
   }
-  cp_async_wait<0>();
 }
 
-// c2c pass over a strided axis; tile -> (comp, outer, column tile).
-template <int N, bool INV, int NBUF, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_fft_cols(float2* data, long long comp_stride, ColGeo g, int ncomp,
-                                                const float2* __restrict__ tw) {
+// A whole transform of the tile's W lines: load(t, l) gives element t of line l. JIN / JOUT: the first /
+// last stage's global side runs along the lines. The tile must not be in use when it starts.
+template <int N, bool INV, int T, int TS, int MR, bool JIN, bool JOUT, int W = TW, typename Load, typename Store>
+__device__ __forceinline__ void direct_fft(float2* sm, const float2* __restrict__ tw, const Load& load,
+                                           const Store& store) {
+  constexpr int R = next_radix<N, MR>();
+  constexpr int NB = N / R;
+  using Map = StageMap<NB, JIN, W>;
+  constexpr int BPT = (Map::SPAN + T - 1) / T;
+  float2 v[BPT][R];
+#pragma unroll
+  for (int b = 0; b < BPT; ++b) {
+    const int q = threadIdx.x + b * T;
+    if ((Map::SPAN % T == 0 && !JIN) || Map::ok(q)) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[b][r] = load(Map::j(q) + r * NB, Map::l(q));
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < BPT; ++b) {
+    const int q = threadIdx.x + b * T;
+    if ((Map::SPAN % T == 0 && !JIN) || Map::ok(q)) {
+      const int l = Map::l(q), j = Map::j(q);
+      dft<R, INV>(v[b]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if constexpr (R == N)
+          store(j + r, l, v[b][r]);
+        else
+          sm[tile_at<W>(j * R + r, l)] = v[b][r];
+      }
+    }
+  }
+  if constexpr (R < N) {
+    __syncthreads();
+    direct_rest<N, R, INV, T, TS, MR, JOUT, W>(sm, tw, store);
+  }
+}
+
+// The same with the result left in the tile (the stages after the first in place), complete for all
+// threads when it returns.
+template <int N, int NS, bool INV, int T, int TS, int MR, int W>
+__device__ __forceinline__ void in_place_rest(float2* sm, const float2* __restrict__ tw) {
+  if constexpr (NS < N) {
+    constexpr int R = next_radix<N / NS, MR>();
+    constexpr int NB = N / R;
+    using Map = StageMap<NB, false, W>;
+    constexpr int BPT = (Map::SPAN + T - 1) / T;
+    float2 v[BPT][R];
+#pragma unroll
+    for (int b = 0; b < BPT; ++b) {
+      const int q = threadIdx.x + b * T;
+      if (Map::SPAN % T == 0 || Map::ok(q)) {
+        const int l = Map::l(q), j = Map::j(q), k = j % NS;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[b][r] = sm[tile_at<W>(j + r * NB, l)];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          float2 w = __ldg(tw + r * k * (N / (NS * R)) * TS);
+          if (INV) w.y = -w.y;
+          v[b][r] = cmul(v[b][r], w);
+        }
+        dft<R, INV>(v[b]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < BPT; ++b) {
+      const int q = threadIdx.x + b * T;
+      if (Map::SPAN % T == 0 || Map::ok(q)) {
+        const int l = Map::l(q), j = Map::j(q), base = (j / NS) * NS * R + j % NS;
+#pragma unroll
+        for (int r = 0; r < R; ++r) sm[tile_at<W>(base + r * NS, l)] = v[b][r];
+      }
+    }
+    __syncthreads();
+    in_place_rest<N, NS * R, INV, T, TS, MR, W>(sm, tw);
+  }
+}
+
+template <int N, bool INV, int T, int TS, int MR, int W, typename Load>
+__device__ __forceinline__ void direct_fft_in_place(float2* sm, const float2* __restrict__ tw, const Load& load) {
+  constexpr int R = next_radix<N, MR>();
+  constexpr int NB = N / R;
+  using Map = StageMap<NB, true, W>;
+  constexpr int BPT = (Map::SPAN + T - 1) / T;
+  float2 v[BPT][R];
+#pragma unroll
+  for (int b = 0; b < BPT; ++b) {
+    const int q = threadIdx.x + b * T;
+    if (Map::ok(q)) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[b][r] = load(Map::j(q) + r * NB, Map::l(q));
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < BPT; ++b) {
+    const int q = threadIdx.x + b * T;
+    if (Map::ok(q)) {
+      dft<R, INV>(v[b]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) sm[tile_at<W>(Map::j(q) * R + r, Map::l(q))] = v[b][r];
+    }
+  }
+  __syncthreads();
+  in_place_rest<N, R, INV, T, TS, MR, W>(sm, tw);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The passes on the direct transforms: one tile (of 16 lines) per CTA.
+// ---------------------------------------------------------------------------------------------
+// A CTA's tile of a strided pass: W adjacent columns of one outer index.
+template <int W>
+struct ColTile {
+  long long base;  // element 0 of line 0
+  int valid, outer, col;
+  __device__ ColTile(const ColGeo& g, int tile) {
+    const int tiles = (g.cols + W - 1) / W;
+    outer = tile / tiles;
+    col = (tile % tiles) * W;
+    valid = min(W, g.cols - col);
+    base = g.offset(outer) + col;
+  }
+};
+template <int W>
+int col_tile_count(const ColGeo& g) {
+  return g.outer * ((g.cols + W - 1) / W);
+}
+// Stores of a pass whose spectra are larger than L2: evict-first (STREAM). Left in L2 as ordinary stores, the
+// strided lines of a 512^3 mesh reach DRAM 1.3 to 1.6 times each; meshes that L2 holds part of for the next
+// pass are faster with ordinary ones.
+template <bool STREAM>
+__device__ __forceinline__ void put(float2* p, float2 v) {
+  if constexpr (STREAM)
+    __stcs(p, v);
+  else
+    *p = v;
+}
+
+// c2c pass over a strided axis; block -> (comp, tile).
+template <int N, bool INV, int T, int MR, bool STREAM>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_cols(float2* data, long long comp_stride, ColGeo g,
+                                                            const float2* __restrict__ tw) {
   extern __shared__ float2 smem[];
-  const int per_comp = g.outer * g.col_tiles;
-  auto locate = [&](int tile, long long& base, int& valid, float2*& d) {
-    const int comp = tile / per_comp, rest = tile % per_comp;
-    const int o = rest / g.col_tiles, ct = rest % g.col_tiles;
-    d = data + (long long)comp * comp_stride;
-    base = g.offset(o) + (long long)ct * TW;
-    valid = min(TW, g.cols - ct * TW);
-  };
-  pipeline<NBUF>(
-      smem, N * TLD, ncomp * per_comp,
-      [&](float2* buf, int tile) {
-        long long base;
-        int valid;
-        float2* d;
-        locate(tile, base, valid, d);
-        async_load_cols<N, T>(buf, d, base, g.elem_stride, valid);
-      },
-      [&](float2* cur, int tile) {
-        long long base;
-        int valid;
-        float2* d;
-        locate(tile, base, valid, d);
-        fft_lines<N, INV, T, 1, MR>(cur, tw);
-        store_cols<N, T>(cur, d, base, g.elem_stride, valid);
+  constexpr int W = col_width(N);
+  const int per_comp = g.outer * ((g.cols + W - 1) / W);
+  const ColTile<W> c(g, blockIdx.x % per_comp);
+  const int es = (int)g.elem_stride;
+  float2* d = data + (long long)(blockIdx.x / per_comp) * comp_stride + c.base;
+  direct_fft<N, INV, T, 1, MR, false, false, W>(
+      smem, tw, [&](int t, int l) { return l < c.valid ? d[t * es + l] : make_float2(0.0f, 0.0f); },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(d + t * es + l, v);
       });
 }
 
 // c2c pass over contiguous rows (the z lines of a full complex n^3 array).
-template <int N, bool INV, int NBUF, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_fft_rows(float2* data, int rows, const float2* __restrict__ tw) {
+template <int N, bool INV, int T, int MR>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_rows(float2* data, int rows, const float2* __restrict__ tw) {
   extern __shared__ float2 smem[];
-  pipeline<NBUF>(
-      smem, N * TLD, (rows + TW - 1) / TW,
-      [&](float2* buf, int tile) {
-        const int row0 = tile * TW, valid = min(TW, rows - row0);
-        for (int q = threadIdx.x; q < row_span<N>(N); q += T) {
-          const int t = row_t<N>(q), l = row_l<N>(q);
-          if (l < valid && t < N) cp_async8(buf + t * TLD + l, data + (size_t)(row0 + l) * N + t);
-        }
-      },
-      [&](float2* cur, int tile) {
-        const int row0 = tile * TW, valid = min(TW, rows - row0);
-        fft_lines<N, INV, T, 1, MR>(cur, tw);
-#pragma unroll 4
-        for (int q = threadIdx.x; q < row_span<N>(N); q += T) {
-          const int t = row_t<N>(q), l = row_l<N>(q);
-          if (l < valid && t < N) data[(size_t)(row0 + l) * N + t] = cur[t * TLD + l];
-        }
+  const int row0 = blockIdx.x * RW, valid = min(RW, rows - row0);
+  float2* d = data + (size_t)row0 * N;
+  direct_fft<N, INV, T, 1, MR, true, true, RW>(
+      smem, tw, [&](int t, int l) { return l < valid ? d[l * N + t] : make_float2(0.0f, 0.0f); },
+      [&](int t, int l, float2 v) {
+        if (l < valid) d[l * N + t] = v;
       });
 }
 
-// z pass, forward: TW real rows of length N -> N/2+1 complex each (rows of the padded half
-// spectrum), as an N/2-point complex transform of z[m] = x[2m] + i x[2m+1]. Input: f32 delta, or
-// the u64 fixed-point mass mesh (c = fx * 2^-k in f32, delta = c / mean - 1). Each thread loads its
-// input pairs straight into registers (16-byte loads of two u64 cells, all of a tile's loads issued
-// before any is used), converts them and writes the complex tile: shared memory holds only that
-// tile, so several CTAs per SM keep the loads of their tiles in flight.
-template <int N, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_r2c_z(const float* __restrict__ delta,
-                                             const unsigned long long* __restrict__ fx, float inv_scale, float mean,
-                                             float2* __restrict__ spec, int rows, const float2* __restrict__ tw) {
+// z pass, forward: real rows of length N -> N/2+1 complex each (rows of the padded half spectrum), as an
+// N/2-point complex transform of z[m] = x[2m] + i x[2m+1]. Input: f32 delta, or the u64 fixed-point mass
+// mesh (c = fx * 2^-k in f32, delta = c / mean - 1), converted on its way into the first stage.
+template <int N, int T, int MR>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_rows_r2c(const float* __restrict__ delta,
+                                                                const unsigned long long* __restrict__ fx,
+                                                                float inv_scale, float mean, float inv_mean,
+                                                                float2* __restrict__ spec, int rows,
+                                                                const float2* __restrict__ tw) {
   extern __shared__ float2 smem[];
-  constexpr int M = N / 2, NH = N / 2 + 1, NHP = N / 2 + 2;
-  constexpr int SPAN = TW * ((M + 15) / 16) * 16;  // row_span<M>(M)
-  constexpr int PER = (SPAN + T - 1) / T;
-  float2* cplx = smem;
-  const int tiles = (rows + TW - 1) / TW;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int row0 = tile * TW, valid = min(TW, rows - row0);
-    float2 v[PER];
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int q = threadIdx.x + k * T;
-      const int m = row_t<M>(q), l = row_l<M>(q);
-      v[k] = make_float2(0.0f, 0.0f);
-      if (q < SPAN && l < valid && m < M) {
-        const size_t gi = (size_t)(row0 + l) * N + 2 * m;
-        if (fx) {
-          const ulonglong2 u = __ldg(reinterpret_cast<const ulonglong2*>(fx + gi));
-          const float c0 = __fmul_rn(__ull2float_rn(u.x), inv_scale);
-          const float c1 = __fmul_rn(__ull2float_rn(u.y), inv_scale);
-          v[k] = make_float2(__fsub_rn(__fdiv_rn(c0, mean), 1.0f), __fsub_rn(__fdiv_rn(c1, mean), 1.0f));
-        } else {
-          v[k] = __ldg(reinterpret_cast<const float2*>(delta + gi));
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int q = threadIdx.x + k * T;
-      const int m = row_t<M>(q), l = row_l<M>(q);
-      if (q < SPAN && m < M) cplx[m * TLD + l] = v[k];
-    }
-    __syncthreads();
-    fft_lines<M, false, T, 2, MR>(cplx, tw);
-    // X[k] = (Z[k] + conj(Z[M-k]))/2 + w^k (Z[k] - conj(Z[M-k]))/(2i), w = exp(-2 pi i / N)
-    for (int q = threadIdx.x; q < row_span<M>(NH); q += T) {
-      const int k = row_t<M>(q), l = row_l<M>(q);
-      if (l >= valid || k >= NH) continue;
-      // Z is M-periodic: Z[M] = Z[0] (k runs over 0..M)
-      const float2 zk = cplx[(k == M ? 0 : k) * TLD + l];
-      const float2 zm = cplx[(k == 0 ? 0 : M - k) * TLD + l];
-      const float2 fe = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      const float2 fo = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
-      spec[(size_t)(row0 + l) * NHP + k] = cadd(fe, cmul(__ldg(tw + k), fo));
-    }
-    __syncthreads();  // the next tile overwrites the complex tile
+  constexpr int M = N / 2, NH = N / 2 + 1, NHP = half_row(N);
+  const int row0 = blockIdx.x * RW, valid = min(RW, rows - row0);
+  if (fx) {
+    const unsigned long long* src = fx + (size_t)row0 * N;
+    direct_fft_in_place<M, false, T, 2, MR, RW>(smem, tw, [&](int m, int l) {
+      if (l >= valid) return make_float2(0.0f, 0.0f);
+      const ulonglong2 u = __ldg(reinterpret_cast<const ulonglong2*>(src + l * N + 2 * m));
+      const float c0 = __fmul_rn(__ull2float_rn(u.x), inv_scale);
+      const float c1 = __fmul_rn(__ull2float_rn(u.y), inv_scale);
+      // (a mean that is a power of two has an exact reciprocal: the same quotients without a division)
+      if (inv_mean != 0.0f)
+        return make_float2(__fsub_rn(__fmul_rn(c0, inv_mean), 1.0f), __fsub_rn(__fmul_rn(c1, inv_mean), 1.0f));
+      return make_float2(__fsub_rn(__fdiv_rn(c0, mean), 1.0f), __fsub_rn(__fdiv_rn(c1, mean), 1.0f));
+    });
+  } else {
+    const float* src = delta + (size_t)row0 * N;
+    direct_fft_in_place<M, false, T, 2, MR, RW>(smem, tw, [&](int m, int l) {
+      return l < valid ? __ldg(reinterpret_cast<const float2*>(src + l * N + 2 * m)) : make_float2(0.0f, 0.0f);
+    });
+  }
+  // X[k] = (Z[k] + conj(Z[M-k]))/2 + w^k (Z[k] - conj(Z[M-k]))/(2i), w = exp(-2 pi i / N)
+  for (int q = threadIdx.x; q < StageMap<NH, true, RW>::SPAN; q += T) {
+    const int k = StageMap<NH, true, RW>::j(q), l = StageMap<NH, true, RW>::l(q);
+    if (l >= valid || k >= NH) continue;
+    // Z is M-periodic: Z[M] = Z[0] (k runs over 0..M)
+    const float2 zk = smem[tile_at<RW>(k == M ? 0 : k, l)];
+    const float2 zm = smem[tile_at<RW>(k == 0 ? 0 : M - k, l)];
+    const float2 fe = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+    const float2 fo = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+    spec[(size_t)(row0 + l) * NHP + k] = cadd(fe, cmul(__ldg(tw + k), fo));
   }
 }
 
 // z pass, inverse: N/2+1 complex per row -> N real values times scale, as an N/2-point complex
-// inverse transform of Z'[k] = (X[k] + conj(X[M-k])) + i (X[k] - conj(X[M-k])) conj(w^k), whose
-// output is x[2m] + i x[2m+1]. tile -> (comp, row tile). Shared memory: NBUF tiles of (M+1)*TLD.
-template <int N, int NBUF, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_c2r_z(const float2* __restrict__ spec, long long comp_stride,
-                                             float* __restrict__ out0, float* __restrict__ out1,
-                                             float* __restrict__ out2, float scale, int rows,
-                                             const float2* __restrict__ tw) {
+// inverse transform of Z'[k] = (X[k] + conj(X[M-k])) + i (X[k] - conj(X[M-k])) conj(w^k), whose output is
+// x[2m] + i x[2m+1]; block -> (comp, row tile). The first stage's inputs Z'[k] are formed from X[k] and
+// X[M-k] as they are loaded (every row is in L1 for its second reading).
+template <int N, int T, int MR>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_rows_c2r(const float2* __restrict__ spec, long long comp_stride,
+                                                                float* __restrict__ out0, float* __restrict__ out1,
+                                                                float* __restrict__ out2, float scale, int rows,
+                                                                const float2* __restrict__ tw) {
   extern __shared__ float2 smem[];
-  constexpr int M = N / 2, NH = N / 2 + 1, NHP = N / 2 + 2;
-  const int row_tiles = (rows + TW - 1) / TW;
-  pipeline<NBUF>(
-      smem, (M + 1) * TLD, 3 * row_tiles,
-      [&](float2* buf, int tile) {
-        const int comp = tile / row_tiles, row0 = (tile % row_tiles) * TW, valid = min(TW, rows - row0);
-        const float2* sp = spec + (long long)comp * comp_stride;
-        for (int q = threadIdx.x; q < row_span<M>(NH); q += T) {
-          const int t = row_t<M>(q), l = row_l<M>(q);
-          if (l < valid && t < NH) cp_async8(buf + t * TLD + l, sp + (size_t)(row0 + l) * NHP + t);
+  constexpr int M = N / 2, NHP = half_row(N);
+  const int row_tiles = (rows + RW - 1) / RW;
+  const int comp = blockIdx.x / row_tiles, row0 = (blockIdx.x % row_tiles) * RW, valid = min(RW, rows - row0);
+  const float2* sp = spec + (long long)comp * comp_stride + (size_t)row0 * NHP;
+  float2* out = reinterpret_cast<float2*>((comp == 0 ? out0 : (comp == 1 ? out1 : out2)) + (size_t)row0 * N);
+  direct_fft<M, true, T, 2, MR, true, true, RW>(
+      smem, tw,
+      [&](int k, int l) {
+        if (l >= valid) return make_float2(0.0f, 0.0f);
+        // the upper of the pair k, M - k by w^(M-k) = -conj(w^k)
+        const int lo = min(k, M - k);
+        float2 x = __ldg(sp + l * NHP + lo), y = __ldg(sp + l * NHP + M - lo);
+        // X[0] and X[M] enter the real output through their real parts only (as in Re of a
+        // full complex inverse); their imaginary parts are round-off of the Hermitian planes.
+        if (lo == 0) x.y = y.y = 0.0f;
+        const float2 w = __ldg(tw + lo);
+        if (k == lo) {
+          const float2 a = cadd(x, conjf2(y)), b = csub(x, conjf2(y));
+          const float2 bw = cmul(b, conjf2(w));
+          return make_float2(a.x - bw.y, a.y + bw.x);
         }
+        const float2 a = cadd(y, conjf2(x)), b = csub(y, conjf2(x));
+        const float2 bw = cmul(b, make_float2(-w.x, -w.y));
+        return make_float2(a.x - bw.y, a.y + bw.x);
       },
-      [&](float2* cur, int tile) {
-        const int comp = tile / row_tiles, row0 = (tile % row_tiles) * TW, valid = min(TW, rows - row0);
-        float* out = comp == 0 ? out0 : (comp == 1 ? out1 : out2);
-        for (int q = threadIdx.x; q < (M / 2 + 1) * TW; q += T) {
-          const int l = q % TW, k = q / TW;
-          float2 xk = cur[k * TLD + l], xm = cur[(M - k) * TLD + l];
-          // X[0] and X[M] enter the real output through their real parts only (as in Re of a
-          // full complex inverse); their imaginary parts are round-off of the Hermitian planes.
-          if (k == 0) xk.y = xm.y = 0.0f;
-          const float2 wk = __ldg(tw + k);
-          // Z'[k] and, for 0 < k < M/2, Z'[M-k] (w^(M-k) = -conj(w^k))
-          const float2 a = cadd(xk, conjf2(xm)), b = csub(xk, conjf2(xm));
-          const float2 bw = cmul(b, conjf2(wk));
-          cur[k * TLD + l] = make_float2(a.x - bw.y, a.y + bw.x);
-          if (k > 0 && 2 * k < M) {
-            const float2 a2 = cadd(xm, conjf2(xk)), b2 = csub(xm, conjf2(xk));
-            const float2 bw2 = cmul(b2, make_float2(-wk.x, -wk.y));
-            cur[(M - k) * TLD + l] = make_float2(a2.x - bw2.y, a2.y + bw2.x);
-          }
-        }
-        __syncthreads();
-        fft_lines<M, true, T, 2, MR>(cur, tw);
-#pragma unroll 4
-        for (int q = threadIdx.x; q < row_span<M>(M); q += T) {
-          const int m = row_t<M>(q), l = row_l<M>(q);
-          if (l < valid && m < M) {
-            const float2 v = cur[m * TLD + l];
-            reinterpret_cast<float2*>(out + (size_t)(row0 + l) * N)[m] =
-                make_float2(__fmul_rn(v.x, scale), __fmul_rn(v.y, scale));
-          }
-        }
+      [&](int m, int l, float2 v) {
+        if (l < valid) out[l * (N / 2) + m] = make_float2(__fmul_rn(v.x, scale), __fmul_rn(v.y, scale));
       });
 }
 
-// x pass of the Poisson solve for TW kz columns at fixed ky (tile -> (iy, column tile)): forward
-// c2c along x, the Green's function of poisson.rs:52-74, then
-//   x component: inverse x transform of -i k_x phi;
-//   y, z components: -i k_y and -i k_z times the inverse x transform of phi (k_y, k_z constant
-//   along the line, so the factor commutes with the transform), applied by k_grad_yz.
+// x pass of the Poisson solve for XW kz columns at fixed ky: forward c2c along x, the Green's function of
+// poisson.rs:52-74 (phi_k into a second tile), then the inverse transforms
+//   of -i k_x phi (the x component) to slot 0;
+//   of phi to slot 1, from which the y pass forms the y and z components: -i k_y and -i k_z are
+//   constant along the line, so the factors commute with the transform.
 // The gradient factor is the reference's (phi * (0 - i k_a), poisson.rs:70); for y and z it
 // multiplies the transformed phi instead, which differs only in round-off.
-// Shared memory: NBUF input tiles, then one work tile for -i k_x phi.
-template <int N, int NBUF, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_poisson_x(const float2* __restrict__ spec_in, float2* spec_out,
-                                                 long long comp_stride, ColGeo g, PoissonParams pp,
-                                                 const float* __restrict__ deconv, const float2* __restrict__ tw) {
+// (Two tiles of 16 lines leave one CTA per SM; phi_k kept in slot 1 instead went to DRAM and back: 1.12 ms at
+// n = 512, now 0.72.)
+template <int N, int T, int MR, bool STREAM>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_x_poisson(float2* spec, long long comp_stride, ColGeo g,
+                                                                 PoissonParams pp, const float* __restrict__ deconv,
+                                                                 const float2* __restrict__ tw) {
   extern __shared__ float2 smem[];
-  float2* gxb = smem + NBUF * N * TLD;
-  pipeline<NBUF>(
-      smem, N * TLD, g.outer * g.col_tiles,
-      [&](float2* buf, int tile) {
-        const int iy = tile / g.col_tiles, ct = tile % g.col_tiles;
-        const long long base = g.offset(iy) + (long long)ct * TW;
-        async_load_cols<N, T>(buf, spec_in, base, g.elem_stride, min(TW, g.cols - ct * TW));
-      },
-      [&](float2* phi, int tile) {
-        const int iy = tile / g.col_tiles, ct = tile % g.col_tiles;
-        const int valid = min(TW, g.cols - ct * TW);
-        const long long base = g.offset(iy) + (long long)ct * TW;
-        const int z0 = ct * TW;
-        const float prefactor = pp.prefactor_dev ? *pp.prefactor_dev : pp.prefactor;
-        fft_lines<N, false, T, 1, MR>(phi, tw);
-        const float ky = wavenumber(g.in_box(iy), N, pp.two_pi_over_l);
-        for (int q = threadIdx.x; q < N * TW; q += T) {
-          const int l = q % TW, t = q / TW;
-          const float kx = wavenumber(t, N, pp.two_pi_over_l);
-          const float kz = wavenumber(min(z0 + l, N / 2), N, pp.two_pi_over_l);
-          float k2 = -0.0f;
-          k2 = __fadd_rn(k2, __fmul_rn(kx, kx));
-          k2 = __fadd_rn(k2, __fmul_rn(ky, ky));
-          k2 = __fadd_rn(k2, __fmul_rn(kz, kz));
-          float2 v = phi[t * TLD + l];
-          if (k2 == 0.0f || l >= valid) {
-            v = make_float2(0.0f, 0.0f);
-          } else {
-            // phi_k = delta_k * (-prefactor / k^2 * exp(-k^2 r_s^2)), k = 0 skipped (left zero)
-            const float filter = expf(__fmul_rn(__fmul_rn(-k2, pp.r_split), pp.r_split));
-            float sc = __fmul_rn(__fdiv_rn(-prefactor, k2), filter);
-            if (deconv) sc = __fmul_rn(sc, __fmul_rn(__fmul_rn(deconv[t], deconv[g.in_box(iy)]), deconv[z0 + l]));
-            v = make_float2(__fmul_rn(v.x, sc), __fmul_rn(v.y, sc));
-          }
-          phi[t * TLD + l] = v;
-          // -i k_x phi: re = phi.re*0 - phi.im*(-k_x), im = phi.re*(-k_x) + phi.im*0
-          const float nk = -kx;
-          gxb[t * TLD + l] = make_float2(__fsub_rn(__fmul_rn(v.x, 0.0f), __fmul_rn(v.y, nk)),
-                                         __fadd_rn(__fmul_rn(v.x, nk), __fmul_rn(v.y, 0.0f)));
-        }
-        __syncthreads();
-        fft_lines2<N, true, T, 1, MR>(gxb, phi, tw);
-        // -i k_x phi to slot 0; the x-transformed phi to slot 1, from which the y pass forms the
-        // y and z components (k_y and k_z are constant along an x line)
-        store_cols<N, T>(gxb, spec_out, base, g.elem_stride, valid);
-        store_cols<N, T>(phi, spec_out + comp_stride, base, g.elem_stride, valid);
-      });
-}
-
-// Inverse y pass of the y and z gradient components: reads the x-transformed potential of slot 1
-// once, forms -i k_y phi and -i k_z phi (the f32 operations of k_green_grad) and writes their
-// inverse y transforms to slots 1 and 2; tile -> (x, column tile), lines along y.
-template <int N, int NBUF, int T, int MR = 8>
-__global__ void __launch_bounds__(T) k_grad_yz(float2* spec, long long comp_stride, ColGeo g, PoissonParams pp,
-                                               const float2* __restrict__ tw) {
-  extern __shared__ float2 smem[];
-  float2* gzb = smem + NBUF * N * TLD;
-  float2* phi_slot = spec + comp_stride;
-  pipeline<NBUF>(
-      smem, N * TLD, g.outer * g.col_tiles,
-      [&](float2* buf, int tile) {
-        const int o = tile / g.col_tiles, ct = tile % g.col_tiles;
-        const long long base = g.offset(o) + (long long)ct * TW;
-        async_load_cols<N, T>(buf, phi_slot, base, g.elem_stride, min(TW, g.cols - ct * TW));
-      },
-      [&](float2* cur, int tile) {
-        const int o = tile / g.col_tiles, ct = tile % g.col_tiles;
-        const int valid = min(TW, g.cols - ct * TW);
-        const long long base = g.offset(o) + (long long)ct * TW;
-        const int z0 = ct * TW;
-        for (int q = threadIdx.x; q < N * TW; q += T) {
-          const int l = q % TW, t = q / TW;
-          const float2 p = cur[t * TLD + l];
-          const float nky = -wavenumber(t, N, pp.two_pi_over_l);
-          const float nkz = -wavenumber(z0 + l, N, pp.two_pi_over_l);
-          cur[t * TLD + l] = make_float2(__fsub_rn(__fmul_rn(p.x, 0.0f), __fmul_rn(p.y, nky)),
-                                         __fadd_rn(__fmul_rn(p.x, nky), __fmul_rn(p.y, 0.0f)));
-          gzb[t * TLD + l] = make_float2(__fsub_rn(__fmul_rn(p.x, 0.0f), __fmul_rn(p.y, nkz)),
-                                         __fadd_rn(__fmul_rn(p.x, nkz), __fmul_rn(p.y, 0.0f)));
-        }
-        __syncthreads();
-        fft_lines2<N, true, T, 1, MR>(cur, gzb, tw);
-        store_cols<N, T>(cur, phi_slot, base, g.elem_stride, valid);
-        store_cols<N, T>(gzb, spec + 2 * comp_stride, base, g.elem_stride, valid);
-      });
-}
-
-// Green's function and gradient of poisson.rs:52-74 applied elementwise to the half spectrum in
-// slot 0, writing -i k_a phi to slots 0..2 (the same f32 operations as k_poisson_x). Used where
-// the fused x pass does not fit in shared memory.
-__global__ void k_green_grad(float2* spec, long long comp, int n, PoissonParams pp, const float* __restrict__ deconv) {
-  const int nh = n / 2 + 1, nhp = n / 2 + 2;
-  const long long total = (long long)n * n * nh;
+  float2* phi = smem + direct_elems(N, XW);
+  const ColTile<XW> c(g, blockIdx.x);
+  const int es = (int)g.elem_stride, iy = g.in_box(c.outer);
+  float2* s0 = spec + c.base;
+  float2* s1 = s0 + comp_stride;
   const float prefactor = pp.prefactor_dev ? *pp.prefactor_dev : pp.prefactor;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int kz = (int)(e % nh);
-    const long long line = e / nh;
-    const int iy = (int)(line % n), ix = (int)(line / n);
-    const long long gi = line * nhp + kz;
-    const float kx = wavenumber(ix, n, pp.two_pi_over_l), ky = wavenumber(iy, n, pp.two_pi_over_l);
-    const float kzv = wavenumber(kz, n, pp.two_pi_over_l);
-    float k2 = -0.0f;
-    k2 = __fadd_rn(k2, __fmul_rn(kx, kx));
-    k2 = __fadd_rn(k2, __fmul_rn(ky, ky));
-    k2 = __fadd_rn(k2, __fmul_rn(kzv, kzv));
-    float2 v = spec[gi];
-    if (k2 == 0.0f) {
-      v = make_float2(0.0f, 0.0f);
-    } else {
-      const float filter = expf(__fmul_rn(__fmul_rn(-k2, pp.r_split), pp.r_split));
-      float sc = __fmul_rn(__fdiv_rn(-prefactor, k2), filter);
-      if (deconv) sc = __fmul_rn(sc, __fmul_rn(__fmul_rn(deconv[ix], deconv[iy]), deconv[kz]));
-      v = make_float2(__fmul_rn(v.x, sc), __fmul_rn(v.y, sc));
-    }
-    const float nk[3] = {-kx, -ky, -kzv};
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-      spec[a * comp + gi] = make_float2(__fsub_rn(__fmul_rn(v.x, 0.0f), __fmul_rn(v.y, nk[a])),
-                                        __fadd_rn(__fmul_rn(v.x, nk[a]), __fmul_rn(v.y, 0.0f)));
-  }
+  const float ky = wavenumber(iy, N, pp.two_pi_over_l);
+  direct_fft<N, false, T, 1, MR, false, false, XW>(
+      smem, tw, [&](int t, int l) { return l < c.valid ? s0[t * es + l] : make_float2(0.0f, 0.0f); },
+      [&](int t, int l, float2 v) {
+        const int iz = c.col + l;
+        const float kx = wavenumber(t, N, pp.two_pi_over_l), kz = wavenumber(min(iz, N / 2), N, pp.two_pi_over_l);
+        float k2 = -0.0f;
+        k2 = __fadd_rn(k2, __fmul_rn(kx, kx));
+        k2 = __fadd_rn(k2, __fmul_rn(ky, ky));
+        k2 = __fadd_rn(k2, __fmul_rn(kz, kz));
+        if (k2 == 0.0f || l >= c.valid) {
+          v = make_float2(0.0f, 0.0f);
+        } else {
+          // phi_k = delta_k * (-prefactor / k^2 * exp(-k^2 r_s^2)), k = 0 skipped (left zero)
+          const float filter = expf(__fmul_rn(__fmul_rn(-k2, pp.r_split), pp.r_split));
+          float sc = __fmul_rn(__fdiv_rn(-prefactor, k2), filter);
+          if (deconv) sc = __fmul_rn(sc, __fmul_rn(__fmul_rn(deconv[t], deconv[iy]), deconv[iz]));
+          v = make_float2(__fmul_rn(v.x, sc), __fmul_rn(v.y, sc));
+        }
+        phi[tile_at<XW>(t, l)] = v;
+      });
+  __syncthreads();  // phi_k of the tile is complete, the exchange tile free
+  direct_fft<N, true, T, 1, MR, false, false, XW>(
+      smem, tw,
+      [&](int t, int l) {
+        // -i k_x phi: re = phi.re*0 - phi.im*(-k_x), im = phi.re*(-k_x) + phi.im*0
+        const float2 v = phi[tile_at<XW>(t, l)];
+        const float nk = -wavenumber(t, N, pp.two_pi_over_l);
+        return make_float2(__fsub_rn(__fmul_rn(v.x, 0.0f), __fmul_rn(v.y, nk)),
+                           __fadd_rn(__fmul_rn(v.x, nk), __fmul_rn(v.y, 0.0f)));
+      },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(s0 + t * es + l, v);
+      });
+  __syncthreads();
+  direct_fft<N, true, T, 1, MR, false, false, XW>(
+      smem, tw, [&](int t, int l) { return phi[tile_at<XW>(t, l)]; },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(s1 + t * es + l, v);
+      });
+}
+
+// Inverse y pass of the three components, tile by tile: the x component (slot 0), and from the
+// x-transformed potential (slot 1) the z component -i k_z phi (slot 2), then the y component -i k_y
+// phi over the potential.
+template <int N, int T, int MR, bool STREAM>
+__global__ void __launch_bounds__(T, direct_ctas(T)) k_y_gradient(float2* spec, long long comp_stride, ColGeo g,
+                                                                  PoissonParams pp, const float2* __restrict__ tw) {
+  extern __shared__ float2 smem[];
+  constexpr int W = col_width(N);
+  const ColTile<W> c(g, blockIdx.x);
+  const int es = (int)g.elem_stride;
+  float2* s0 = spec + c.base;
+  float2 *s1 = s0 + comp_stride, *s2 = s1 + comp_stride;
+  auto times = [&](float2 p, float nk) {  // -i k phi with nk = -k, as k_x_poisson
+    return make_float2(__fsub_rn(__fmul_rn(p.x, 0.0f), __fmul_rn(p.y, nk)),
+                       __fadd_rn(__fmul_rn(p.x, nk), __fmul_rn(p.y, 0.0f)));
+  };
+  direct_fft<N, true, T, 1, MR, false, false, W>(
+      smem, tw, [&](int t, int l) { return l < c.valid ? s0[t * es + l] : make_float2(0.0f, 0.0f); },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(s0 + t * es + l, v);
+      });
+  __syncthreads();
+  direct_fft<N, true, T, 1, MR, false, false, W>(
+      smem, tw,
+      [&](int t, int l) {
+        return l < c.valid ? times(s1[t * es + l], -wavenumber(c.col + l, N, pp.two_pi_over_l)) : make_float2(0.0f, 0.0f);
+      },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(s2 + t * es + l, v);
+      });
+  __syncthreads();
+  direct_fft<N, true, T, 1, MR, false, false, W>(
+      smem, tw,
+      [&](int t, int l) {
+        return l < c.valid ? times(s1[t * es + l], -wavenumber(t, N, pp.two_pi_over_l)) : make_float2(0.0f, 0.0f);
+      },
+      [&](int t, int l, float2 v) {
+        if (l < c.valid) put<STREAM>(s1 + t * es + l, v);
+      });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -828,7 +641,7 @@ const char* fft_sizes_text() {
   return "4, 8, 16, 32, 48, 64, 80, 96, 128, 160, 192, 256, 320, 384, 512 or 1024";
 }
 
-size_t half_spectrum_elems(int n) { return (size_t)n * n * (size_t)(n / 2 + 2); }
+size_t half_spectrum_elems(int n) { return (size_t)n * n * (size_t)half_row(n); }
 
 cudaError_t fft_plan_init(FftPlan& p, int n) {
   if (p.n == n && p.twiddle.p && p.deconv.p) return cudaSuccess;
@@ -860,61 +673,44 @@ void fft_plan_free(FftPlan& p) {
   p.n = 0;
 }
 
-static int num_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
+// 1 / x when x is a power of two (whose reciprocal is exact), else 0.
+static float exact_inverse(float x) {
+  int e = 0;
+  return x > 1e-30f && x < 1e30f && std::frexp(x, &e) == 0.5f ? 1.0f / x : 0.0f;
 }
 
-// Persistent launch: as many CTAs as fit on all SMs at once, at most one per tile.
+// Meshes whose strided passes store evict-first: the five passes of 512^3 3.48 -> 3.19 ms when it was
+// introduced; 384^3 1.75 -> 1.81, 320^3 1.02 -> 1.05 (256^3 0.400 -> 0.394 later).
+constexpr int STREAM_MESH = 512;
+
+// One tile per CTA.
 template <typename K, typename... Args>
-static void launch_persistent(K kernel, int threads, size_t smem, int total, cudaStream_t s, Args... args) {
+static void launch_tiles(K kernel, int threads, size_t smem, int tiles, cudaStream_t s, Args... args) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const int grid = std::max(1, std::min(total, per_sm * num_sms()));
   count_launch();
-  kernel<<<grid, threads, smem, s>>>(args...);
+  kernel<<<tiles, threads, smem, s>>>(args...);
 }
 
-constexpr size_t c_tile(int rows_of_tile) { return (size_t)rows_of_tile * TLD * sizeof(float2); }
-
-template <int N, int MR = 8>
-static void cols_pass(float2* data, long long comp_stride, int ncomp, ColGeo g, int inverse, const float2* tw,
-                      cudaStream_t s) {
-  constexpr int T = threads_for<N, MR>();
-  constexpr int NB = 2 * c_tile(N) <= SMEM_LIMIT ? 2 : 1;
-  const size_t smem = NB * c_tile(N);
-  g.col_tiles = (g.cols + TW - 1) / TW;
-  const int total = ncomp * g.outer * g.col_tiles;
-  if (inverse)
-    launch_persistent(k_fft_cols<N, true, NB, T, MR>, T, smem, total, s, data, comp_stride, g, ncomp, tw);
-  else
-    launch_persistent(k_fft_cols<N, false, NB, T, MR>, T, smem, total, s, data, comp_stride, g, ncomp, tw);
+template <int N, int MR>
+static void cols_direct(float2* data, long long comp_stride, int ncomp, ColGeo g, int inverse, const float2* tw,
+                        cudaStream_t s) {
+  constexpr int T = direct_threads<N, col_width(N)>();
+  constexpr bool ST = N >= STREAM_MESH;
+  launch_tiles(inverse ? k_cols<N, true, T, MR, ST> : k_cols<N, false, T, MR, ST>, T, direct_tile(N, col_width(N)),
+               ncomp * col_tile_count<col_width(N)>(g), s, data, comp_stride, g, tw);
 }
 
 template <int N>
 static void fft3_c2c_n(float2* data, int inverse, const float2* tw, cudaStream_t s) {
-  constexpr int T = threads_for<N>();
-  constexpr int NB = 2 * c_tile(N) <= SMEM_LIMIT ? 2 : 1;
-  const size_t smem = NB * c_tile(N);
+  constexpr int T = direct_threads<N, RW>();
   const long long n = N;
   const int rows = N * N;
-  const int total = (rows + TW - 1) / TW;
-  if (inverse)
-    launch_persistent(k_fft_rows<N, true, NB, T>, T, smem, total, s, data, rows, tw);
-  else
-    launch_persistent(k_fft_rows<N, false, NB, T>, T, smem, total, s, data, rows, tw);
+  launch_tiles(inverse ? k_rows<N, true, T, 8> : k_rows<N, false, T, 8>, T, direct_tile(N, RW), (rows + RW - 1) / RW, s,
+               data, rows, tw);
   // y lines: elements n apart, columns along z adjacent, outer = x
-  cols_pass<N>(data, 0, 1, ColGeo{n * n, n, N, 0, N}, inverse, tw, s);
+  cols_direct<N, 8>(data, 0, 1, ColGeo{n * n, n, N, N}, inverse, tw, s);
   // x lines: elements n*n apart, outer = y
-  cols_pass<N>(data, 0, 1, ColGeo{n, n * n, N, 0, N}, inverse, tw, s);
+  cols_direct<N, 8>(data, 0, 1, ColGeo{n, n * n, N, N}, inverse, tw, s);
 }
 
 void launch_fft3_c2c(const FftPlan& p, float2* data, int inverse, cudaStream_t s) {
@@ -934,77 +730,45 @@ template <int N>
 static void r2c3_n(const FftPlan& p, const float* delta, const unsigned long long* fx, int fx_shift, float mean,
                    float2* spec, cudaStream_t s) {
   const float2* tw = static_cast<const float2*>(p.twiddle.p);
-  constexpr int M = N / 2, NH = N / 2 + 1, NHP = N / 2 + 2;
+  constexpr int M = N / 2, NH = N / 2 + 1, NHP = half_row(N);
   const long long n = N;
   const int rows = N * N;
   {
-    constexpr int T = threads_for<M>();
-    launch_persistent(k_r2c_z<N, T>, T, c_tile(M), (rows + TW - 1) / TW, s, delta, fx, std::ldexp(1.0f, -fx_shift),
-                      mean, spec, rows, tw);
+    constexpr int T = direct_threads<M, RW>();
+    launch_tiles(k_rows_r2c<N, T, 8>, T, direct_tile(M, RW), (rows + RW - 1) / RW, s, delta, fx, std::ldexp(1.0f, -fx_shift),
+                 mean, exact_inverse(mean), spec, rows, tw);
   }
-  cols_pass<N>(spec, 0, 1, ColGeo{n * NHP, NHP, NH, 0, N}, 0, tw, s);  // y lines, outer = x
-  cols_pass<N>(spec, 0, 1, ColGeo{NHP, n * NHP, NH, 0, N}, 0, tw, s);  // x lines, outer = y
+  cols_direct<N, 8>(spec, 0, 1, ColGeo{n * NHP, NHP, NH, N}, 0, tw, s);  // y lines, outer = x
+  cols_direct<N, 8>(spec, 0, 1, ColGeo{NHP, n * NHP, NH, N}, 0, tw, s);  // x lines, outer = y
 }
 
 template <int N, int MR>
 static void poisson_n(const FftPlan& p, const PoissonParams& pp, const float* delta, const unsigned long long* fx,
-                      int fx_shift, float mean, float2* spec, float* gx, float* gy, float* gz, cudaStream_t s) {
+                      int fx_shift, float mean, float2* spec, float* gx, float* gy_out, float* gz, cudaStream_t s) {
   const float2* tw = static_cast<const float2*>(p.twiddle.p);
   const float* deconv = pp.deconvolve ? static_cast<const float*>(p.deconv.p) : nullptr;
-  constexpr int M = N / 2, NH = N / 2 + 1, NHP = N / 2 + 2;
+  constexpr int M = N / 2, NH = N / 2 + 1, NHP = half_row(N);
   const long long n = N;
   const int nb = pp.boxes > 1 ? pp.boxes : 1;  // a batch of nb meshes, one after another
   const long long comp = nb * n * n * NHP;     // elements per half spectrum (every box)
   const int rows = nb * N * N;
-  const int row_tiles = (rows + TW - 1) / TW;
-  if constexpr (2 * c_tile(N) > SMEM_LIMIT) {
-    // The fused x pass needs two N-point tiles: not on one SM at this size. Forward R2C, the
-    // Green's function and gradient elementwise, then inverse x and y passes on three spectra.
-    r2c3_n<N>(p, delta, fx, fx_shift, mean, spec, s);
-    const long long total = n * n * NH;
-    const int grid = (int)std::min<long long>((total + 255) / 256, 16LL * num_sms());
-    count_launch();
-    k_green_grad<<<grid, 256, 0, s>>>(spec, comp, N, pp, deconv);
-    cols_pass<N, MR>(spec, comp, 3, ColGeo{NHP, n * NHP, NH, 0, N}, 1, tw, s);  // x lines, outer = y
-  } else {
-    // Slot 0 holds the forward spectrum; the x pass reads each tile of it before writing the
-    // same tile of slots 0..2, and tiles are disjoint, so the update in place is safe.
-    float2* s0 = spec;
-    {  // 1. z: R2C into slot 0 (one complex tile in shared memory per CTA)
-      constexpr int T = threads_for<M, MR>();
-      launch_persistent(k_r2c_z<N, T, MR>, T, c_tile(M), row_tiles, s, delta, fx, std::ldexp(1.0f, -fx_shift), mean, s0,
-                        rows, tw);
-    }
-    // 2. y forward on slot 0: lines along y (stride NHP), columns along kz adjacent, outer = x
-    //    (the x planes of a batch's boxes form one run)
-    cols_pass<N, MR>(s0, 0, 1, ColGeo{n * NHP, NHP, NH, 0, nb * N}, 0, tw, s);
-    {  // 3. x forward + Green + gradient + x inverse -> slots 0 (-i k_x phi) and 1 (phi); outer = y
-      constexpr int T = threads_for<N, MR>();
-      constexpr int NBX = 3 * c_tile(N) <= SMEM_LIMIT ? 2 : 1;
-      const size_t smem = (NBX + 1) * c_tile(N);
-      ColGeo g{NHP, n * NHP, NH, (NH + TW - 1) / TW, nb * N, nb > 1 ? N : 0, n * n * NHP};
-      launch_persistent(k_poisson_x<N, NBX, T, MR>, T, smem, g.outer * g.col_tiles, s, s0, spec, comp, g, pp, deconv, tw);
-    }
-    // 4. y inverse: slot 0 (x component), then slots 1, 2 (y, z components) from the potential
-    cols_pass<N, MR>(spec, comp, 1, ColGeo{n * NHP, NHP, NH, 0, nb * N}, 1, tw, s);
-    {
-      constexpr int T = threads_for<N, MR>();
-      constexpr int NBY = 3 * c_tile(N) <= SMEM_LIMIT ? 2 : 1;
-      const size_t smem = (NBY + 1) * c_tile(N);
-      ColGeo g{n * NHP, NHP, NH, (NH + TW - 1) / TW, nb * N};
-      launch_persistent(k_grad_yz<N, NBY, T, MR>, T, smem, g.outer * g.col_tiles, s, spec, comp, g, pp, tw);
-    }
-  }
-  if constexpr (2 * c_tile(N) > SMEM_LIMIT) {
-    // 4. y inverse on the three component spectra
-    cols_pass<N, MR>(spec, comp, 3, ColGeo{n * NHP, NHP, NH, 0, N}, 1, tw, s);
-  }
-  {  // 5. z: C2R with 1/n^3
-    constexpr int T = threads_for<M, MR>();
-    constexpr int NB = 2 * c_tile(M + 1) <= SMEM_LIMIT ? 2 : 1;
-    const size_t smem = NB * c_tile(M + 1);
-    launch_persistent(k_c2r_z<N, NB, T, MR>, T, smem, 3 * row_tiles, s, spec, comp, gx, gy, gz, pp.scale, rows, tw);
-  }
+  // Slot 0 holds the forward spectrum; every pass reads a tile of it before it writes the same tile of
+  // slots 0..2, and tiles are disjoint, so the update in place is safe. y lines: columns along kz
+  // adjacent, outer = x (the x planes of a batch's boxes form one run); x lines: outer = y.
+  const ColGeo gy{n * NHP, NHP, NH, nb * N};
+  const ColGeo gxl{NHP, n * NHP, NH, nb * N, nb > 1 ? N : 0, n * n * NHP};
+  constexpr int TM = direct_threads<M, RW>(), TX = direct_threads<N, XW>(), TY = direct_threads<N, col_width(N)>();
+  const int rt = (rows + RW - 1) / RW;
+  constexpr bool ST = N >= STREAM_MESH;
+  launch_tiles(k_rows_r2c<N, TM, MR>, TM, direct_tile(M, RW), rt, s, delta, fx, std::ldexp(1.0f, -fx_shift), mean,
+               exact_inverse(mean), spec, rows, tw);
+  cols_direct<N, MR>(spec, 0, 1, gy, 0, tw, s);
+  launch_tiles(k_x_poisson<N, TX, MR, ST>, TX, 2 * direct_tile(N, XW), col_tile_count<XW>(gxl), s, spec, comp, gxl, pp,
+               deconv, tw);
+  launch_tiles(k_y_gradient<N, TY, MR, ST>, TY, direct_tile(N, col_width(N)), col_tile_count<col_width(N)>(gy), s, spec,
+               comp, gy, pp, tw);
+  launch_tiles(k_rows_c2r<N, TM, MR>, TM, direct_tile(M, RW), 3 * rt, s, spec, comp, gx, gy_out, gz, pp.scale, rows,
+               tw);
 }
 
 void launch_r2c3(const FftPlan& p, const float* delta, const unsigned long long* fx, int fx_shift, float mean,
@@ -1025,8 +789,6 @@ void launch_poisson(const FftPlan& p, const PoissonParams& pp, const float* delt
   case N:                                                                    \
     if (p.max_radix == 4)                                                    \
       poisson_n<N, 4>(p, pp, delta, fx, fx_shift, mean, spec, gx, gy, gz, s); \
-    else if (p.max_radix == 0)                                               \
-      poisson_n<N, 0>(p, pp, delta, fx, fx_shift, mean, spec, gx, gy, gz, s); \
     else                                                                     \
       poisson_n<N, 8>(p, pp, delta, fx, fx_shift, mean, spec, gx, gy, gz, s); \
     break;

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(PK_THREADS) k_pk_bin(const float2* __restrict_
     sc[s] = 0u;
   }
   __syncthreads();
-  const int nh = n / 2 + 1, nhp = n / 2 + 2;
+  const int nh = n / 2 + 1, nhp = half_row(n);
   const int runs = (nh + PK_RUN - 1) / PK_RUN;
   const long long items = (long long)n * n * runs;
   const double smax = (double)n_shells + 0.5;

@@ -263,8 +263,7 @@ static int sim_accelerations(cpm_sim* s, float a, const StepScalars* dev = nullp
 // own first state (after its first force evaluation, so the mesh, the sorted particles and the tree
 // are real), and the fastest is kept:
 //   FFT plan of the Poisson passes        Stockham stages of largest radix 8 (512 = 8.8.8) or 4
-//                                         (4.4.4.4.2) over the CTA, or (0) one warp per 256- or
-//                                         512-point line with register stages (radix 8 elsewhere)
+//                                         (4.4.4.4.2)
 //   deposit tile                          256 x {2, 4, 8} sorted particles per CTA
 //   walk group                            {2, 4, 8} warps of 32 particles per block
 // Each candidate runs once untimed and twice timed with CUDA events on the simulation's stream;
@@ -331,13 +330,14 @@ static int sim_autotune(cpm_sim* s) {
   PoissonParams pp =
       make_poisson_params(mn, s->box, s->P.cosmo.omega_m, s->a, r_split, (s->P.flags & CPM_SIM_DECONVOLVE) ? 1 : 0);
   pp.boxes = s->nb;
-  for (int k = 0; k < 3; ++k) {
+  for (int k = 0; k < 2; ++k) {
     s->plan.max_radix = TUNE_PLANS[k];
     c.ms[k] = time_ms(s->stream, e0, e1, [&] {
       launch_poisson(s->plan, pp, nullptr, as<unsigned long long>(s->fx), s->shift, s->mean, as<float2>(s->spec),
                      as<float>(s->gx), as<float>(s->gy), as<float>(s->gz), s->stream);
     });
   }
+  c.ms[2] = c.ms[0];  // plan 0 is plan 8
   for (int k = 0; k < 3; ++k) {
     c.ms[3 + k] = time_ms(s->stream, e0, e1, [&] {
       launch_deposit_fixed(as<float>(s->x), s->n, 1.0f, mn, s->h, s->shift, as<unsigned long long>(s->fx), s->stream,

@@ -341,8 +341,7 @@ int cpm_step_factors(const cpm_cosmology* cosmo, double a0, double a1, int fp64,
 /* No counterpart in the reference. The launch choices the autotuner made when the simulation was
  * created (each candidate timed on the simulation's own first state; cached per workload, and in the
  * file named by the environment variable CPM_TUNE_CACHE when set): the FFT plan of the Poisson passes
- * (8 or 4: shared-memory Stockham stages of largest radix 8 or 4 over the CTA; 0: one warp per
- * 256- or 512-point line with register stages, radix 8 for other lengths), the deposit tile (512,
+ * (8 or 4: Stockham stages of largest radix 8 or 4; 0: the same as 8), the deposit tile (512,
  * 1024 or 2048 sorted particles per CTA) and the walk group (2, 4 or 8 warps of 32 particles per
  * block). ms9 (may be NULL) receives the measured ms per call: plan 8, 4, 0; tile 512, 1024, 2048;
  * warps 2, 4, 8 (0 where not timed). */
