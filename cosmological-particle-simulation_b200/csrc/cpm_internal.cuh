@@ -240,12 +240,18 @@ struct TreeNodes {
   DevBuf quad;      // per node 2 float4: second moments about the centre of mass (quadrupole mode)
   bool has_quad = false;  // the last build computed `quad`; the walk then adds quadrupole terms
   int walk_warps = 4;     // warps (groups of 32 particles) per walk block: 2, 4 or 8 (autotuned)
+  bool trajectories = false;  // a simulation's tree: dense boxes take the ordered walk (see k_walk_ordered)
   uint32_t n_box = 0;     // batch of boxes: particles per box (a multiple of 32), root of group = box
   size_t capacity = 0;
   void* walk_fit = nullptr;  // fitted pair-force coefficients of the last split (walk.cu)
 };
-// The words after the n packed positions: 1 when a position lies outside [0, L]; the walk's group counter.
-constexpr int WALK_OUTSIDE = 0, WALK_TICKET = 1;
+// The words after the n packed positions: 1 when a position lies outside [0, L]; the walk's group counter;
+// per box of a batch (one box: the first) 1 when the build marked it dense: a node was split at least
+// ORDERED_DEPTH levels below the level of as many cells as the box has particles, and it has at most
+// ORDERED_PARTICLES of them (see k_walk_ordered).
+constexpr int WALK_OUTSIDE = 0, WALK_TICKET = 1, WALK_DENSE = 4, WALK_WORDS = 4 + 64;
+constexpr size_t ORDERED_PARTICLES = 1 << 20;
+constexpr int ORDERED_DEPTH = 4;
 inline uint32_t* tree_words(TreeNodes& t, size_t n) { return reinterpret_cast<uint32_t*>(static_cast<float4*>(t.x4.p) + n); }
 __device__ __forceinline__ bool outside_box(float a, float b, float c, float box) {
   return !(fminf(a, fminf(b, c)) >= 0.0f && fmaxf(a, fmaxf(b, c)) <= box);

@@ -429,7 +429,8 @@ __device__ __forceinline__ D3 chunk_prefix(const D3* chunk, const D3* totals, ui
 // Centre of mass of one node, and NODE_FLAT for an inner node whose children all have no octant-0
 // child (bit 0 of the mask, which the flag's store leaves as it is for the parents that read it).
 __device__ __forceinline__ void finish_node(uint32_t node, uint4* link, const float4* __restrict__ x4, const D3* chunk,
-                                            const D3* totals, float4* mass) {
+                                            const D3* totals, float4* mass, uint32_t dense_depth, uint32_t n_box,
+                                            uint32_t* words) {
   const uint4 L = __ldcg(link + node);
   D3 s;
   if (L.y - L.x <= SUM_DIRECT) {
@@ -442,6 +443,7 @@ __device__ __forceinline__ void finish_node(uint32_t node, uint4* link, const fl
   }
   const double c = (double)(L.y - L.x);
   mass[node] = make_float4((float)(s.x / c), (float)(s.y / c), (float)(s.z / c), (float)(L.y - L.x));
+  if ((L.w & 0xFFu) != 0u && ((L.w >> 8) & 0x7Fu) >= dense_depth) words[WALK_DENSE + (n_box ? L.x / n_box : 0u)] = 1u;
   if (L.w & 1u) {
     const uint32_t nch = (uint32_t)__popc(L.w & 0xFFu);
     uint32_t any = 0;
@@ -452,12 +454,13 @@ __device__ __forceinline__ void finish_node(uint32_t node, uint4* link, const fl
 
 __global__ void __launch_bounds__(BUILD_THREADS) k_tree_com(uint4* link, const float4* __restrict__ x4, const D3* chunk,
                                                             const D3* totals, float4* mass,
-                                                            const uint32_t* __restrict__ counters, uint32_t capacity) {
+                                                            const uint32_t* __restrict__ counters, uint32_t capacity,
+                                                            uint32_t dense_depth, uint32_t n_box, uint32_t* words) {
   uint32_t total = 0;
   for (int j = 0; j <= KEY_LEVELS; ++j) total += counters[j];
   total = min(total, capacity);
   for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < total; node += gridDim.x * blockDim.x)
-    finish_node(node, link, x4, chunk, totals, mass);
+    finish_node(node, link, x4, chunk, totals, mass, dense_depth, n_box, words);
 }
 
 // The top of a single box's tree: CTA 0 finds where each of the 8^TOP_LEVEL cells of level TOP_LEVEL
@@ -680,9 +683,9 @@ __global__ void k_tree_quad(const uint4* __restrict__ link, const float4* __rest
 }
 
 cudaError_t tree_positions(TreeNodes& t, size_t n, cudaStream_t s) {
-  cudaError_t e = ensure(t.x4, (n + 1) * sizeof(float4));
+  cudaError_t e = ensure(t.x4, n * sizeof(float4) + WALK_WORDS * sizeof(uint32_t));
   if (e != cudaSuccess) return e;
-  return cudaMemsetAsync(tree_words(t, n), 0, sizeof(float4), s);
+  return cudaMemsetAsync(tree_words(t, n), 0, WALK_WORDS * sizeof(uint32_t), s);
 }
 
 cudaError_t tree_pack(TreeNodes& t, const float* sorted_x3, size_t n, float box, cudaStream_t s) {
@@ -742,7 +745,12 @@ cudaError_t tree_build(TreeNodes& t, const uint64_t* sorted_keys, const float* s
                                                           roots, (uint32_t)n_box, link, geo, counters, capacity, totals,
                                                           tiles, st);
   count_launch();
-  k_tree_com<<<2 * BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, x4, chunk, totals, mass, counters, capacity);
+  // a node split at level d or below marks its box dense
+  int box_spread = 0;
+  for (size_t c = n_box ? n_box : n; c > 1; c >>= 3) ++box_spread;
+  const uint32_t dense_depth = (n_box ? n_box : n) <= ORDERED_PARTICLES ? (uint32_t)(box_spread + ORDERED_DEPTH) : 0x80u;
+  k_tree_com<<<2 * BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, x4, chunk, totals, mass, counters, capacity, dense_depth,
+                                                        (uint32_t)n_box, tree_words(t, n));
   t.has_quad = quad_half_max > 0.0f;
   if (t.has_quad) {
     if ((e = ensure(t.quad, 2 * t.capacity * sizeof(float4))) != cudaSuccess) return e;

@@ -97,6 +97,13 @@ struct PairConst2 {
   float2 eps2;        // softening^2
 };
 
+// The same for the ordered walk.
+struct OrderedConst {
+  float2 tiny, inv_two_rs, scale0, offset0;
+  float2 c0[FIT_DEG + 1];
+  float2 neg_log2e, eps2, neg_m;
+};
+
 struct WalkParams {
   float box;
   float guard;  // |x| below this: round(x / L) == 0 exactly
@@ -116,6 +123,7 @@ struct WalkParams {
   uint32_t n_box;  // batch of boxes: particles per box (multiple of 32); a warp starts at root i / n_box
   SFit fit;
   PairConst2 p2;
+  OrderedConst ordered;
 };
 
 // ------------------------------------------------------------------ host: the fit of R(u)
@@ -546,9 +554,14 @@ __device__ __forceinline__ void quad_term(float d0, float d1, float d2, const fl
   A2.y += a * d2 + b * (tr * d2 + 2.0f * td2);
 }
 
+// Whether box `box` takes the ordered walk (positions outside the box take the other one's strict tests).
+__device__ __forceinline__ bool walk_ordered(const uint32_t* __restrict__ words, uint32_t box) {
+  return words[WALK_DENSE + box] != 0u && words[WALK_OUTSIDE] == 0u;
+}
+
 // One warp (or `team` warps of a block, each with its share of the direct nodes and accepted nodes)
 // walks for a group of 32 particles.
-template <bool QUAD, bool LIST, int WARPS>
+template <bool QUAD, bool LIST, int WARPS, bool SKIP = false>
 __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_walk(const uint4* __restrict__ link,
                                                             const float4* __restrict__ geo,
                                                             const float4* __restrict__ mass,
@@ -590,7 +603,10 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
     const size_t t = (size_t)ticket * 32 + lane;
     const bool valid = t < walked;
     const size_t i = LIST ? (valid ? (size_t)list[t] : 0) : t;
-    const unsigned group = __ballot_sync(FULL, valid);
+    const unsigned lanes = __ballot_sync(FULL, valid);
+    // (SKIP: the groups of boxes that k_walk_ordered walks are left out)
+    const bool elsewhere = SKIP && lanes && walk_ordered(words, ticket / (w.n_box ? w.n_box / 32 : 0x7FFFFFFFu));
+    const unsigned group = elsewhere ? 0u : lanes;
     const float4 xi = valid ? __ldg(x4 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const float x0 = xi.x, x1 = xi.y, x2 = xi.z;
     const uint32_t self = (uint32_t)i;
@@ -918,7 +934,7 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
     }
     // tree.rs:61-66 multiplies every pair by the coupling K; here the unit-coupling sum is scaled once
     const float a0 = kk * s0, a1 = kk * s1, a2 = kk * s2;
-    if (valid && sub == 0) {
+    if (valid && sub == 0 && !elsewhere) {
       if (accumulate) {
         acc3[3 * i] = __fadd_rn(acc3[3 * i], a0);
         acc3[3 * i + 1] = __fadd_rn(acc3[3 * i + 1], a1);
@@ -930,6 +946,450 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
       }
     }
     __syncwarp();
+  }
+  if (counters) {
+    unsigned long long p = n_pairs, a = n_accepts, c = n_cand;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      p += __shfl_xor_sync(FULL, p, o);
+      a += __shfl_xor_sync(FULL, a, o);
+      c += __shfl_xor_sync(FULL, c, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&counters[0], p);
+      atomicAdd(&counters[1], a);
+      atomicAdd(&counters[2], c);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The walk in the order of the reference's chunks. Every lane classifies every node of a step, the step's direct
+// sums follow at once, in chunks of 32 sources of the concatenated nodes, and a lane adds its pairs of a chunk
+// two by two: the order in which a particle's terms are added depends on nothing but the tree and the group.
+// It is slower than k_tree_walk (walk of 91,125 clustered particles 0.90 ms against 0.50) and serves the
+// boxes of up to ORDERED_PARTICLES particles in which the build split nodes ORDERED_DEPTH levels and more below
+// the level of a smooth distribution (WALK_DENSE): in their cores, where pairs lie closer than the softening,
+// one rounding of a position moves an acceleration by up to 1e-3 of the box's RMS, so that another
+// order of f32 sums shows there after ten steps (largest difference of an acceleration after 18 steps, of the
+// RMS, eight boxes each: 3.7e-4 where the deepest split is 4 levels below a smooth box's, 21^3 particles;
+// 8.6e-4 at 5 levels, 27^3; 1.2e-2 at 6, 64^3), and trajectories of such boxes are kept as they were. Larger
+// boxes go by statistics, and their walk is most of their step.
+// ---------------------------------------------------------------------------------------------
+constexpr int ORDERED_WARPS = 4;
+constexpr int ORDERED_MERGE_SP = 96;
+constexpr int ORDERED_STACK_CAP = ORDERED_MERGE_SP + SLOTS + 7 * KEY_LEVELS + 8;
+
+// pair_factor for two pairs at once (f32x2 arithmetic), unit coupling.
+__device__ __forceinline__ float2 ordered_factor(float2 r2, const WalkParams& w, const float* __restrict__ far) {
+  const OrderedConst& c = w.ordered;
+  const float2 rr = __fadd2_rn(r2, c.tiny);
+  const float2 r = __fmul2_rn(r2, make_float2(rsqrt_approx(rr.x), rsqrt_approx(rr.y)));
+  const float2 u = __fmul2_rn(r, c.inv_two_rs);
+  float2 S;
+  if (fmaxf(u.x, u.y) <= w.fit.umax0) {
+    const float2 x = __ffma2_rn(u, c.scale0, c.offset0);
+    float2 R = c.c0[FIT_DEG];
+#pragma unroll
+    for (int j = FIT_DEG - 1; j >= 0; --j) R = __ffma2_rn(R, x, c.c0[j]);
+    // e^{-u^2} = 2^{-uu log2 e} (1 - err) with uu + err = u*u exactly
+    const float2 uu = __fmul2_rn(u, u);
+    const float2 nerr = __ffma2_rn(__fmul2_rn(u, make_float2(-1.0f, -1.0f)), u, uu);
+    const float2 ea = __fmul2_rn(uu, c.neg_log2e);
+    const float2 e = make_float2(exp2_approx(ea.x), exp2_approx(ea.y));
+    S = __fmul2_rn(__ffma2_rn(e, nerr, e), R);
+  } else {
+    S = make_float2(short_range_S(u.x, w.fit, far), short_range_S(u.y, w.fit, far));
+  }
+  const float2 q = __fadd2_rn(r2, c.eps2);
+  const float2 rs = make_float2(rsqrt_approx(q.x), rsqrt_approx(q.y));
+  return __fmul2_rn(__fmul2_rn(c.neg_m, S), __fmul2_rn(__fmul2_rn(rs, rs), rs));
+}
+
+struct OrderedShared {
+  uint2 stack[ORDERED_STACK_CAP];          // (first node | (count - 1) << 29, lane mask): a batch of siblings
+  float4 geo[2][SLOTS];            // the current and the next step's nodes: centre, half
+  float4 mass[2][SLOTS];           //                                        centre of mass, count
+  uint4 link[2][SLOTS];            //                                        start, end, first child, child mask
+  float prune2[SLOTS];             // per node of the current step: prune radius^2
+  uint32_t dbeg[SLOTS], dend[SLOTS], dsrc[SLOTS];  // direct sums: node c's sources are positions
+                                                   // dbeg .. dend - 1 of the concatenation,
+                                                   // particles dsrc + (position - dbeg)
+  float nx[32], ny[32], nz[32];    // a chunk of direct-sum sources, negated: -x, -y, -z
+  float4 box_c, box_h;             // the warp's bounding box: centre, half extent (+ tolerance)
+};
+
+// Direct-sum phase 1 for one chunk: bit t set when source t of `reach` lies within r_cut of the lane's
+// particle, by the reference's own arithmetic: the differences and squares of two sources per instruction
+// (f32x2, each element rounded like the scalar operation), the sums scalar (a packed multiply feeding a packed
+// add can be contracted into one FMA).
+template <bool WRAP>
+__device__ __forceinline__ uint32_t ordered_pairs(const OrderedShared& sh, uint32_t reach, float x0, float x1, float x2,
+                                                  const WalkParams& w) {
+  uint32_t pm = 0;
+  const float2 X0 = make_float2(x0, x0), X1 = make_float2(x1, x1), X2 = make_float2(x2, x2);
+  while (reach) {
+    const int a = __ffs(reach) - 1;
+    reach &= reach - 1;
+    const int b = reach ? __ffs(reach) - 1 : a;
+    reach &= reach - 1;
+    float2 d0 = __fadd2_rn(X0, make_float2(sh.nx[a], sh.nx[b]));
+    float2 d1 = __fadd2_rn(X1, make_float2(sh.ny[a], sh.ny[b]));
+    float2 d2 = __fadd2_rn(X2, make_float2(sh.nz[a], sh.nz[b]));
+    if (WRAP) {
+      min_image3(d0.x, d1.x, d2.x, w);
+      min_image3(d0.y, d1.y, d2.y, w);
+    }
+    const float2 q0 = __fmul2_rn(d0, d0), q1 = __fmul2_rn(d1, d1), q2 = __fmul2_rn(d2, d2);
+    const float ra = __fadd_rn(__fadd_rn(q0.x, q1.x), q2.x), rb = __fadd_rn(__fadd_rn(q0.y, q1.y), q2.y);
+    pm |= ((uint32_t)!(ra > w.cut2) << a) | ((uint32_t)!(rb > w.cut2) << b);
+  }
+  return pm;
+}
+
+// Direct-sum phase 2: the pair forces of the sources in pm, two per iteration, added to the
+// packed accumulators (even and odd pairs).
+template <bool WRAP>
+__device__ __forceinline__ void chunk_forces(const OrderedShared& sh, uint32_t pm, float x0, float x1, float x2,
+                                             const WalkParams& w, const float* __restrict__ far, float2& A0,
+                                             float2& A1, float2& A2) {
+  const float2 X0 = make_float2(x0, x0), X1 = make_float2(x1, x1), X2 = make_float2(x2, x2);
+  while (pm) {
+    const int t1 = __ffs(pm) - 1;
+    pm &= pm - 1;
+    int t2 = t1;
+    float keep = 0.0f;  // a lone last pair is evaluated twice and its copy weighted by 0
+    if (pm) {
+      t2 = __ffs(pm) - 1;
+      pm &= pm - 1;
+      keep = 1.0f;
+    }
+    float2 d0 = __fadd2_rn(X0, make_float2(sh.nx[t1], sh.nx[t2]));
+    float2 d1 = __fadd2_rn(X1, make_float2(sh.ny[t1], sh.ny[t2]));
+    float2 d2 = __fadd2_rn(X2, make_float2(sh.nz[t1], sh.nz[t2]));
+    if (WRAP) {
+      min_image3(d0.x, d1.x, d2.x, w);
+      min_image3(d0.y, d1.y, d2.y, w);
+    }
+    const float2 r2 = __ffma2_rn(d2, d2, __ffma2_rn(d1, d1, __fmul2_rn(d0, d0)));
+    const float2 f = __fmul2_rn(ordered_factor(r2, w, far), make_float2(1.0f, keep));
+    A0 = __ffma2_rn(d0, f, A0);
+    A1 = __ffma2_rn(d1, f, A1);
+    A2 = __ffma2_rn(d2, f, A2);
+  }
+}
+
+template <bool QUAD>
+__global__ void __launch_bounds__(ORDERED_WARPS * 32) k_walk_ordered(const uint4* __restrict__ link,
+                                                            const float4* __restrict__ geo,
+                                                            const float4* __restrict__ mass,
+                                                            const float4* __restrict__ x4, size_t n,
+                                                            const __grid_constant__ WalkParams w,
+                                                            const float* __restrict__ far, float* __restrict__ acc3,
+                                                            int accumulate, unsigned long long* counters,
+                                                            DevStatus* st, const float* __restrict__ k_dev,
+                                                            const float4* __restrict__ quad,
+                                                            const uint32_t* __restrict__ words) {
+  // Dynamic shared memory: ORDERED_WARPS OrderedShared records, then (quadrupoles) the node index of each slot.
+  extern __shared__ __align__(16) unsigned char walk_smem[];
+  OrderedShared* shared = reinterpret_cast<OrderedShared*>(walk_smem);
+  uint32_t(*node_ids)[2][SLOTS] = reinterpret_cast<uint32_t(*)[2][SLOTS]>(walk_smem + ORDERED_WARPS * sizeof(OrderedShared));
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t i = ((size_t)blockIdx.x * ORDERED_WARPS + warp) * 32 + lane;
+  const bool valid = i < n;
+  const unsigned group = __ballot_sync(FULL, valid);
+  if (group == 0 || !walk_ordered(words, w.n_box ? (uint32_t)(i / w.n_box) : 0u)) return;
+  OrderedShared& sh = shared[warp];
+  const float4 xi = valid ? __ldg(x4 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float x0 = xi.x, x1 = xi.y, x2 = xi.z;
+  const uint32_t self = (uint32_t)i;
+
+  // Bounding box of the warp's particles (centre cg, half extent hg), for a conservative
+  // warp-level prune test: a node farther than r_cut + sqrt(3) half from the whole box is pruned
+  // by every lane, whose own test is then skipped.
+  float lo0 = valid ? x0 : INFINITY, lo1 = valid ? x1 : INFINITY, lo2 = valid ? x2 : INFINITY;
+  float hi0 = valid ? x0 : -INFINITY, hi1 = valid ? x1 : -INFINITY, hi2 = valid ? x2 : -INFINITY;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo0 = fminf(lo0, __shfl_xor_sync(FULL, lo0, o));
+    lo1 = fminf(lo1, __shfl_xor_sync(FULL, lo1, o));
+    lo2 = fminf(lo2, __shfl_xor_sync(FULL, lo2, o));
+    hi0 = fmaxf(hi0, __shfl_xor_sync(FULL, hi0, o));
+    hi1 = fmaxf(hi1, __shfl_xor_sync(FULL, hi1, o));
+    hi2 = fmaxf(hi2, __shfl_xor_sync(FULL, hi2, o));
+  }
+  if (lane == 0) {
+    const float tol = 1e-5f * w.box;  // far above the rounding of positions and differences
+    sh.box_c = make_float4(0.5f * (lo0 + hi0), 0.5f * (lo1 + hi1), 0.5f * (lo2 + hi2), 0.0f);
+    sh.box_h = make_float4(0.5f * (hi0 - lo0) + tol, 0.5f * (hi1 - lo1) + tol, 0.5f * (hi2 - lo2) + tol, 0.0f);
+  }
+  // Accumulators of the even and odd pairs (x: even pairs and accepted nodes).
+  float2 A0 = make_float2(0.0f, 0.0f), A1 = A0, A2 = A0;
+  uint32_t n_pairs = 0, n_accepts = 0, n_cand = 0;
+
+  // A step of the walk handles up to SLOTS nodes, one per lane: one or more stack entries (each the
+  // children of an opened node, with the mask of the lanes that opened it) placed in consecutive
+  // slots. `mine` holds the slots this lane walks. Lane c copies slot c's three records into shared
+  // buffer `cur` asynchronously; the next step's copies are in flight while the current step is
+  // summed. The walk starts at the root: node 0, or in a batch of boxes the root of the warp's box
+  // (nodes 0 .. boxes - 1; a box's particles fill whole warps, and a list keeps each box's
+  // particles in whole warps, so the first valid lane's box is the warp's).
+  const uint32_t root = w.n_box ? __shfl_sync(FULL, (uint32_t)(i / w.n_box), __ffs(group) - 1) : 0u;
+  uint32_t b_count = 1, mine = (group >> lane) & 1u;
+  int cur = 0;
+  if (lane == 0) {
+    cp_async16(&sh.geo[0][0], geo + root);
+    cp_async16(&sh.mass[0][0], mass + root);
+    cp_async16(&sh.link[0][0], link + root);
+    if constexpr (QUAD) node_ids[warp][0][0] = root;
+  }
+  int sp = 0;
+  for (;;) {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncwarp();
+    const float4* bgeo = sh.geo[cur];
+    const float4* bmass = sh.mass[cur];
+    const uint4* blink = sh.link[cur];
+
+    // Warp-level prune test, lane c for node c. It applies where no lane can need a periodic
+    // image (|centre - x| < 0.49 L on every axis for the whole box), so that the lanes' own
+    // distances are the raw differences; it keeps a node unless even the box's nearest point is
+    // beyond r_cut + sqrt(3) half by a relative margin of 1e-5.
+    bool keep = false, far_edge = false, direct = false;
+    if ((uint32_t)lane < b_count) {
+      const float4 bc = sh.box_c, bh = sh.box_h, pg = bgeo[lane];
+      const float e0 = fabsf(pg.x - bc.x), e1 = fabsf(pg.y - bc.y), e2 = fabsf(pg.z - bc.z);
+      const float mr = __fadd_rn(w.r_cut, __fmul_rn(SQRT_3, pg.w));
+      sh.prune2[lane] = __fmul_rn(mr, mr);
+      direct = (blink[lane].w & 1u) == 0u;
+      keep = true;
+      const float emax = fmaxf(e0 + bh.x, fmaxf(e1 + bh.y, e2 + bh.z));
+      if (emax < w.guard) {
+        const float g0 = fmaxf(e0 - bh.x, 0.0f), g1 = fmaxf(e1 - bh.y, 0.0f), g2 = fmaxf(e2 - bh.z, 0.0f);
+        keep = !(g0 * g0 + g1 * g1 + g2 * g2 > mr * mr * 1.00001f);
+      }
+      // No lane needs a periodic image for this node: every difference between a lane's
+      // particle and the node's centre, centre of mass or particles (all inside the cube) is
+      // below 0.49 L on every axis.
+      far_edge = emax + pg.w < w.guard;
+    }
+    const uint32_t cand = __ballot_sync(FULL, keep);
+    const uint32_t nwall = __ballot_sync(FULL, far_edge);
+    const uint32_t dbits = __ballot_sync(FULL, direct);
+    __syncwarp();
+
+    // Classify every remaining node of this lane for its particle: prune, direct sum, accept or open.
+    uint32_t dmask = 0, nwmask = 0, amask = 0, omask = 0;
+    const uint32_t todo = cand & mine;
+    if ((todo & ~nwall) == 0u) {
+      // No node of the step involves a periodic image: raw differences.
+      for (uint32_t rem = todo; rem; rem &= rem - 1) {
+        const uint32_t c = __ffs(rem) - 1;
+        const float4 G = bgeo[c];
+        const float P = sh.prune2[c];
+        const float t0 = __fsub_rn(G.x, x0), t1 = __fsub_rn(G.y, x1), t2 = __fsub_rn(G.z, x2);
+        if (norm2(t0, t1, t2) > P) continue;
+        if ((dbits >> c) & 1u) {
+          dmask |= 1u << c;
+          continue;
+        }
+        const float4 M = bmass[c];
+        const float s0 = __fsub_rn(M.x, x0), s1 = __fsub_rn(M.y, x1), s2 = __fsub_rn(M.z, x2);
+        if (accept_node_sq(norm2(s0, s1, s2), bgeo[c].w, w))
+          amask |= 1u << c;
+        else
+          omask |= 1u << c;
+      }
+      nwmask = dmask;
+    } else {
+      for (uint32_t rem = todo; rem; rem &= rem - 1) {
+        const uint32_t c = __ffs(rem) - 1;
+        const float4 G = bgeo[c];
+        const float P = sh.prune2[c];
+        float t0 = __fsub_rn(G.x, x0), t1 = __fsub_rn(G.y, x1), t2 = __fsub_rn(G.z, x2);
+        // every source y of the node lies in [centre - half, centre + half]
+        const bool nowrap = fmaxf(fabsf(t0), fmaxf(fabsf(t1), fabsf(t2))) + G.w < w.guard;
+        min_image3(t0, t1, t2, w);
+        if (norm2(t0, t1, t2) > P) continue;
+        if ((dbits >> c) & 1u) {
+          // children[0] == NO_CHILD: direct sum over the node's particles (tree.rs:286-298)
+          dmask |= 1u << c;
+          nwmask |= (uint32_t)nowrap << c;
+          continue;
+        }
+        const float4 M = bmass[c];
+        float s0 = __fsub_rn(M.x, x0), s1 = __fsub_rn(M.y, x1), s2 = __fsub_rn(M.z, x2);
+        min_image3(s0, s1, s2, w);
+        if (accept_node_sq(norm2(s0, s1, s2), bgeo[c].w, w))
+          amask |= 1u << c;
+        else
+          omask |= 1u << c;
+      }
+    }
+
+    // Push the opened nodes' children as new stack entries (any order gives each lane the same
+    // set of interactions; only the order of its sums differs). Higher slots go deeper into the
+    // stack, so that the entries popped first, which fill the lowest slots, have their children
+    // popped first again.
+    const uint32_t ouni = __reduce_or_sync(FULL, omask);
+    if (ouni) {
+      uint32_t opened_by = 0;
+      for (uint32_t rem = ouni; rem; rem &= rem - 1) {
+        const int c = __ffs(rem) - 1;
+        const uint32_t b = __ballot_sync(FULL, (omask >> c) & 1u);
+        if (lane == c) opened_by = b;
+      }
+      const int npush = __popc(ouni);
+      // (node indices above 29 bits, trees of more than 2^28 particles, do not fit an entry)
+      const bool wide = __any_sync(FULL, ((ouni >> lane) & 1u) && (blink[lane].z >> FIRST_BITS) != 0u);
+      if (sp + npush > ORDERED_STACK_CAP || wide) {
+        if (lane == 0) dev_fail(st, DEV_STACK_OVERFLOW, sp);
+        break;
+      }
+      if ((ouni >> lane) & 1u) {
+        const uint4 L = blink[lane];
+        const int slot = sp + __popc(ouni >> lane) - 1;
+        sh.stack[slot] = make_uint2(L.z | ((uint32_t)(__popc(L.w & 0xFFu) - 1) << FIRST_BITS), opened_by);
+      }
+      sp += npush;
+      __syncwarp();
+    }
+
+    // Pop the next step: the top entry, and while the stack is shallow, further entries as long as
+    // they fit in the slots. Its copies complete during the work below.
+    uint32_t nx_count = 0, nx_mine = 0;
+    if (sp > 0) {
+      const bool merge = sp <= ORDERED_MERGE_SP;
+      for (;;) {
+        const uint2 e = sh.stack[--sp];
+        const uint32_t first = e.x & ((1u << FIRST_BITS) - 1u), cnt = (e.x >> FIRST_BITS) + 1u;
+        if ((uint32_t)lane >= nx_count && (uint32_t)lane < nx_count + cnt) {
+          const uint32_t node = first + ((uint32_t)lane - nx_count);
+          cp_async16(&sh.geo[cur ^ 1][lane], geo + node);
+          cp_async16(&sh.mass[cur ^ 1][lane], mass + node);
+          cp_async16(&sh.link[cur ^ 1][lane], link + node);
+          if constexpr (QUAD) node_ids[warp][cur ^ 1][lane] = node;
+        }
+        if ((e.y >> lane) & 1u) nx_mine |= bit_span(nx_count, cnt);
+        nx_count += cnt;
+        if (!merge || sp == 0 || nx_count + (sh.stack[sp - 1].x >> FIRST_BITS) + 1u > (uint32_t)SLOTS) break;
+      }
+    }
+
+    // Accepted centres of mass (tree.rs:299-305).
+    for (; amask; amask &= amask - 1) {
+      const int c = __ffs(amask) - 1;
+      const float4 M = bmass[c];
+      float s0 = __fsub_rn(M.x, x0), s1 = __fsub_rn(M.y, x1), s2 = __fsub_rn(M.z, x2);
+      min_image3(s0, s1, s2, w);
+      const float f = pair_factor(norm2(s0, s1, s2), -M.w, w, far);
+      A0.x = fmaf(-s0, f, A0.x);
+      A1.x = fmaf(-s1, f, A1.x);
+      A2.x = fmaf(-s2, f, A2.x);
+      if constexpr (QUAD) {
+        const size_t node = node_ids[warp][cur][c];
+        quad_term(s0, s1, s2, __ldg(quad + 2 * node), __ldg(quad + 2 * node + 1), w, A0, A1, A2);
+      }
+      ++n_accepts;
+    }
+
+    // Direct sums: the sources of all direct nodes of the step, concatenated in slot order, in
+    // chunks of 32.
+    const uint32_t dset = __reduce_or_sync(FULL, dmask);
+    if (dset) {
+      uint32_t cnt = 0, first = 0;
+      if ((dset >> lane) & 1u) {
+        const uint4 L = blink[lane];
+        cnt = L.y - L.x;
+        first = L.x;
+      }
+      uint32_t end = cnt;  // inclusive prefix sum over the slots
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, end, o);
+        if (lane >= o) end += v;
+      }
+      sh.dbeg[lane] = end - cnt;
+      sh.dend[lane] = end;
+      sh.dsrc[lane] = first;
+      const uint32_t total = __shfl_sync(FULL, end, 31);
+      __syncwarp();
+      // This lane's candidates, and its own particle's position in the concatenation (j != i).
+      uint32_t selfpos = 0xffffffffu;
+      for (uint32_t rem = dmask; rem; rem &= rem - 1) {
+        const int c = __ffs(rem) - 1;
+        const uint32_t b0 = sh.dbeg[c], e0 = sh.dend[c], f0 = sh.dsrc[c];
+        n_cand += e0 - b0;
+        if (self - f0 < e0 - b0) selfpos = b0 + (self - f0);
+      }
+      const bool wrap = (dmask & ~nwmask) != 0u;
+      uint32_t open_d = dmask;  // this lane's direct nodes not yet wholly behind the current chunk
+      for (uint32_t base = 0; base < total; base += 32) {
+        // Lane q loads source base + q: node c, the last with dbeg <= base + q (binary search).
+        const uint32_t g = base + (uint32_t)lane;
+        bool near = false;
+        if (g < total) {
+          int c = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1)
+            if (sh.dend[c + step - 1] <= g) c += step;
+          const float4 y = __ldg(x4 + sh.dsrc[c] + (g - sh.dbeg[c]));
+          sh.nx[lane] = -y.x;
+          sh.ny[lane] = -y.y;
+          sh.nz[lane] = -y.z;
+          const float4 bc = sh.box_c, bh = sh.box_h;
+          const float g0 = axis_gap(y.x, bc.x, bh.x, 0.0f, w.box), g1 = axis_gap(y.y, bc.y, bh.y, 0.0f, w.box),
+                      g2 = axis_gap(y.z, bc.z, bh.z, 0.0f, w.box);
+          near = !(g0 * g0 + g1 * g1 + g2 * g2 > w.cull2);
+        }
+        const uint32_t reach = __ballot_sync(FULL, near);  // the sources within r_cut of the warp's box
+        // `live`: the chunk positions of this lane's direct nodes, without its own particle.
+        const uint32_t top = base + 32u;
+        uint32_t live = 0;
+        while (open_d) {
+          const int c = __ffs(open_d) - 1;
+          const uint32_t b0 = sh.dbeg[c], e0 = sh.dend[c];
+          if (b0 >= top) break;
+          const uint32_t lo = max(b0, base), hi = min(e0, top);
+          live |= bit_span(lo - base, hi - lo);
+          if (e0 > top) break;
+          open_d &= open_d - 1;
+        }
+        if (selfpos - base < 32u) live &= ~(1u << (selfpos - base));
+        __syncwarp();
+        live &= reach;
+        if (live) {
+          const uint32_t pairs = (wrap ? ordered_pairs<true>(sh, reach, x0, x1, x2, w)
+                                       : ordered_pairs<false>(sh, reach, x0, x1, x2, w)) & live;
+          n_pairs += __popc(pairs);
+          if (wrap)
+            chunk_forces<true>(sh, pairs, x0, x1, x2, w, far, A0, A1, A2);
+          else
+            chunk_forces<false>(sh, pairs, x0, x1, x2, w, far, A0, A1, A2);
+        }
+        __syncwarp();
+      }
+    }
+    if (nx_count == 0) break;
+    b_count = nx_count;
+    mine = nx_mine;
+    cur ^= 1;
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  // tree.rs:61-66 multiplies every pair by the coupling K; here the unit-coupling sum is scaled once
+  const float kk = k_dev ? *k_dev : w.k;
+  const float a0 = kk * (A0.x + A0.y), a1 = kk * (A1.x + A1.y), a2 = kk * (A2.x + A2.y);
+  if (valid) {
+    if (accumulate) {
+      acc3[3 * i] = __fadd_rn(acc3[3 * i], a0);
+      acc3[3 * i + 1] = __fadd_rn(acc3[3 * i + 1], a1);
+      acc3[3 * i + 2] = __fadd_rn(acc3[3 * i + 2], a2);
+    } else {
+      acc3[3 * i] = a0;
+      acc3[3 * i + 1] = a1;
+      acc3[3 * i + 2] = a2;
+    }
   }
   if (counters) {
     unsigned long long p = n_pairs, a = n_accepts, c = n_cand;
@@ -1013,14 +1473,25 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
   for (int j = 0; j <= FIT_DEG; ++j) w.p2.c0[j] = dup(fc.fit.c0[j]);
   w.p2.exp_scale = dup((float)(-1.4426950408889634 * inv_two_rs * inv_two_rs));
   w.p2.eps2 = dup(w.eps2);
+  w.ordered.tiny = dup(1e-30f);
+  w.ordered.inv_two_rs = dup(w.inv_two_rs);
+  w.ordered.scale0 = dup(fc.fit.scale0);
+  w.ordered.offset0 = dup(fc.fit.offset0);
+  for (int j = 0; j <= FIT_DEG; ++j) w.ordered.c0[j] = dup(fc.fit.c0[j]);
+  w.ordered.neg_log2e = dup(-1.44269504f);
+  w.ordered.eps2 = dup(w.eps2);
+  w.ordered.neg_m = dup(-1.0f);
   const size_t groups = (n + 31) / 32;
+  const bool ordered = t.trajectories && !list && (t.n_box ? t.n_box : n) <= ORDERED_PARTICLES;
   // warps per block: the autotuned group count for the plain and list walks; 4 with quadrupoles
   // A batch goes by the groups of one box, so that a box's sums are those of its own simulation.
   const size_t box_groups = t.n_box ? (t.n_box + 31) / 32 : groups;
   const int team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
-  const int warps = t.has_quad || team > 1 ? 4 : (t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
+  const int warps = t.has_quad || team > 1 || ordered ? 4 : (t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
   unsigned blocks = (unsigned)((groups * team + warps - 1) / warps);
-  auto kernel = t.has_quad ? (list ? k_tree_walk<true, true, 4> : k_tree_walk<true, false, 4>)
+  auto kernel = t.has_quad ? (list ? k_tree_walk<true, true, 4> : ordered ? k_tree_walk<true, false, 4, true>
+                                                                          : k_tree_walk<true, false, 4>)
+              : ordered    ? k_tree_walk<false, false, 4, true>
               : warps == 2 ? (list ? k_tree_walk<false, true, 2> : k_tree_walk<false, false, 2>)
               : warps == 8 ? (list ? k_tree_walk<false, true, 8> : k_tree_walk<false, false, 8>)
                            : (list ? k_tree_walk<false, true, 4> : k_tree_walk<false, false, 4>);
@@ -1038,6 +1509,17 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
                                          static_cast<const float*>(fc.far_dev.p), acc3, accumulate,
                                          reinterpret_cast<unsigned long long*>(counters), st, k_dev, list, list_n,
                                          t.has_quad ? static_cast<const float4*>(t.quad.p) : nullptr, words, team);
+  if (ordered) {
+    auto second = t.has_quad ? k_walk_ordered<true> : k_walk_ordered<false>;
+    const size_t smem2 = ORDERED_WARPS * (sizeof(OrderedShared) + (t.has_quad ? 2 * SLOTS * sizeof(uint32_t) : 0));
+    if (smem2 > 48 * 1024) cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    count_launch();
+    second<<<(unsigned)((groups + ORDERED_WARPS - 1) / ORDERED_WARPS), ORDERED_WARPS * 32, smem2, s>>>(
+        static_cast<const uint4*>(t.link.p), static_cast<const float4*>(t.geo.p), static_cast<const float4*>(t.mass.p),
+        as<float4>(tm.x4), n, w, static_cast<const float*>(fc.far_dev.p), acc3, accumulate,
+        reinterpret_cast<unsigned long long*>(counters), st, k_dev,
+        t.has_quad ? static_cast<const float4*>(t.quad.p) : nullptr, words);
+  }
 }
 
 float quad_half_bound(const cpm_force_split& split) {

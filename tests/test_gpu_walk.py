@@ -58,3 +58,55 @@ def test_edges_of_the_box(cpm, orc):
 @pytest.mark.parametrize("n", [1, 8, 9, 33, 3552 * 32, 3552 * 32 + 1, 7104 * 32, 7104 * 32 + 33])
 def test_group_counts(cpm, orc, n):
     check(cpm, orc, clumped(n, 7), (0.12, 0.4, 0.01, 0.5))
+
+
+def dense(n):
+    """clumped() with a core at a corner of the box and one inside it."""
+    x = clumped(n, 9)
+    rng, m = np.random.default_rng(10), n // 5
+    x[:m] = np.mod(0.005 * rng.standard_normal((m, 3)) + np.array([[0.0], [7.3]])[np.arange(m) % 2], BOX)
+    return x % np.float32(BOX)
+
+
+def dense_simulation(cpm, x, split, flags):
+    cc = cpm.Cosmology(0.0, 0.3, 0.7, 70.0)
+    sim = cpm.Simulation(cc, BOX, 32, x, np.zeros_like(x), 0.5, cpm.ForceSplit(*split), flags=flags)
+    depth, spread = sim.tree_depth()["max_depth"], 0
+    while len(x) >> (3 * spread) > 1:
+        spread += 1
+    assert depth >= spread + 4
+    return sim
+
+
+@pytest.mark.parametrize("n,r_cut", [(500, 1.5), (4000, 4.0), (4000, 8.0), (33333, 0.7)])
+def test_dense_simulations_walk_in_order(cpm, orc, n, r_cut):
+    """A simulation whose tree is deep takes the ordered walk, the function call does not: both are the
+    oracle's force, of the same pairs and accepts."""
+    x, split = dense(n), (0.35, r_cut, 0.02, 0.5)
+    sim = dense_simulation(cpm, x, split, 0)
+    k = 1.5 * 0.3 * BOX ** 3 / (4.0 * np.pi * 0.5 * n)
+    sr = sim.short_range().astype(np.float64)
+    ref = orc.tree_accelerations_com64(x, BOX, orc.Split(*split), k).astype(np.float64)
+    assert np.sqrt(((sr - ref) ** 2).sum()) <= 1e-5 * np.sqrt((ref ** 2).sum())
+    stats = {}
+    cpm.tree_accelerations(x, BOX, cpm.ForceSplit(*split), k, stats=stats)
+    counters = sim.counters()
+    assert (counters["leaf_pairs"], counters["node_accepts"]) == (stats["leaf_pairs"], stats["node_accepts"])
+    sim.close()
+
+
+def test_dense_simulations_with_quadrupoles(cpm, orc):
+    """Quadrupole terms in the ordered walk: none where no node is accepted (theta = 0), and at theta 0.5
+    a smaller error against the sum over all pairs than without them."""
+    x, nat = dense(4000), cpm._native
+    exact = orc.tree_accelerations_com64(x, BOX, orc.Split(0.35, 1.5, 0.02, 0.0),
+                                         1.5 * 0.3 * BOX ** 3 / (4.0 * np.pi * 0.5 * len(x))).astype(np.float64)
+    sr = {}
+    for theta in (0.0, 0.5):
+        for flags in (0, nat.SIM_QUADRUPOLE):
+            sim = dense_simulation(cpm, x, (0.35, 1.5, 0.02, theta), flags)
+            sr[theta, flags] = sim.short_range().astype(np.float64)
+            sim.close()
+    assert np.array_equal(sr[0.0, 0], sr[0.0, nat.SIM_QUADRUPOLE])
+    err = [np.sqrt(((sr[0.5, f] - exact) ** 2).sum()) for f in (0, nat.SIM_QUADRUPOLE)]
+    assert err[1] < err[0]
