@@ -1,9 +1,17 @@
 // api.cu — the fine-grained C ABI (include/cpm.h): contexts and the per-function entry points
 // that stand in for mesh.rs, fft.rs, poisson.rs and tree.rs.
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "cpm_internal.cuh"
@@ -37,6 +45,62 @@ int check_device_once(std::string* err) {
   }
   state = 0;
   return CPM_OK;
+}
+
+// A copy to pageable memory that was never touched (a fresh numpy array) faults its pages in one by one,
+// 25 ms per 100 MB on one core against 8 ms for the copy itself. They are populated here in pieces of
+// PAGES_PIECE by this thread and up to PAGES_HELPERS more, while the steps launched before still run.
+// A piece that cannot be populated (older kernels, read-only or special mappings) is left to the copy.
+constexpr size_t PAGES_MIN = size_t(1) << 18, PAGES_PIECE = size_t(1) << 20;
+constexpr size_t PAGES_HELPERS = 3;
+
+void host_pages(std::initializer_list<HostSpan> spans) {
+#ifdef MADV_POPULATE_WRITE
+  struct Range {
+    uintptr_t begin, end;
+  };
+  Range ranges[8];
+  size_t n = 0, pieces = 0;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  for (const HostSpan& s : spans) {
+    if (!s.p || s.bytes < PAGES_MIN || n == 8) continue;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, s.p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
+      cudaGetLastError();
+      continue;
+    }
+    const uintptr_t b = (uintptr_t)s.p;
+    ranges[n] = {b / page * page, (b + s.bytes + page - 1) / page * page};
+    pieces += (ranges[n].end - ranges[n].begin + PAGES_PIECE - 1) / PAGES_PIECE;
+    ++n;
+  }
+  if (n == 0) return;
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t i; (i = next.fetch_add(1)) < pieces;) {
+      size_t r = 0;
+      for (;; ++r) {
+        const size_t c = (ranges[r].end - ranges[r].begin + PAGES_PIECE - 1) / PAGES_PIECE;
+        if (i < c) break;
+        i -= c;
+      }
+      const uintptr_t b = ranges[r].begin + i * PAGES_PIECE;
+      madvise((void*)b, std::min(PAGES_PIECE, (size_t)(ranges[r].end - b)), MADV_POPULATE_WRITE);
+    }
+  };
+  std::thread helpers[PAGES_HELPERS];
+  const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+  const size_t want = std::min({PAGES_HELPERS, pieces - 1, cores - 1});
+  try {
+    for (size_t k = 0; k < want; ++k) helpers[k] = std::thread(work);
+  } catch (const std::system_error&) {  // no more threads: those that started and this one do it
+  }
+  work();
+  for (std::thread& t : helpers)
+    if (t.joinable()) t.join();
+#else
+  (void)spans;
+#endif
 }
 
 }  // namespace cpm
@@ -209,6 +273,7 @@ static int deposit_common(cpm_ctx* c, const float* x3, size_t n, float mass, int
                        c->stream);
   const float mean = (float)n / (float)m;
   launch_fixed_to_f32(as<unsigned long long>(c->mesh_fx), m, shift, to_delta, mean, as<float>(c->mesh_a), c->stream);
+  host_pages({{out, m * sizeof(float)}});
   CPM_CU(c, cudaMemcpyAsync(out, c->mesh_a.p, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   return sync_and_check(c);
 }
@@ -284,6 +349,7 @@ int cpm_mesh_interpolate(cpm_ctx* c, const float* cells, const float* x3, size_t
   CPM_CU(c, ensure(c->out, n * sizeof(float)));
   launch_interpolate(as<float>(c->mesh_a), as<float>(c->x), n, c->n_mesh, c->box / (float)c->n_mesh, as<float>(c->out),
                      c->stream);
+  host_pages({{out, n * sizeof(float)}});
   CPM_CU(c, cudaMemcpyAsync(out, c->out.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   return sync_and_check(c);
 }
@@ -308,6 +374,7 @@ int cpm_mesh_interpolate3(cpm_ctx* c, const float* gx, const float* gy, const fl
   CPM_CU(c, ensure(c->acc, 3 * n * sizeof(float)));
   launch_interpolate3(as<float>(c->mesh_a), as<float>(c->mesh_b), as<float>(c->mesh_c), as<float>(c->x), n, c->n_mesh,
                       c->box / (float)c->n_mesh, as<float>(c->acc), c->stream);
+  host_pages({{out3, 3 * n * sizeof(float)}});
   CPM_CU(c, cudaMemcpyAsync(out3, c->acc.p, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   return sync_and_check(c);
 }
@@ -358,6 +425,7 @@ int cpm_poisson_accel(cpm_ctx* c, const float* delta, int n, const cpm_cosmology
   PoissonParams pp = make_poisson_params(n, c->box, cosmo->omega_m, a, r_split, 0);
   launch_poisson(c->plan, pp, as<float>(c->mesh_d), nullptr, 0, 0.0f, as<float2>(c->spec), as<float>(c->mesh_a),
                  as<float>(c->mesh_b), as<float>(c->mesh_c), c->stream);
+  host_pages({{gx, m * sizeof(float)}, {gy, m * sizeof(float)}, {gz, m * sizeof(float)}});
   CPM_CU(c, cudaMemcpyAsync(gx, c->mesh_a.p, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   CPM_CU(c, cudaMemcpyAsync(gy, c->mesh_b.p, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   CPM_CU(c, cudaMemcpyAsync(gz, c->mesh_c.p, m * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -412,6 +480,7 @@ int cpm_tree_accel(cpm_ctx* c, const float* x3, size_t n, float box_size, const 
   launch_tree_walk(c->tree, n, box_size, *split, k, as<float>(c->acc_sorted), 0,
                    as<TreeCounters>(c->tree_counters), as<DevStatus>(c->status), c->stream);
   launch_scatter3(as<float>(c->acc_sorted), as<uint32_t>(c->vals), n, as<float>(c->acc), c->stream);
+  host_pages({{acc3, 3 * n * sizeof(float)}});
   CPM_CU(c, cudaMemcpyAsync(acc3, c->acc.p, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   rc = sync_and_check(c);
   if (rc) return rc;

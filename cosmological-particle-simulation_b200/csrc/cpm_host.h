@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cmath>
+#include <initializer_list>
 #include <string>
 
 #include "cpm_internal.cuh"
@@ -14,6 +15,14 @@ namespace cpm {
 extern thread_local std::string g_last_error;
 int set_error(std::string* slot, int code, const std::string& msg);
 int check_device_once(std::string* err);
+
+// Backs the pages of host outputs before the copies write them, while the device still works (null
+// pointers, pinned and device memory, and small outputs are left alone; contents stay as they are).
+struct HostSpan {
+  const void* p;
+  size_t bytes;
+};
+void host_pages(std::initializer_list<HostSpan> spans);
 
 inline PoissonParams make_poisson_params(int n, float box, float omega_m, float a, float r_split, int deconvolve) {
   PoissonParams pp;

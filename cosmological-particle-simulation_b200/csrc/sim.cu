@@ -663,6 +663,8 @@ int cpm_sim_get_state(cpm_sim* s, float* x3, float* p3, float* acc3, float* delt
   const size_t n = s->n;
   const float* srcs[3] = {as<float>(s->x), as<float>(s->p), as<float>(s->acc)};
   float* dsts[3] = {x3, p3, acc3};
+  const size_t bytes = 3 * n * sizeof(float);
+  host_pages({{x3, bytes}, {p3, bytes}, {acc3, bytes}, {delta, mesh_cells(s) * (size_t)s->nb * sizeof(float)}});
   for (int q = 0; q < 3; ++q) {
     if (!dsts[q]) continue;
     launch_scatter3(srcs[q], as<uint32_t>(s->id), n, as<float>(s->x2), s->stream);
@@ -953,6 +955,7 @@ int cpm_sim_short_range(cpm_sim* s, float* sr3) {
   launch_tree_walk(s->tree, n, s->box, s->P.split, k, as<float>(s->host_tmp), 0, nullptr,
                    as<DevStatus>(s->status), s->stream);
   launch_scatter3(as<float>(s->host_tmp), as<uint32_t>(s->id), n, as<float>(s->x2), s->stream);
+  host_pages({{sr3, 3 * n * sizeof(float)}});
   SIM_CU(s, cudaMemcpyAsync(sr3, s->x2.p, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
   return sim_check(s);
 }
@@ -1212,8 +1215,9 @@ int cpm_ensemble_get_state(cpm_ensemble* e, int cls, int box, float* x3, float* 
     return set_error(e ? &e->err : nullptr, CPM_E_INVALID, "cpm_ensemble_get_state: bad ensemble or class");
   cpm_sim* s = e->classes[(size_t)cls];
   if (box < 0 || box >= s->nb) return set_error(&e->err, CPM_E_INVALID, "cpm_ensemble_get_state: bad box");
+  const size_t nb = s->n_box, off = (size_t)box * nb, bytes = 3 * nb * sizeof(float);
+  host_pages({{x3, bytes}, {p3, bytes}, {acc3, bytes}});
   SIM_CU(s, cudaStreamSynchronize(e->stream));
-  const size_t nb = s->n_box, off = (size_t)box * nb;
   const float* srcs[3] = {as<float>(s->x), as<float>(s->p), as<float>(s->acc)};
   float* dsts[3] = {x3, p3, acc3};
   for (int k = 0; k < 3; ++k) {
