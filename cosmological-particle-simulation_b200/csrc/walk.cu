@@ -37,8 +37,8 @@
 // 5.2, marking 5.1 and pair forces 9.0 thousand warp instructions, of 88 pairs per particle; in a
 // clustered state 12.7, 5.5, 9.4 and 24.8 thousand, of 325 pairs. Testing every particle against
 // every direct node and chunk of 32 sources, without the group's decisions, the culled window and
-// the flat nodes, this walk took 4.38 and 6.06 ms there; now 2.13 and 4.38 (256^3 / 512^3: 31.1,
-// now 16.0 ms).
+// the flat nodes, this walk took 4.38 and 6.06 ms there; now 2.03 and 4.28 (256^3 / 512^3: 31.1,
+// now 15.4 ms).
 //
 // Pair force. f = -K m S(r) / (r^2 + eps^2)^{3/2}, S(r) = erfc(u) + (2/sqrt(pi)) u e^{-u^2},
 // u = r / (2 r_s). S is evaluated as e^{-u^2} R(u) with R(u) = erfcx(u) + 2u/sqrt(pi), a smooth
@@ -69,8 +69,8 @@ constexpr int STACK_CAP = MERGE_SP + SLOTS + 7 * KEY_LEVELS + 8;
 constexpr int WINDOW = 448;   // direct-sum sources collected before they are summed (words of 32)
 // Groups are walked by teams of 2 or 4 warps while that keeps a launch within WALK_FILL warps (about
 // five rounds of the chip): the few groups of a small launch leave warps idle, and its time is that
-// of its slowest group. Walk of 91,125 clustered particles (2848 groups) 0.888 ms with single warps,
-// 0.600 with teams of 4; of 262,144 (8192 groups) 0.426 with single warps, 0.505 with teams of 2,
+// of its slowest group. Walk of 91,125 clustered particles (2848 groups, through the function call)
+// 0.888 ms with single warps, 0.500 with teams of 4; of 262,144 (8192 groups) 0.426 with single warps, 0.505 with teams of 2,
 // whose warps each repeat the traversal.
 constexpr size_t WALK_FILL = 148 * 96;
 constexpr int WALK_WARPS_PER_SM = 20;  // resident warps the register budget is set for
