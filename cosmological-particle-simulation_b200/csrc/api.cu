@@ -233,7 +233,7 @@ static int deposit_fixed_ctx(cpm_ctx* c, const float* x3, size_t n, float mass, 
     launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<DevStatus>(c->status),
                        c->stream);
     CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
-                              3 * KEY_LEVELS, c->sort, c->stream));
+                              3 * KEY_LEVELS, c->sort, as<DevStatus>(c->status), c->stream));
     launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
   }
   const float h = c->box / (float)c->n_mesh;
@@ -264,7 +264,7 @@ static int deposit_common(cpm_ctx* c, const float* x3, size_t n, float mass, int
     launch_octant_keys(as<float>(c->x), n, c->box, KEY_LEVELS, as<uint64_t>(c->keys), as<DevStatus>(c->status),
                        c->stream);
     CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
-                              3 * KEY_LEVELS, c->sort, c->stream));
+                              3 * KEY_LEVELS, c->sort, as<DevStatus>(c->status), c->stream));
     launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
   }
   const float h = c->box / (float)c->n_mesh;
@@ -474,7 +474,7 @@ int cpm_tree_accel(cpm_ctx* c, const float* x3, size_t n, float box_size, const 
   launch_octant_keys(as<float>(c->x), n, box_size, KEY_LEVELS, nullptr, as<DevStatus>(c->status), c->stream, 0,
                      as<uint64_t>(c->keys));
   CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n,
-                            3 * KEY_LEVELS, c->sort, c->stream));
+                            3 * KEY_LEVELS, c->sort, as<DevStatus>(c->status), c->stream));
   launch_permute3(as<float>(c->x), as<uint32_t>(c->vals), n, as<float>(c->x_sorted), c->stream);
   CPM_CU(c, tree_pack(c->tree, as<float>(c->x_sorted), n, box_size, c->stream));
   CPM_CU(c, tree_build(c->tree, as<uint64_t>(c->keys_sorted), as<float>(c->x_sorted), n, box_size,
@@ -516,7 +516,7 @@ int cpm_octant_keys(cpm_ctx* c, const float* x3, size_t n, float box_size, int l
   if (perm_out) {
     CPM_CU(c, ensure(c->keys_sorted, n * sizeof(uint64_t)));
     CPM_CU(c, radix_sort_keys(as<uint64_t>(c->keys), as<uint64_t>(c->keys_sorted), as<uint32_t>(c->vals), n, 3 * levels,
-                              c->sort, c->stream));
+                              c->sort, as<DevStatus>(c->status), c->stream));
     CPM_CU(c, cudaMemcpyAsync(perm_out, c->vals.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   }
   return sync_and_check(c);

@@ -22,6 +22,7 @@ enum DevError : int {
   DEV_NODE_CAPACITY = 2,    // octree needs more nodes than allocated
   DEV_STACK_OVERFLOW = 3,   // walk stack deeper than its bound
   DEV_DEPTH_LIMIT = 4,      // more than LEAF_SIZE particles share all key digits (informational)
+  DEV_WAIT_LIMIT = 5,       // a wait between CTAs of one launch ran out (Phases)
 };
 
 struct DevStatus {
@@ -32,6 +33,61 @@ struct DevStatus {
 __device__ __forceinline__ void dev_fail(DevStatus* st, int code, int detail) {
   if (atomicCAS(&st->code, 0, code) == 0) st->detail = detail;
 }
+
+// Phases of work over all CTAs of one launch, each beginning when the one before it is complete. The items of
+// all phases form one sequence; CTAs take them in order from a ticket counter, and whoever holds an item of a later
+// phase waits until all items of the earlier ones are done. Those are held by CTAs that run already, so nothing
+// has to be resident at once. Waits end after 2^32 cycles. Used by all threads of a CTA together; what one phase
+// writes for the next is read past L1.
+class Phases {
+ public:
+  // words[0]: the next ticket, words[1]: the items done; zero at launch
+  __device__ explicit Phases(uint32_t* words) : words_(words) {}
+  // The CTA's next item of the current phase of `count` items; false when it has no more.
+  __device__ bool take(uint32_t count, uint32_t& item) {
+    __shared__ uint32_t shared;
+    if (!held_) {
+      if (threadIdx.x == 0) shared = atomicAdd(words_, 1u);
+      __syncthreads();
+      ticket_ = shared;
+    }
+    held_ = ticket_ - base_ >= count;  // a ticket of a later phase is kept
+    item = ticket_ - base_;
+    return !held_;
+  }
+  // The taken item is complete.
+  __device__ void done() {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(words_ + 1, 1u);
+    }
+  }
+  // Ends a phase of `count` items after take() has returned false: waits until all of them are done.
+  __device__ bool next(uint32_t count) {
+    base_ += count;
+    int ok = 1;
+    if (threadIdx.x == 0) {
+      const long long t0 = clock64();
+      for (;;) {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(words_ + 1) : "memory");
+        if (v >= base_) break;
+        if (clock64() - t0 > (1ll << 32)) {
+          ok = 0;
+          break;
+        }
+        __nanosleep(32);
+      }
+    }
+    return __syncthreads_and(ok) != 0;
+  }
+
+ private:
+  uint32_t* words_;
+  uint32_t base_ = 0, ticket_ = 0;
+  bool held_ = false;
+};
 
 // Kernels launched by this library (every launch site calls count_launch() first).
 unsigned long long launch_count();
@@ -143,7 +199,7 @@ void launch_octant_keys(const float* x3, size_t n, float box, int levels, uint64
                         cudaStream_t s, size_t n_box = 0, uint64_t* hkeys = nullptr);
 // Stable sort of keys below 2^bits: sorted[i] = keys[perm[i]]; keys stays as it is.
 cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* perm, size_t n, int bits,
-                            SortScratch& sc, cudaStream_t s);
+                            SortScratch& sc, DevStatus* st, cudaStream_t s);
 // Exclusive scan of u32 (in place allowed); `tmp` is grown as needed.
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DevBuf& tmp, cudaStream_t s);
 

@@ -197,7 +197,7 @@ static int sim_accelerations(cpm_sim* s, float a, const StepScalars* dev = nullp
   launch_octant_keys(as<float>(s->x), n, s->box, s->levels, nullptr, as<DevStatus>(s->status), s->stream,
                      batch_box(s), as<uint64_t>(s->keys));
   SIM_CU(s, radix_sort_keys(as<uint64_t>(s->keys), as<uint64_t>(s->keys_sorted), as<uint32_t>(s->vals), n, 63, s->sort,
-                            s->stream));
+                            as<DevStatus>(s->status), s->stream));
   if (s->P.use_tree) SIM_CU(s, tree_positions(s->tree, n, s->stream));
   launch_reorder(as<uint32_t>(s->vals), n, as<float>(s->x), as<float>(s->p), as<uint32_t>(s->id),
                  fixed_point(s) ? as<uint32_t>(s->q) : nullptr, as<float>(s->x2), as<float>(s->p2),

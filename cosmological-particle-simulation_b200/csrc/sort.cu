@@ -363,9 +363,9 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DevB
 // 32-bit index); the last pass fetches each element's whole key. The particles of a simulation then
 // are in order but for short runs that share a cube of level 10 or 11 (0.16 of the mean spacing at
 // 256^3 particles; a handful of particles, a few hundred in the core of a cluster): a run of up to
-// RUN_SHORT elements is put in order by one thread, of up to RUN_MID by one warp, a longer one by one
-// CTA, whatever its length (a rank count in shared memory, or for runs over RUN_RANKED LSD passes over
-// the run). Eight passes of (u64 key, u32 index) moved 3.2 GB at 256^3 instead of 1.1.
+// RUN_SHORT elements is put in order by one thread, of up to RUN_MID by one warp, of up to RUN_BLOCK by one
+// CTA, and longer ones by LSD passes of the whole chip over these runs. At 256^3 the scatters move 1.3 GB and
+// the counts read 0.5; eight passes of (u64 key, u32 index) moved 3.2 and 1.1.
 //
 // Per pass: digit counts per tile of 4096 (digit-major), their exclusive scan (one CTA per digit), then
 // a stable scatter. Within a tile each warp ranks a contiguous sub-tile in warp-striped rounds (lanes with
@@ -380,6 +380,16 @@ constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
 static_assert(RS_THREADS == RS_BINS, "one thread per digit");
+
+constexpr int RUN_SHORT = 8;
+constexpr int RUN_MID = 256;
+constexpr int RUN_BLOCK_BITS = 12;
+constexpr int RUN_BLOCK = 1 << RUN_BLOCK_BITS;
+
+// The lists of runs: RUNS_LISTED of more than RUN_SHORT elements, their starts from RUNS_WORDS on; RUNS_LONG of
+// more than RUN_MID, their starts from the end downwards. Then the words of k_long_runs: its phases, and the
+// number of runs over RUN_BLOCK (upper half) and of their tiles.
+constexpr int RUNS_LISTED = 0, RUNS_LONG = 1, RUNS_PHASES = 2, RUNS_TILES = 4, RUNS_WORDS = 6;
 
 // The lanes whose 9-bit value d equals this lane's (a digit, or 0x100 | lane for a lane without
 // an element): one ballot per bit, the same mask as __match_any_sync.
@@ -403,7 +413,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const uint64_t* __res
                                                            uint32_t* __restrict__ runs) {
   __shared__ uint32_t h[RS_BINS];
   h[threadIdx.x] = 0;
-  if (runs && blockIdx.x == 0 && threadIdx.x < 2) runs[threadIdx.x] = 0;
+  if (runs && blockIdx.x == 0 && threadIdx.x < RUNS_WORDS) runs[threadIdx.x] = 0;
   __syncthreads();
   const size_t base = (size_t)blockIdx.x * RS_TILE;
   uint32_t v[RS_ITEMS];
@@ -534,13 +544,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint64_t* __
 // The runs of elements that share key >> drop, put in order by their lower bits (stable: a run arrives
 // in input order).
 // ---------------------------------------------------------------------------------------------
-constexpr int RUN_SHORT = 8;
-constexpr int RUN_MID = 256;
-constexpr int RUN_RANKED = 2048;
-
-// The lists of runs: runs[0] of more than RUN_SHORT elements, their starts from runs[2]; runs[1] of
-// more than RUN_MID, their starts from the end downwards.
-
 // The thread of a run's first element sorts it by insertion, or lists it.
 __global__ void k_short_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop, uint32_t* runs) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -552,7 +555,7 @@ __global__ void k_short_runs(uint64_t* sorted, uint32_t* perm, size_t n, int dro
   int len = 2;
   while (len <= RUN_SHORT && i + len < n && (keys[i + len] >> drop) == h) ++len;
   if (len > RUN_SHORT) {
-    runs[2 + atomicAdd(&runs[0], 1u)] = (uint32_t)i;
+    runs[RUNS_WORDS + atomicAdd(&runs[RUNS_LISTED], 1u)] = (uint32_t)i;
     return;
   }
   uint64_t* k = sorted + i;
@@ -577,9 +580,9 @@ __global__ void __launch_bounds__(256) k_mid_runs(uint64_t* sorted, uint32_t* pe
   constexpr int PER = RUN_MID / 32;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const uint32_t count = runs[0];
+  const uint32_t count = runs[RUNS_LISTED];
   for (uint32_t r = blockIdx.x * 8 + (threadIdx.x >> 5); r < count; r += gridDim.x * 8) {
-    const size_t start = runs[2 + r];
+    const size_t start = runs[RUNS_WORDS + r];
     const uint64_t h = sorted[start] >> drop;
     uint64_t k[PER];
     uint32_t v[PER];
@@ -596,7 +599,7 @@ __global__ void __launch_bounds__(256) k_mid_runs(uint64_t* sorted, uint32_t* pe
       len += __popc(__ballot_sync(FULL, in));
     }
     if (len == RUN_MID && start + RUN_MID < n && (sorted[start + RUN_MID] >> drop) == h) {
-      if (lane == 0) runs[runs_end - 1 - atomicAdd(&runs[1], 1u)] = (uint32_t)start;
+      if (lane == 0) runs[runs_end - 1 - atomicAdd(&runs[RUNS_LONG], 1u)] = (uint32_t)start;
       continue;
     }
     int place[PER] = {};
@@ -617,89 +620,234 @@ __global__ void __launch_bounds__(256) k_mid_runs(uint64_t* sorted, uint32_t* pe
   }
 }
 
-// One CTA per run of more than RUN_MID elements. Up to RUN_RANKED elements: every element's place is the number of elements
-// before it. Longer ones: LSD passes over the run through the scratch arrays, an even number of them.
-__global__ void __launch_bounds__(RS_THREADS) k_long_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop,
-                                                          const uint32_t* __restrict__ runs, uint32_t runs_end,
-                                                          uint64_t* kalt, uint32_t* valt) {
-  __shared__ uint64_t sk[RUN_RANKED];
-  __shared__ uint32_t sv[RUN_RANKED];
-  __shared__ uint32_t base[RS_BINS], wc[RS_WARPS][RS_BINS], ws[SC_THREADS / 32];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint64_t low = (1ull << drop) - 1ull;
-  for (uint32_t r = blockIdx.x; r < runs[1]; r += gridDim.x) {
-    const size_t start = runs[runs_end - 1 - r];
-    const uint64_t h = sorted[start] >> drop;
-    size_t len = 0;
-    for (int got = RS_THREADS; got == RS_THREADS; len += got) {
-      const size_t i = start + len + t;
-      got = __syncthreads_count(i < n && (sorted[i] >> drop) == h);
-    }
-    if (len <= (size_t)RUN_RANKED) {
-      for (int q = t; q < (int)len; q += RS_THREADS) {
-        sk[q] = sorted[start + q];
-        sv[q] = perm[start + q];
-      }
-      __syncthreads();
-      for (int q = t; q < (int)len; q += RS_THREADS) {
-        const uint64_t k = sk[q];
-        int place = 0;
-        for (int j = 0; j < (int)len; ++j) place += (int)(sk[j] < k || (sk[j] == k && j < q));
-        sorted[start + place] = k;
-        perm[start + place] = sv[q];
-      }
-      __syncthreads();
-      continue;
-    }
-    uint64_t *ka = sorted + start, *kb = kalt + start;
-    uint32_t *va = perm + start, *vb = valt + start;
-    const int passes = (drop + 15) / 16 * 2;
-    for (int p = 0; p < passes; ++p) {
-      const int shift = 8 * p;
-      base[t] = 0;
-      __syncthreads();
-      for (size_t i = t; i < len; i += RS_THREADS) atomicAdd(&base[(ka[i] & low) >> shift & (RS_BINS - 1)], 1u);
-      __syncthreads();
-      const uint32_t c = base[t];
-      uint32_t sum;
-      const uint32_t before = block_exclusive_scan(c, &sum, ws);
-      base[t] = before;
-      for (size_t i0 = 0; i0 < len; i0 += RS_THREADS) {  // in order, one element per thread
-        const size_t i = i0 + t;
-        const bool valid = i < len;
-        const uint64_t k = valid ? ka[i] : 0ull;
-        const uint32_t v = valid ? va[i] : 0u;
-        const uint32_t d = valid ? (uint32_t)((k & low) >> shift) & (RS_BINS - 1) : (0x100u | (uint32_t)lane);
-        const uint32_t peers = match_digit(d);
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) wc[w][t] = 0;
-        __syncthreads();
-        if (valid && (__ffs(peers) - 1) == lane) wc[warp][d] = (uint32_t)__popc(peers);
-        __syncthreads();
-        uint32_t run = base[t];  // thread t = digit t: where each warp's elements go
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) {
-          const uint32_t q = wc[w][t];
-          wc[w][t] = run;
-          run += q;
-        }
-        base[t] = run;
-        __syncthreads();
-        if (valid) {
-          const uint32_t pos = wc[warp][d] + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-          kb[pos] = k;
-          vb[pos] = v;
-        }
-        __syncthreads();
-      }
-      uint64_t* tk = ka;
-      ka = kb;
-      kb = tk;
-      uint32_t* tv = va;
-      va = vb;
-      vb = tv;
-    }
+// The runs of more than RUN_MID elements, in phases over all CTAs (Phases): first each run's end; runs of up to
+// RUN_BLOCK elements are sorted by one CTA in shared memory (bitonic, by the lower bits and then the place in the run).
+// The longer ones (a collapsed core in a large box, coincident particles) go through LSD passes together, cut into
+// tiles of LONG_TILE elements that each belong to one run: digit counts per tile, their scan per run and digit, the
+// scatter, which ranks as k_radix_scatter does. The work is that of these runs' elements and spread over the chip, so
+// the sort takes about as long for any input: 10^6 particles in one halo of 1e-4 of the box 0.31 ms with keys and reorder
+// (a uniform box 0.15), 4e6 0.87 (0.35); one CTA per run, of whatever length, took 12.9 and 53 ms.
+constexpr int LONG_ITEMS = 8;
+constexpr int LONG_TILE = RS_THREADS * LONG_ITEMS;
+constexpr int LONG_CTAS = 148 * 2;
+// The tables of these runs, in words that the caller provides: starts, ends, first tiles, digit totals, tile counts.
+// At most n / (RUN_BLOCK + 1) runs of n / LONG_TILE tiles and one more each: less than 0.26 n words.
+struct LongTables {
+  uint32_t *start, *end, *tile0, *totals, *hist;
+  __device__ LongTables(uint32_t* words, size_t n) {
+    const size_t cap = n / (RUN_BLOCK + 1);
+    start = words;
+    end = start + cap;
+    tile0 = end + cap;
+    totals = tile0 + cap;
+    hist = totals + cap * RS_BINS;
   }
+};
+
+__global__ void __launch_bounds__(RS_THREADS) k_long_runs(uint64_t* sorted, uint32_t* perm, size_t n, int drop,
+                                                          uint32_t* runs, uint32_t runs_end, uint64_t* kalt,
+                                                          uint32_t* valt, uint32_t* tables, DevStatus* st) {
+  __shared__ __align__(16) unsigned char smem[RUN_BLOCK * sizeof(uint64_t)];
+  __shared__ uint32_t wc[RS_WARPS][RS_BINS], gbase[RS_BINS], ws[SC_THREADS / 32];
+  static_assert(LONG_TILE * (sizeof(uint64_t) + sizeof(uint32_t)) <= sizeof(smem), "a tile in shared memory");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t nlong = runs[RUNS_LONG];
+  if (nlong == 0u) return;
+  const uint64_t low = (1ull << drop) - 1ull;
+  const LongTables T(tables, n);
+  Phases phases(runs + RUNS_PHASES);
+  uint32_t item;
+
+  uint64_t* comp = reinterpret_cast<uint64_t*>(smem);
+  while (phases.take(nlong, item)) {
+    const size_t start = runs[runs_end - 1 - item];
+    const uint64_t h = __ldcg(sorted + start) >> drop;
+    size_t lo = start + RUN_MID, hi = n;  // everything before lo is in the run, nothing from hi on
+    while (lo < hi) {
+      const size_t len = hi - lo;
+      const int in = __syncthreads_count((__ldcg(sorted + lo + len * t / RS_THREADS) >> drop) == h);
+      if (in < RS_THREADS) hi = lo + len * in / RS_THREADS;
+      if (in > 0) lo += len * (in - 1) / RS_THREADS + 1;
+    }
+    const uint32_t len = (uint32_t)(lo - start);
+    if (len > (uint32_t)RUN_BLOCK) {
+      if (t == 0) {
+        const unsigned long long tiles = (len + LONG_TILE - 1) / LONG_TILE;
+        const unsigned long long old =
+            atomicAdd(reinterpret_cast<unsigned long long*>(runs + RUNS_TILES), (1ull << 32) | tiles);
+        const uint32_t r = (uint32_t)(old >> 32);
+        __stcg(T.start + r, (uint32_t)start);
+        __stcg(T.end + r, (uint32_t)lo);
+        __stcg(T.tile0 + r, (uint32_t)old);
+      }
+    } else {
+      uint32_t size = 2 * RUN_MID;
+      while (size < len) size <<= 1;
+      for (uint32_t q = t; q < size; q += RS_THREADS)
+        comp[q] = q < len ? ((sorted[start + q] & low) << RUN_BLOCK_BITS) | q : ~0ull;
+      __syncthreads();
+      for (uint32_t k = 2; k <= size; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+          for (uint32_t q = t; q < size / 2; q += RS_THREADS) {
+            const uint32_t a = 2 * q - (q & (j - 1)), b = a + j;
+            const uint64_t x = comp[a], y = comp[b];
+            if ((x > y) == ((a & k) == 0u)) {
+              comp[a] = y;
+              comp[b] = x;
+            }
+          }
+          __syncthreads();
+        }
+      uint32_t v[RUN_BLOCK / RS_THREADS];
+#pragma unroll
+      for (int m = 0; m < RUN_BLOCK / RS_THREADS; ++m) {
+        const uint32_t q = t + m * RS_THREADS;
+        if (q < len) v[m] = perm[start + (comp[q] & (RUN_BLOCK - 1))];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < RUN_BLOCK / RS_THREADS; ++m) {
+        const uint32_t q = t + m * RS_THREADS;
+        if (q < len) {
+          sorted[start + q] = (h << drop) | (comp[q] >> RUN_BLOCK_BITS);
+          perm[start + q] = v[m];
+        }
+      }
+    }
+    phases.done();
+  }
+  bool ok = phases.next(nlong);
+  const unsigned long long found = __ldcg(reinterpret_cast<unsigned long long*>(runs + RUNS_TILES));
+  const uint32_t nrun = (uint32_t)(found >> 32), ntile = (uint32_t)found;
+  if (ok && nrun == 0u) return;
+
+  auto run_of = [&](uint32_t tile) {  // the last run that starts at or before the tile
+    uint32_t a = 0, b = nrun;
+    while (b - a > 1) {
+      const uint32_t m = (a + b) / 2;
+      if (__ldcg(T.tile0 + m) <= tile)
+        a = m;
+      else
+        b = m;
+    }
+    return a;
+  };
+  auto tiles_of = [&](uint32_t r) { return (__ldcg(T.end + r) - __ldcg(T.start + r) + LONG_TILE - 1) / LONG_TILE; };
+  uint64_t *ka = sorted, *kb = kalt, *sk = comp;
+  uint32_t *va = perm, *vb = valt, *sv = reinterpret_cast<uint32_t*>(sk + LONG_TILE);
+  const int passes = (drop + 15) / 16 * 2;  // an even number: the result is back in place
+  for (int p = 0; p < passes && ok; ++p) {
+    const int shift = 8 * p;
+    auto digit = [&](uint64_t k) { return (uint32_t)((k & low) >> shift) & (RS_BINS - 1); };
+    while (phases.take(ntile, item)) {
+      const uint32_t r = run_of(item), tile0 = __ldcg(T.tile0 + r), tile = item - tile0;
+      const size_t first = (size_t)__ldcg(T.start + r) + (size_t)tile * LONG_TILE;
+      const uint32_t count = min((uint32_t)LONG_TILE, __ldcg(T.end + r) - (uint32_t)first);
+      gbase[t] = 0;
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < LONG_ITEMS; ++j) {
+        const uint32_t q = t + j * RS_THREADS;
+        const bool valid = q < count;
+        const uint32_t d = valid ? digit(__ldcg(ka + first + q)) : 0u;
+        const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
+        const bool same = __all_sync(0xffffffffu, valid && d == d0);
+        if (same ? lane == 0 : valid) atomicAdd(&gbase[d], same ? 32u : 1u);
+      }
+      __syncthreads();
+      __stcg(T.hist + (size_t)tile0 * RS_BINS + (size_t)t * tiles_of(r) + tile, gbase[t]);
+      phases.done();
+    }
+    ok = phases.next(ntile);
+    while (ok && phases.take(nrun * (RS_BINS / RS_WARPS), item)) {  // a warp per run and digit
+      const uint32_t row = item * RS_WARPS + warp, r = row / RS_BINS, d = row % RS_BINS, tiles = tiles_of(r);
+      uint32_t* h = T.hist + (size_t)__ldcg(T.tile0 + r) * RS_BINS + (size_t)d * tiles;
+      uint32_t carry = 0;
+      for (uint32_t i0 = 0; i0 < tiles; i0 += 32) {
+        const uint32_t i = i0 + lane, x = i < tiles ? __ldcg(h + i) : 0u;
+        uint32_t incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        if (i < tiles) __stcg(h + i, carry + incl - x);
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) __stcg(T.totals + row, carry);
+      phases.done();
+    }
+    ok = ok && phases.next(nrun * (RS_BINS / RS_WARPS));
+    while (ok && phases.take(ntile, item)) {
+      const uint32_t r = run_of(item), tile0 = __ldcg(T.tile0 + r), tile = item - tile0;
+      const size_t start = __ldcg(T.start + r), first = start + (size_t)tile * LONG_TILE;
+      const uint32_t count = min((uint32_t)LONG_TILE, __ldcg(T.end + r) - (uint32_t)first);
+#pragma unroll
+      for (int w = 0; w < RS_WARPS; ++w) wc[w][t] = 0;
+      uint32_t sum;
+      const uint32_t before = __ldcg(T.hist + (size_t)tile0 * RS_BINS + (size_t)t * tiles_of(r) + tile) +
+                              block_exclusive_scan(__ldcg(T.totals + (size_t)r * RS_BINS + t), &sum, ws);
+      uint64_t k[LONG_ITEMS];
+      uint32_t v[LONG_ITEMS], rank[LONG_ITEMS];
+#pragma unroll
+      for (int j = 0; j < LONG_ITEMS; ++j) {
+        const uint32_t q = (uint32_t)(warp * LONG_ITEMS + j) * 32 + lane;
+        k[j] = q < count ? __ldcg(ka + first + q) : 0ull;
+        v[j] = q < count ? __ldcg(va + first + q) : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < LONG_ITEMS; ++j) {
+        const bool valid = (uint32_t)(warp * LONG_ITEMS + j) * 32 + lane < count;
+        const uint32_t d = valid ? digit(k[j]) : (0x100u | (uint32_t)lane);
+        const uint32_t peers = match_digit(d);
+        uint32_t prev = 0;
+        if (valid) prev = wc[warp][d];
+        __syncwarp();
+        rank[j] = prev + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        if (valid && (__ffs(peers) - 1) == lane) wc[warp][d] = prev + (uint32_t)__popc(peers);
+        __syncwarp();
+      }
+      __syncthreads();
+      uint32_t tot = 0;
+#pragma unroll
+      for (int w = 0; w < RS_WARPS; ++w) tot += wc[w][t];
+      uint32_t run = block_exclusive_scan(tot, &sum, ws);
+      gbase[t] = before - run;
+#pragma unroll
+      for (int w = 0; w < RS_WARPS; ++w) {
+        const uint32_t c = wc[w][t];
+        wc[w][t] = run;
+        run += c;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < LONG_ITEMS; ++j)
+        if ((uint32_t)(warp * LONG_ITEMS + j) * 32 + lane < count) {
+          const uint32_t q = wc[warp][digit(k[j])] + rank[j];
+          sk[q] = k[j];
+          sv[q] = v[j];
+        }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < LONG_ITEMS; ++j) {
+        const uint32_t q = t + j * RS_THREADS;
+        if (q < count) {
+          const size_t pos = start + (gbase[digit(sk[q])] + q);
+          __stcg(kb + pos, sk[q]);
+          __stcg(vb + pos, sv[q]);
+        }
+      }
+      phases.done();
+    }
+    ok = ok && phases.next(ntile);
+    uint64_t* tk = ka;
+    ka = kb;
+    kb = tk;
+    uint32_t* tv = va;
+    va = vb;
+    vb = tv;
+  }
+  if (!ok && t == 0) dev_fail(st, DEV_WAIT_LIMIT, (int)nlong);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -725,7 +873,7 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS)
   const uint32_t rounds = (n + SS_CTAS * SS_THREADS - 1) / (SS_CTAS * SS_THREADS);
   const uint32_t first = ((cta * SS_WARPS + warp) * rounds) * 32 + lane;
   const unsigned lt_mask = (1u << lane) - 1u;
-  if (runs && cta == 0 && t < 2) runs[t] = 0;
+  if (runs && cta == 0 && t < RUNS_WORDS) runs[t] = 0;
   for (int p = 0; p < passes; ++p) {
     // the last pass writes to `sorted`, the passes before it alternate
     const bool to_sorted = ((passes - 1 - p) & 1) == 0;
@@ -803,7 +951,7 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS)
 }
 
 cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* perm, size_t n, int bits,
-                            SortScratch& sc, cudaStream_t s) {
+                            SortScratch& sc, DevStatus* st, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (n > 0xFFFFFFFFull || bits < 1 || bits > 64) return cudaErrorInvalidValue;
   const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
@@ -817,7 +965,7 @@ cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* pe
   const int drop = std::max(0, bits - (small ? 24 : 32));
   uint32_t* runs = nullptr;
   // a listed run holds more than RUN_SHORT elements, one of the second list more than RUN_MID
-  const uint32_t runs_end = (uint32_t)(2 + n / (RUN_SHORT + 1) + n / (RUN_MID + 1) + 2);
+  const uint32_t runs_end = (uint32_t)(RUNS_WORDS + n / (RUN_SHORT + 1) + n / (RUN_MID + 1) + 2);
   if (drop) {
     if ((e = ensure(sc.runs, (size_t)runs_end * sizeof(uint32_t))) != cudaSuccess) return e;
     runs = as<uint32_t>(sc.runs);
@@ -850,8 +998,10 @@ cudaError_t radix_sort_keys(const uint64_t* keys, uint64_t* sorted, uint32_t* pe
     count_launch();
     k_mid_runs<<<(unsigned)std::min<size_t>(n / 2048 + 1, 148 * 8), 256, 0, s>>>(sorted, perm, n, drop, runs, runs_end);
     count_launch();
-    k_long_runs<<<148, RS_THREADS, 0, s>>>(sorted, perm, n, drop, runs, runs_end, as<uint64_t>(sc.pairs),
-                                           as<uint32_t>(sc.pairs_alt));
+    // pairs_alt: n indices, and the tables in its other half
+    uint32_t* valt = as<uint32_t>(sc.pairs_alt);
+    k_long_runs<<<LONG_CTAS, RS_THREADS, 0, s>>>(sorted, perm, n, drop, runs, runs_end, as<uint64_t>(sc.pairs), valt,
+                                                 valt + n, st);
   }
   return cudaGetLastError();
 }
