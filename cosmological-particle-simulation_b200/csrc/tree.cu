@@ -31,9 +31,12 @@ constexpr int TOP_LEVEL = 3;             // the levels down to it are made in on
 constexpr size_t CLUSTER_TAIL = 262144;  // particles up to which the deep levels start early in one cluster
 
 // counters layout (u32): [0..KEY_LEVELS+1] per-level node counts (level 0 = root),
-// [32] nodes that hit the key-depth limit with > LEAF_SIZE particles, [33] max depth.
+// [32] nodes that hit the key-depth limit with > LEAF_SIZE particles, [33] max depth, [34] the level that
+// k_tree_cluster left to k_tree_com (0: none), [40..41] the phases of those.
 constexpr int CNT_DEPTH_LIMIT = 32;
 constexpr int CNT_MAX_DEPTH = 33;
+constexpr int CNT_WIDE = 34;
+constexpr int CNT_PHASES = 40;
 constexpr int CNT_WORDS = 64;
 
 __device__ __forceinline__ uint32_t digit_at(uint64_t key, int shift) { return (uint32_t)(key >> shift) & 7u; }
@@ -452,10 +455,33 @@ __device__ __forceinline__ void finish_node(uint32_t node, uint4* link, const fl
   }
 }
 
-__global__ void __launch_bounds__(BUILD_THREADS) k_tree_com(uint4* link, const float4* __restrict__ x4, const D3* chunk,
-                                                            const D3* totals, float4* mass,
-                                                            const uint32_t* __restrict__ counters, uint32_t capacity,
-                                                            uint32_t dense_depth, uint32_t n_box, uint32_t* words) {
+// The centres of mass of all nodes, after the levels from counters[CNT_WIDE] on that k_tree_cluster found too wide
+// for itself, each a phase over all CTAs.
+__global__ void __launch_bounds__(BUILD_THREADS, 5) k_tree_com(int levels, const uint64_t* __restrict__ keys, uint4* link,
+                                                            float4* geo, const float4* __restrict__ x4,
+                                                            const D3* chunk, const D3* totals, float4* mass,
+                                                            uint32_t* counters, uint32_t capacity,
+                                                            uint32_t dense_depth, uint32_t n_box, uint32_t* words,
+                                                            DevStatus* st) {
+  if (const int wide = (int)counters[CNT_WIDE]) {
+    Phases phases(counters + CNT_PHASES);
+    uint32_t lb = 0, cnt = __ldcg(counters + wide);
+    for (int d = 0; d < wide; ++d) lb += __ldcg(counters + d);
+    for (int d = wide; d <= levels && cnt; ++d) {
+      const uint32_t blocks = min(gridDim.x, (cnt + BUILD_THREADS / 32 - 1) / (BUILD_THREADS / 32));
+      uint32_t item;
+      while (phases.take(blocks, item)) {
+        split_level(d, levels, lb, cnt, keys, x4, link, geo, counters, capacity, st, item, blocks);
+        phases.done();
+      }
+      if (!phases.next(blocks)) {
+        if (threadIdx.x == 0) dev_fail(st, DEV_WAIT_LIMIT, d);
+        return;
+      }
+      lb += cnt;
+      cnt = __ldcg(counters + d + 1);
+    }
+  }
   uint32_t total = 0;
   for (int j = 0; j <= KEY_LEVELS; ++j) total += counters[j];
   total = min(total, capacity);
@@ -603,8 +629,11 @@ __global__ void __launch_bounds__(TOP_THREADS) k_tree_top(int levels, const uint
 // Levels first .. last of the build by one cluster of CTAs in one launch, a level per cluster barrier,
 // ending at the deepest level there is: the top levels of a batch, and the levels below every node of a
 // smooth distribution, of which a clustered one has some and a smooth one none (as launches of their
-// own they are 2 to 4 us each). first = 0 also makes the roots; with `chunk` one CTA scans the tile
-// totals.
+// own they are 2 to 4 us each). A level of more than WIDE_LEVEL nodes ends it and is left to k_tree_com with all
+// below: 65,536 particles in 100 haloes take 0.142 ms with levels of up to 16,384 nodes here and 0.171 with up
+// to 8192, larger levels want the chip (4e6 particles in haloes of 1500 0.48 ms, all levels here 2.2).
+// first = 0 makes the roots (and no level is too wide); with `totals` one CTA scans the tile totals.
+constexpr uint32_t WIDE_LEVEL = 16384;
 constexpr int CLUSTER_CTAS = 8;
 constexpr int CLUSTER_THREADS = 1024;
 __global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
@@ -624,6 +653,10 @@ __global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_T
   for (int d = first; d <= last; ++d) {
     const uint32_t cnt = __ldcg(counters + d);
     if (cnt == 0) break;
+    if (first > 0 && cnt > WIDE_LEVEL) {
+      if (block == 0 && threadIdx.x == 0) counters[CNT_WIDE] = (uint32_t)d;
+      break;
+    }
     split_level(d, levels, lb, cnt, keys, x4, link, geo, counters, capacity, st, block, CLUSTER_CTAS);
     lb += cnt;
     cluster.sync();
@@ -749,8 +782,8 @@ cudaError_t tree_build(TreeNodes& t, const uint64_t* sorted_keys, const float* s
   int box_spread = 0;
   for (size_t c = n_box ? n_box : n; c > 1; c >>= 3) ++box_spread;
   const uint32_t dense_depth = (n_box ? n_box : n) <= ORDERED_PARTICLES ? (uint32_t)(box_spread + ORDERED_DEPTH) : 0x80u;
-  k_tree_com<<<2 * BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(link, x4, chunk, totals, mass, counters, capacity, dense_depth,
-                                                        (uint32_t)n_box, tree_words(t, n));
+  k_tree_com<<<2 * BUILD_BLOCKS, BUILD_THREADS, 0, s>>>(levels, sorted_keys, link, geo, x4, chunk, totals, mass, counters,
+                                                        capacity, dense_depth, (uint32_t)n_box, tree_words(t, n), st);
   t.has_quad = quad_half_max > 0.0f;
   if (t.has_quad) {
     if ((e = ensure(t.quad, 2 * t.capacity * sizeof(float4))) != cudaSuccess) return e;

@@ -67,3 +67,28 @@ def test_sort_time_of_a_concentrated_box(cpm, n):
     uniform = phases(cpm, rng.uniform(0, 1, (n, 3)).astype(np.float32), None)["sort"]
     for x in (0.3 + 1e-4 * rng.standard_normal((n, 3)), np.full((n, 3), 0.25)):
         assert phases(cpm, x.astype(np.float32), None)["sort"] < 6.0 * uniform
+
+
+def haloes(n, members, sigma, seed=5):
+    rng = np.random.default_rng(seed)
+    centres = rng.uniform(0.1, 0.9, (max(1, n // members), 3))
+    return (centres[rng.integers(0, len(centres), n)] + sigma * rng.standard_normal((n, 3))).astype(np.float32)
+
+
+def test_tree_of_wide_deep_levels_is_the_oracles(cpm, orc):
+    """400,000 particles in haloes of 10,000, each smaller than a level-12 cube: levels of tens of thousands of
+    nodes from there on, after narrow ones."""
+    x = haloes(400000, 10000, 2e-5)
+    stats = {}
+    got = cpm.tree_accelerations(x, 1.0, cpm.ForceSplit(5e-7, 2e-6, 1e-7, 0.5), 1.0, stats=stats).astype(np.float64)
+    tree = orc.tree_build(x, 1.0)
+    assert stats["nodes"] == len(tree["count"])
+    ref = orc.tree_accelerations_com64(x, 1.0, orc.Split(5e-7, 2e-6, 1e-7, 0.5), 1.0).astype(np.float64)
+    assert np.sqrt(((got - ref) ** 2).sum()) <= 1e-5 * np.sqrt((ref ** 2).sum())
+
+
+def test_build_time_of_a_concentrated_box(cpm):
+    n = 4000000
+    split = cpm.ForceSplit(1e-6, 4e-6, 1e-7, 0.5)
+    uniform = phases(cpm, np.random.default_rng(4).uniform(0, 1, (n, 3)).astype(np.float32), split)["build"]
+    assert phases(cpm, haloes(n, 1500, 5e-5), split)["build"] < 4.0 * uniform
