@@ -53,6 +53,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cpm_host.h"
@@ -562,9 +563,15 @@ __device__ __forceinline__ bool walk_ordered(const uint32_t* __restrict__ words,
   return words[WALK_DENSE + box] != 0u && words[WALK_OUTSIDE] == 0u;
 }
 
+// The box of a group in a batch: that of its first valid lane (a box's particles fill whole groups, and a list
+// keeps each box's particles in whole groups).
+__device__ __forceinline__ uint32_t group_box(uint32_t lanes, size_t i, const WalkParams& w) {
+  return w.n_box ? __shfl_sync(0xffffffffu, (uint32_t)(i / w.n_box), __ffs(lanes) - 1) : 0u;
+}
+
 // One warp (or `team` warps of a block, each with its share of the direct nodes and accepted nodes)
 // walks for a group of 32 particles.
-template <bool QUAD, bool LIST, int WARPS, bool SKIP = false>
+template <bool QUAD, bool LIST, int WARPS, bool SKIP>
 __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_walk(const uint4* __restrict__ link,
                                                             const float4* __restrict__ geo,
                                                             const float4* __restrict__ mass,
@@ -608,7 +615,7 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
     const size_t i = LIST ? (valid ? (size_t)list[t] : 0) : t;
     const unsigned lanes = __ballot_sync(FULL, valid);
     // (SKIP: the groups of boxes that k_walk_ordered walks are left out)
-    const bool elsewhere = SKIP && lanes && walk_ordered(words, ticket / (w.n_box ? w.n_box / 32 : 0x7FFFFFFFu));
+    const bool elsewhere = SKIP && lanes && walk_ordered(words, group_box(lanes, i, w));
     const unsigned group = elsewhere ? 0u : lanes;
     const float4 xi = valid ? __ldg(x4 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const float x0 = xi.x, x1 = xi.y, x2 = xi.z;
@@ -645,10 +652,8 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
       // children of an opened node) placed in consecutive slots. `mine` holds the slots this lane
       // walks. Lane c copies slot c's three records into shared memory asynchronously; the next step's
       // copies are in flight while the direct sums are formed. The walk starts at the root: node 0, or
-      // in a batch of boxes the root of the warp's box (nodes 0 .. boxes - 1; a box's particles fill
-      // whole warps, and a list keeps each box's particles in whole warps, so the first valid lane's
-      // box is the warp's).
-      const uint32_t root = w.n_box ? __shfl_sync(FULL, (uint32_t)(i / w.n_box), __ffs(group) - 1) : 0u;
+      // in a batch of boxes the root of the warp's box (nodes 0 .. boxes - 1).
+      const uint32_t root = group_box(group, i, w);
       uint32_t b_count = 1, mine = (group >> lane) & 1u;
       if (lane == 0) {
         cp_async16(&sh.geo[0], geo + root);
@@ -1098,7 +1103,7 @@ __device__ __forceinline__ void chunk_forces(const OrderedShared& sh, uint32_t p
   }
 }
 
-template <bool QUAD>
+template <bool QUAD, bool LIST>
 __global__ void __launch_bounds__(ORDERED_WARPS * 32, 9) k_walk_ordered(const uint4* __restrict__ link,
                                                             const float4* __restrict__ geo,
                                                             const float4* __restrict__ mass,
@@ -1107,6 +1112,8 @@ __global__ void __launch_bounds__(ORDERED_WARPS * 32, 9) k_walk_ordered(const ui
                                                             const float* __restrict__ far, float* __restrict__ acc3,
                                                             int accumulate, unsigned long long* counters,
                                                             DevStatus* st, const float* __restrict__ k_dev,
+                                                            const uint32_t* __restrict__ list,
+                                                            const uint32_t* __restrict__ list_n,
                                                             const float4* __restrict__ quad,
                                                             const uint32_t* __restrict__ words) {
   // Dynamic shared memory: ORDERED_WARPS OrderedShared records, then (quadrupoles) the node index of each slot.
@@ -1115,10 +1122,13 @@ __global__ void __launch_bounds__(ORDERED_WARPS * 32, 9) k_walk_ordered(const ui
   uint32_t(*node_ids)[2][SLOTS] = reinterpret_cast<uint32_t(*)[2][SLOTS]>(walk_smem + ORDERED_WARPS * sizeof(OrderedShared));
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t i = ((size_t)blockIdx.x * ORDERED_WARPS + warp) * 32 + lane;
-  const bool valid = i < n;
+  const size_t t = ((size_t)blockIdx.x * ORDERED_WARPS + warp) * 32 + lane;
+  const bool valid = t < (LIST ? (size_t)*list_n : n);
+  const size_t i = LIST ? (valid ? (size_t)list[t] : 0) : t;
   const unsigned group = __ballot_sync(FULL, valid);
-  if (group == 0 || !walk_ordered(words, w.n_box ? (uint32_t)(i / w.n_box) : 0u)) return;
+  if (group == 0) return;
+  const uint32_t root = group_box(group, i, w);
+  if (!walk_ordered(words, root)) return;
   OrderedShared& sh = shared[warp];
   const float4 xi = valid ? __ldg(x4 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const float x0 = xi.x, x1 = xi.y, x2 = xi.z;
@@ -1152,9 +1162,7 @@ __global__ void __launch_bounds__(ORDERED_WARPS * 32, 9) k_walk_ordered(const ui
   // slots. `mine` holds the slots this lane walks. Lane c copies slot c's three records into shared
   // buffer `cur` asynchronously; the next step's copies are in flight while the current step is
   // summed. The walk starts at the root: node 0, or in a batch of boxes the root of the warp's box
-  // (nodes 0 .. boxes - 1; a box's particles fill whole warps, and a list keeps each box's
-  // particles in whole warps, so the first valid lane's box is the warp's).
-  const uint32_t root = w.n_box ? __shfl_sync(FULL, (uint32_t)(i / w.n_box), __ffs(group) - 1) : 0u;
+  // (nodes 0 .. boxes - 1).
   uint32_t b_count = 1, mine = (group >> lane) & 1u;
   int cur = 0;
   if (lane == 0) {
@@ -1506,19 +1514,23 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
   w.ordered.eps2 = dup(w.eps2);
   w.ordered.neg_m = dup(-1.0f);
   const size_t groups = (n + 31) / 32;
-  const bool ordered = t.trajectories && !list && (t.n_box ? t.n_box : n) <= ORDERED_PARTICLES;
+  const bool ordered = t.trajectories && (t.n_box ? t.n_box : n) <= ORDERED_PARTICLES;
   // warps per block: the autotuned group count for the plain and list walks; 4 with quadrupoles
   // A batch goes by the groups of one box, so that a box's sums are those of its own simulation.
   const size_t box_groups = t.n_box ? (t.n_box + 31) / 32 : groups;
   const int team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
   const int warps = t.has_quad || team > 1 || ordered ? 4 : (t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
   unsigned blocks = (unsigned)((groups * team + warps - 1) / warps);
-  auto kernel = t.has_quad ? (list ? k_tree_walk<true, true, 4> : ordered ? k_tree_walk<true, false, 4, true>
-                                                                          : k_tree_walk<true, false, 4>)
-              : ordered    ? k_tree_walk<false, false, 4, true>
-              : warps == 2 ? (list ? k_tree_walk<false, true, 2> : k_tree_walk<false, false, 2>)
-              : warps == 8 ? (list ? k_tree_walk<false, true, 8> : k_tree_walk<false, false, 8>)
-                           : (list ? k_tree_walk<false, true, 4> : k_tree_walk<false, false, 4>);
+  auto pick = [&](auto lists, auto skips) {
+    constexpr bool L = decltype(lists)::value, S = decltype(skips)::value;
+    return t.has_quad   ? k_tree_walk<true, L, 4, S>
+           : warps == 2 ? k_tree_walk<false, L, 2, S>
+           : warps == 8 ? k_tree_walk<false, L, 8, S>
+                        : k_tree_walk<false, L, 4, S>;
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  auto kernel = list ? (ordered ? pick(yes, yes) : pick(yes, no)) : (ordered ? pick(no, yes) : pick(no, no));
   const size_t smem = (size_t)warps * (sizeof(WalkShared) + (t.has_quad ? SLOTS * sizeof(uint32_t) : 0));
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (team == 1) {  // as many blocks as fit on the chip at once
@@ -1534,14 +1546,15 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
                                          reinterpret_cast<unsigned long long*>(counters), st, k_dev, list, list_n,
                                          t.has_quad ? static_cast<const float4*>(t.quad.p) : nullptr, words, team);
   if (ordered) {
-    auto second = t.has_quad ? k_walk_ordered<true> : k_walk_ordered<false>;
+    auto second = t.has_quad ? (list ? k_walk_ordered<true, true> : k_walk_ordered<true, false>)
+                             : (list ? k_walk_ordered<false, true> : k_walk_ordered<false, false>);
     const size_t smem2 = ORDERED_WARPS * (sizeof(OrderedShared) + (t.has_quad ? 2 * SLOTS * sizeof(uint32_t) : 0));
     if (smem2 > 48 * 1024) cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     count_launch();
     second<<<(unsigned)((groups + ORDERED_WARPS - 1) / ORDERED_WARPS), ORDERED_WARPS * 32, smem2, s>>>(
         static_cast<const uint4*>(t.link.p), static_cast<const float4*>(t.geo.p), static_cast<const float4*>(t.mass.p),
         as<float4>(tm.x4), n, w, static_cast<const float*>(fc.far_dev.p), acc3, accumulate,
-        reinterpret_cast<unsigned long long*>(counters), st, k_dev,
+        reinterpret_cast<unsigned long long*>(counters), st, k_dev, list, list_n,
         t.has_quad ? static_cast<const float4*>(t.quad.p) : nullptr, words);
   }
 }
