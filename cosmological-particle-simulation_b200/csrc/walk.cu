@@ -74,6 +74,13 @@ constexpr int WINDOW = 448;   // direct-sum sources collected before they are su
 // 0.888 ms with single warps, 0.500 with teams of 4; of 262,144 (8192 groups) 0.426 with single warps, 0.505 with teams of 2,
 // whose warps each repeat the traversal.
 constexpr size_t WALK_FILL = 148 * 96;
+// A batch of boxes takes the team of one of them (the order of a particle's terms is then that of the box's own
+// simulation) as long as its warps fill the chip's rounds no more than eight times over; a larger batch takes single warps, whose
+// sums differ by rounding. A step of 64 boxes of 32^3 (262,144 warps in teams) takes 8.7 ms in its early states and 9.5 in
+// its late ones with teams, 4.5 and 5.5 with single warps; of 16 boxes of 48^3 (221,184) 5.9 and 8.3, and 3.1 and 4.8. The
+// walk before there were teams took 8.5 and 8.4, and 6.5 and 7.2: from about the line on (8 boxes of 48^3, 3.0 and
+// 4.3, before 3.5 and 4.1) the repeated traversals cost more than teams had brought.
+constexpr size_t BATCH_FILL = 8 * WALK_FILL;
 constexpr int WALK_WARPS_PER_SM = 20;  // resident warps the register budget is set for
 constexpr int STAGE = 64;     // candidate sources fetched at a time, two per lane
 constexpr uint32_t FIRST_BITS = 29;  // a stack entry: first node (29 bits) | (count - 1) << 29
@@ -1516,9 +1523,10 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
   const size_t groups = (n + 31) / 32;
   const bool ordered = t.trajectories && (t.n_box ? t.n_box : n) <= ORDERED_PARTICLES;
   // warps per block: the autotuned group count for the plain and list walks; 4 with quadrupoles
-  // A batch goes by the groups of one box, so that a box's sums are those of its own simulation.
+  // A batch goes by the groups of one box, so that a box's sums are those of its own simulation, up to BATCH_FILL.
   const size_t box_groups = t.n_box ? (t.n_box + 31) / 32 : groups;
-  const int team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
+  const int box_team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
+  const int team = groups * box_team <= BATCH_FILL ? box_team : 1;
   const int warps = t.has_quad || team > 1 || ordered ? 4 : (t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
   unsigned blocks = (unsigned)((groups * team + warps - 1) / warps);
   auto pick = [&](auto lists, auto skips) {

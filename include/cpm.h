@@ -369,7 +369,8 @@ int cpm_sim_destroy(cpm_sim* sim);
  * root per box, one walk), and one ensemble step is one CUDA graph in which the classes run as
  * parallel branches. Each box is a Simulation of the reference's step (integrator.rs:174-186) with
  * the class's mesh and split, Zel'dovich ICs (ics.rs:119-182, as cpm_sim_create_zeldovich) from seed
- * first_seed + b, and the common box size, cosmology and schedule; steps are autotuned per class. */
+ * first_seed + b, and the common box size, cosmology and schedule; steps are autotuned per class.
+ * Forces of a box agree with those of its own simulation to f32 rounding. */
 typedef struct cpm_ensemble cpm_ensemble;
 typedef struct {
   int n_side;           /* particles per side of every box of the class; n_side^3 a multiple of 2048 */
