@@ -52,6 +52,9 @@ int check_device_once(std::string* err) {
 // PAGES_PIECE by this thread and up to PAGES_HELPERS more, while the steps launched before still run.
 // Reading 101 MB of six boxes: 32 -> 18 ms with 3 helpers; 27 with 1, 20 with 2, 24 with 7 and 25 with 15 (the
 // kernel's lock on the address space), 22 with pieces of 256 KB.
+// Pieces whose pages are all there (an array that is read into again, memory that malloc had before) are passed
+// over, and without others no helper starts: a state of 64^3 particles into such arrays 0.74 ms, 0.84 with
+// helpers and 0.72 as plain copies; of 32^3 0.167, 0.205 and 0.163; of 200^3 within the timings' noise.
 // A piece that cannot be populated (older kernels, read-only or special mappings) is left to the copy.
 constexpr size_t PAGES_MIN = size_t(1) << 18, PAGES_PIECE = size_t(1) << 20;
 constexpr size_t PAGES_HELPERS = 3;
@@ -77,22 +80,35 @@ void host_pages(std::initializer_list<HostSpan> spans) {
     ++n;
   }
   if (n == 0) return;
-  std::atomic<size_t> next{0};
+  auto piece = [&](size_t i) {
+    size_t r = 0;
+    for (;; ++r) {
+      const size_t c = (ranges[r].end - ranges[r].begin + PAGES_PIECE - 1) / PAGES_PIECE;
+      if (i < c) break;
+      i -= c;
+    }
+    const uintptr_t b = ranges[r].begin + i * PAGES_PIECE;
+    return Range{b, b + std::min(PAGES_PIECE, (size_t)(ranges[r].end - b))};
+  };
+  auto present = [&](const Range& m) {
+    unsigned char there[PAGES_PIECE / 4096];
+    const size_t count = (m.end - m.begin) / page;
+    if (count > sizeof(there) || mincore((void*)m.begin, m.end - m.begin, there) != 0) return false;
+    return std::all_of(there, there + count, [](unsigned char t) { return (t & 1) != 0; });
+  };
+  size_t first = 0;
+  while (first < pieces && present(piece(first))) ++first;
+  if (first == pieces) return;
+  std::atomic<size_t> next{first};
   auto work = [&] {
     for (size_t i; (i = next.fetch_add(1)) < pieces;) {
-      size_t r = 0;
-      for (;; ++r) {
-        const size_t c = (ranges[r].end - ranges[r].begin + PAGES_PIECE - 1) / PAGES_PIECE;
-        if (i < c) break;
-        i -= c;
-      }
-      const uintptr_t b = ranges[r].begin + i * PAGES_PIECE;
-      madvise((void*)b, std::min(PAGES_PIECE, (size_t)(ranges[r].end - b)), MADV_POPULATE_WRITE);
+      const Range m = piece(i);
+      if (i == first || !present(m)) madvise((void*)m.begin, m.end - m.begin, MADV_POPULATE_WRITE);
     }
   };
   std::thread helpers[PAGES_HELPERS];
   const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-  const size_t want = std::min({PAGES_HELPERS, pieces - 1, cores - 1});
+  const size_t want = std::min({PAGES_HELPERS, pieces - first - 1, cores - 1});
   try {
     for (size_t k = 0; k < want; ++k) helpers[k] = std::thread(work);
   } catch (const std::system_error&) {  // no more threads: those that started and this one do it

@@ -40,3 +40,35 @@ def test_state_into_any_buffer(cpm, n_side):
     for k, key in enumerate(("x", "p", "acc")):
         assert np.array_equal(pinned[k].numpy(), want[key])
     sim.close()
+
+
+def test_no_thread_starts_for_a_buffer_whose_pages_are_there(cpm):
+    """Reading into arrays that were written before: the time of a read was up to a quarter longer for threads with
+    nothing to do. Thread ids are given in turn, so the next one tells how many started (other processes' come
+    on top); a read into untouched pages does start some."""
+    import threading
+
+    def next_id():
+        ids = []
+        t = threading.Thread(target=lambda: ids.append(threading.get_native_id()))
+        t.start()
+        t.join()
+        return ids[0]
+
+    n = 45 ** 3
+    x = np.random.default_rng(1).uniform(0, 45, (n, 3)).astype(np.float32) % np.float32(45)
+    sim = cpm.Simulation(cpm.Cosmology(0.0, 0.3, 0.7, 70.0), 45.0, 32, x, np.zeros_like(x), 0.5, None)
+
+    def reads(buffers):
+        before = next_id()
+        for b in buffers:
+            for _ in range(60 // len(buffers)):
+                cpm._native.check(cpm._native.lib().cpm_sim_get_state(sim.h, C.c_void_p(b), None, None, None, None), sim=True)
+        return next_id() - before
+
+    used = np.ones((n, 3), np.float32)
+    maps = [mmap.mmap(-1, 12 * n) for _ in range(60)]
+    fresh = [np.frombuffer(m, np.uint8).ctypes.data for m in maps]
+    assert reads([used.ctypes.data]) < 40 < 60 <= reads(fresh)
+    assert np.array_equal(used, np.frombuffer(maps[-1], np.float32).reshape(n, 3))
+    sim.close()
