@@ -10,7 +10,6 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -111,7 +110,7 @@ void host_pages(std::initializer_list<HostSpan> spans) {
   const size_t want = std::min({PAGES_HELPERS, pieces - first - 1, cores - 1});
   try {
     for (size_t k = 0; k < want; ++k) helpers[k] = std::thread(work);
-  } catch (const std::system_error&) {  // no more threads: those that started and this one do it
+  } catch (...) {  // no more threads: those that started and this one do it
   }
   work();
   for (std::thread& t : helpers)
