@@ -295,7 +295,7 @@ struct TreeNodes {
   DevBuf x4;        // float4 copy of the sorted positions, then the walk's words (WALK_*)
   DevBuf quad;      // per node 2 float4: second moments about the centre of mass (quadrupole mode)
   bool has_quad = false;  // the last build computed `quad`; the walk then adds quadrupole terms
-  int walk_warps = 4;     // warps (groups of 32 particles) per walk block: 2, 4 or 8 (autotuned)
+  int walk_warps = 4;     // warps per walk block asked for: 2, 4 or 8 (autotuned; see tree_walk_warps)
   bool trajectories = false;  // a simulation's tree: dense boxes take the ordered walk (see k_walk_ordered)
   uint32_t n_box = 0;     // batch of boxes: particles per box (a multiple of 32), root of group = box
   size_t capacity = 0;
@@ -343,6 +343,8 @@ float quad_half_bound(const cpm_force_split& split);
 void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_split& split,
                       float k, float* acc3, int accumulate, TreeCounters* counters, DevStatus* st, cudaStream_t s,
                       const float* k_dev = nullptr, const uint32_t* list = nullptr, const uint32_t* list_n = nullptr);
+// Warps per block of a walk of n particles: t.walk_warps, at least a team; 4 with quadrupoles.
+int tree_walk_warps(const TreeNodes& t, size_t n);
 // Releases the walk's per-tree state (the fitted pair-force coefficients).
 void tree_walk_free(TreeNodes& t);
 // ---------------------------------------------------------------------------------------------

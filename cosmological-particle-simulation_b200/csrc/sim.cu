@@ -265,7 +265,7 @@ static int sim_accelerations(cpm_sim* s, float a, const StepScalars* dev = nullp
 //   FFT plan of the Poisson passes        Stockham stages of largest radix 8 (512 = 8.8.8) or 4
 //                                         (4.4.4.4.2)
 //   deposit tile                          256 x {2, 4, 8} sorted particles per CTA
-//   walk group                            {2, 4, 8} warps of 32 particles per block
+//   walk group                            {2, 4, 8} warps per block (small launches: at least a group's team)
 // Each candidate runs once untimed and twice timed with CUDA events on the simulation's stream;
 // the work repeats what the force evaluation did (deposit, Poisson solve) or writes to scratch
 // (walk), so the state is unchanged. Choices are cached per workload (particles, mesh, tree,
@@ -361,6 +361,8 @@ static int sim_autotune(cpm_sim* s) {
     }
   }
   tune_select(c);
+  // Blocks of 4 warps are left only for a gain beyond the timings' noise (where a team of 4 walks a group, 2 is 4).
+  if (c.warps != 4 && c.ms[c.warps == 2 ? 6 : 8] > 0.97f * c.ms[7]) c.warps = 4;
   // The plans round differently: plan 8 is left only for a gain well beyond the timings' noise (meshes of
   // 32 and 48, 0.024 ms against 0.028 and 0.026 against 0.029; from 64 on plan 8 wins or is within 0.002 ms).
   if (c.radix != 8 && c.ms[1] > 0.9f * c.ms[0]) c.radix = 8;
@@ -964,7 +966,7 @@ int cpm_sim_autotune_report(cpm_sim* s, int* fft_radix, int* deposit_tile, int* 
   if (!s) return set_error(nullptr, CPM_E_INVALID, "cpm_sim_autotune_report: sim is NULL");
   if (fft_radix) *fft_radix = s->plan.max_radix;
   if (deposit_tile) *deposit_tile = 256 * s->dep_ppt;
-  if (walk_warps) *walk_warps = s->tree.walk_warps;
+  if (walk_warps) *walk_warps = s->P.use_tree ? tree_walk_warps(s->tree, s->n) : s->tree.walk_warps;
   if (ms9)
     for (int i = 0; i < N_TUNE; ++i) ms9[i] = s->tune_ms[i];
   return CPM_OK;

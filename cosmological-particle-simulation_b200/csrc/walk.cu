@@ -1467,6 +1467,19 @@ void tree_walk_free(TreeNodes& t) {
   t.walk_fit = nullptr;
 }
 
+// Warps that walk one group. A batch goes by the groups of one box, so that a box's sums are those of its own
+// simulation, up to BATCH_FILL.
+static int walk_team(const TreeNodes& t, size_t n) {
+  const size_t groups = (n + 31) / 32, box_groups = t.n_box ? (t.n_box + 31) / 32 : groups;
+  const int box_team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
+  return groups * box_team <= BATCH_FILL ? box_team : 1;
+}
+
+int tree_walk_warps(const TreeNodes& t, size_t n) {
+  if (t.has_quad) return 4;
+  return std::max(walk_team(t, n), t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
+}
+
 void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_split& split,
                       float k, float* acc3, int accumulate, TreeCounters* counters, DevStatus* st, cudaStream_t s,
                       const float* k_dev, const uint32_t* list, const uint32_t* list_n) {
@@ -1522,12 +1535,7 @@ void launch_tree_walk(const TreeNodes& t, size_t n, float box, const cpm_force_s
   w.ordered.neg_m = dup(-1.0f);
   const size_t groups = (n + 31) / 32;
   const bool ordered = t.trajectories && (t.n_box ? t.n_box : n) <= ORDERED_PARTICLES;
-  // warps per block: the autotuned group count for the plain and list walks; 4 with quadrupoles
-  // A batch goes by the groups of one box, so that a box's sums are those of its own simulation, up to BATCH_FILL.
-  const size_t box_groups = t.n_box ? (t.n_box + 31) / 32 : groups;
-  const int box_team = box_groups * 4 <= WALK_FILL ? 4 : (box_groups * 2 <= WALK_FILL ? 2 : 1);
-  const int team = groups * box_team <= BATCH_FILL ? box_team : 1;
-  const int warps = t.has_quad || team > 1 || ordered ? 4 : (t.walk_warps == 2 || t.walk_warps == 8 ? t.walk_warps : 4);
+  const int team = walk_team(t, n), warps = tree_walk_warps(t, n);
   unsigned blocks = (unsigned)((groups * team + warps - 1) / warps);
   auto pick = [&](auto lists, auto skips) {
     constexpr bool L = decltype(lists)::value, S = decltype(skips)::value;
