@@ -16,7 +16,7 @@
 
 namespace cpm {
 
-constexpr int N_TUNE = 9;  // timed candidates: 3 FFT plans, 3 deposit tiles, 3 walk groups
+constexpr int N_TUNE = 9;  // the candidates: FFT plans (0 is the same as 8 and not timed), deposit tiles, walk groups
 
 struct TuneChoice {
   int radix = 8, ppt = 4, warps = 4;

@@ -344,8 +344,8 @@ int cpm_step_factors(const cpm_cosmology* cosmo, double a0, double a1, int fp64,
  * (8 or 4: Stockham stages of largest radix 8 or 4; 0: the same as 8), the deposit tile (512,
  * 1024 or 2048 sorted particles per CTA) and the walk group (2, 4 or 8 warps per block, as the walk runs
  * it: 4 for 2 where 4 warps walk a group of 32 particles together, in boxes of up to 113,664 particles, and
- * 4 with quadrupoles). ms9 (may be NULL) receives the measured ms per call: plan 8, 4, 0; tile 512, 1024, 2048;
- * warps 2, 4, 8 (0 where not timed). */
+ * 4 with quadrupoles). ms9 (may be NULL) receives the measured ms per call: plan 8, 4, 0 (0: never timed); tile 512,
+ * 1024, 2048; warps 2, 4, 8 (0 where not timed). */
 int cpm_sim_autotune_report(cpm_sim* sim, int* fft_radix, int* deposit_tile, int* walk_warps, float* ms9);
 /* Overrides the autotuner's choices (FFT plan 8, 4 or 0, tile 512, 1024 or 2048, warps 2, 4 or 8); the
  * next force evaluation uses them. Deposit tile and walk group do not change any result bit; the FFT
