@@ -319,7 +319,7 @@ cudaError_t tree_pack(TreeNodes& t, const float* sorted_x3, size_t n, float box,
 struct TreeCounters {
   unsigned long long leaf_pairs;    // pairs within r_cut summed directly
   unsigned long long node_accepts;  // accepted centres of mass
-  unsigned long long candidates;    // (particle, source) pairs tested against r_cut in direct nodes
+  unsigned long long candidates;    // (particle, source) pairs put to the distance test (see cpm_sim_walk_candidates)
   unsigned long long reserved;
 };
 // Builds the octree over sorted keys and packed positions (t.x4; sorted x as AoS f32 for the quadrupoles). Returns the node count

@@ -391,9 +391,8 @@ template <int W>
 int col_tile_count(const ColGeo& g) {
   return g.outer * ((g.cols + W - 1) / W);
 }
-// Stores of a pass whose spectra are larger than L2: evict-first (STREAM). Left in L2 as ordinary stores, the
-// strided lines of a 512^3 mesh reach DRAM 1.3 to 1.6 times each; meshes that L2 holds part of for the next
-// pass are faster with ordinary ones.
+// Stores of the strided passes of meshes from STREAM_MESH on: evict-first (STREAM). Left in L2 as ordinary stores,
+// the strided lines of a 512^3 mesh reach DRAM 1.3 to 1.6 times each.
 template <bool STREAM>
 __device__ __forceinline__ void put(float2* p, float2 v) {
   if constexpr (STREAM)
@@ -679,8 +678,9 @@ static float exact_inverse(float x) {
   return x > 1e-30f && x < 1e30f && std::frexp(x, &e) == 0.5f ? 1.0f / x : 0.0f;
 }
 
-// Meshes whose strided passes store evict-first: the five passes of 512^3 3.48 -> 3.19 ms when it was
-// introduced; 384^3 1.75 -> 1.81, 320^3 1.02 -> 1.05 (256^3 0.400 -> 0.394 later).
+// Meshes whose strided passes store evict-first, by measurement and not by the size of L2 (126 MB; a spectrum is 69 MB
+// at 256, 231 at 384, 545 at 512): the five passes of 512^3 3.48 -> 3.19 ms when it was introduced, but 384^3
+// 1.75 -> 1.81 and 320^3 1.02 -> 1.05; 256^3 would gain 1.5 % (0.400 -> 0.394).
 constexpr int STREAM_MESH = 512;
 
 // One tile per CTA.

@@ -32,8 +32,8 @@
 // a superset by a margin of 2e-6; sources that close to the cutoff are settled by the reference's own
 // r^2 in the second phase. Words whose sources may need a periodic image form the nearest image.
 //
-// What bounds it: instruction issue (68 % of the slots at 5 warps per scheduler; FMA pipe 37 %, DRAM
-// idle). Per group at 128^3 particles / 256^3 mesh near the initial state: traversal 6.5, fetching
+// What bounds it: instruction issue (66 % of the slots early in a run, 70 % in clustered states, at 5 warps per
+// scheduler; FMA pipe 33 and 43 %, DRAM idle). Per group at 128^3 particles / 256^3 mesh near the initial state: traversal 6.5, fetching
 // 5.2, marking 5.1 and pair forces 9.0 thousand warp instructions, of 88 pairs per particle; in a
 // clustered state 12.7, 5.5, 9.4 and 24.8 thousand, of 325 pairs. Testing every particle against
 // every direct node and chunk of 32 sources, without the group's decisions, the culled window and
@@ -979,17 +979,20 @@ __global__ void __launch_bounds__(WARPS * 32, WALK_WARPS_PER_SM / WARPS) k_tree_
 }
 
 // ---------------------------------------------------------------------------------------------
-// The walk in the order of the reference's chunks. Every lane classifies every node of a step, the step's direct
-// sums follow at once, in chunks of 32 sources of the concatenated nodes, and a lane adds its pairs of a chunk
-// two by two: the order in which a particle's terms are added depends on nothing but the tree and the group.
-// It is slower than k_tree_walk (walk of 91,125 clustered particles 0.90 ms against 0.50) and serves the
-// boxes of up to ORDERED_PARTICLES particles in which the build split nodes ORDERED_DEPTH levels and more below
-// the level of a smooth distribution (WALK_DENSE): in their cores, where pairs lie closer than the softening,
-// one rounding of a position moves an acceleration by up to 1e-3 of the box's RMS, so that another
-// order of f32 sums shows there after ten steps (largest difference of an acceleration after 18 steps, of the
-// RMS, eight boxes each: 3.7e-4 where the deepest split is 4 levels below a smooth box's, 21^3 particles;
-// 8.6e-4 at 5 levels, 27^3; 1.2e-2 at 6, 64^3), and trajectories of such boxes are kept as they were. Larger
-// boxes go by statistics, and their walk is most of their step.
+// The ordered walk. Every lane classifies every node of a step, the step's direct sums follow at once, in chunks of 32
+// sources of the concatenated nodes, and a lane adds its pairs of a chunk two by two, as this library did before
+// k_tree_walk collected its sources in a window. The order is neither the reference's nor more accurate: against 64
+// bits both walks' forces are off by 8.7e-7 of the RMS at 45^3 late particles, 2.5e-6 at 64^3, 2.4e-5 at 101^3
+// (RMS; medians 1.7e-7 and 1.3e-7, 1.9e-7 both, 3.2e-7 and 2.5e-7). What it keeps is the roundings, and with them the
+// trajectories that dense boxes had: in a core whose pairs lie closer than the softening one rounding of a position moves
+// an acceleration by up to 1e-3 of the box's RMS, so that another order of f32 sums shows after ten steps (largest
+// difference of an acceleration after 18 steps, of the RMS, eight boxes each: 3.7e-4 where the deepest split is 4 levels
+// below a smooth box's, 21^3 particles; 8.6e-4 at 5 levels, 27^3; 1.2e-2 at 6, 64^3). It serves the simulations, with
+// and without a list of walked particles, whose build split nodes ORDERED_DEPTH levels and more below the level of a
+// smooth distribution (WALK_DENSE); until then, and from ORDERED_PARTICLES particles on, a box goes by k_tree_walk. That
+// bound is one of cost, not of rounding: the walk is most of a large box's step, and this one is
+// slower: 0.60 ms against 0.20 at 27^3 late particles, 0.78 against 0.47 at 45^3, 1.10 against 0.81 at 64^3, 3.38 against
+// 2.55 at 101^3.
 // ---------------------------------------------------------------------------------------------
 constexpr int ORDERED_WARPS = 4;
 constexpr int ORDERED_MERGE_SP = 96;

@@ -298,8 +298,10 @@ int cpm_sim_set_state(cpm_sim* sim, const float* x3, const float* p3);
  * [0] kick+drift, [1] keys+sort+reorder, [2] deposit, [3] FFT-Poisson, [4] gather, [5] tree build,
  * [6] tree walk, [7] whole step. Also the number of steps averaged. */
 int cpm_sim_phase_times(cpm_sim* sim, double* ms8, uint64_t* steps, int reset);
-/* (particle, source) pairs the last step's walk tested against r_cut inside direct-summed nodes
- * (leaf pairs are the subset within r_cut). */
+/* (particle, source) pairs that the last step's walk put to the distance test (leaf pairs are the subset
+ * within r_cut): for every particle the sources of its group's direct-summed nodes that lie within r_cut of the
+ * bounding box of the group of 32; in dense boxes, which take another walk, all particles of its direct-summed
+ * nodes. A measure of the walk's work, comparable between states and not between versions. */
 int cpm_sim_walk_candidates(cpm_sim* sim, uint64_t* candidates);
 /* Self-check of the walk's pair kernel (host only): largest relative error of its fitted
  * S(r) = erfc(u) + (2/sqrt(pi)) u e^{-u^2}, u = r / (2 r_split) (tree.rs:54-57), against a
